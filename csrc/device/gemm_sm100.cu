@@ -4,15 +4,14 @@
 
 #include <algorithm>
 #include <atomic>
-#include <map>
-#include <vector>
+#include <cmath>
 #include <mutex>
 
 #include "../core/log.h"
 #include "gemm_api.h"
 #include "gemm_sm100.cuh"
-#include "gemm_sm100_2sm.cuh"
 #include "gemm_sm100_2sm_wide.cuh"
+#include "gemm_sm100_swap.cuh"
 
 namespace hc {
 
@@ -28,21 +27,6 @@ GemmBf16Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 {
     hcgemm::GemmMainLoop<BN>(&tmA, &tmB, shape, hcgemm::GroupedOrder{shape.tilesM < 16 ? shape.tilesM : 16}, hcgemm::NoGate(), epi);
 }
-// CTA-pair variant: 256 x 256 tiles, launched as clusters of two CTAs (see gemm_sm100_2sm.cuh).
-template <int BN>
-__global__ void __launch_bounds__(hcgemm::kThreads, 1)
-GemmBf16PairStagedKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, hcgemm::GemmShape shape, hcgemm::StoreBf16Staged epi, int gm)
-{
-    hcgemm::GemmMainLoopPair<BN, 6>(&tmA, &tmB, shape, hcgemm::GroupedOrder{shape.tilesM < gm ? shape.tilesM : gm}, epi);
-}
-
-template <int BN, int STAGES>
-__global__ void __launch_bounds__(hcgemm::kThreads, 1)
-GemmBf16PairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, hcgemm::GemmShape shape, hcgemm::StoreBf16 epi, int gm)
-{
-    hcgemm::GemmMainLoopPair<BN, STAGES>(&tmA, &tmB, shape, hcgemm::GroupedOrder{shape.tilesM < gm ? shape.tilesM : gm}, epi);
-}
-
 // 256 x 512 tiles, one accumulator per CTA (see gemm_sm100_2sm_wide.cuh).
 __global__ void __launch_bounds__(hcgemm::kWideThreads, 1)
 GemmBf16PairWideKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC, hcgemm::GemmShape shape, int gm)
@@ -50,32 +34,37 @@ GemmBf16PairWideKernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     hcgemm::GemmMainLoopPairWide<4>(&tmA, &tmB, &tmC, shape, hcgemm::GroupedOrder{shape.tilesM < gm ? shape.tilesM : gm});
 }
 
-// Clusters of two CTAs that can be resident at once (0 when the query fails).
-int PairClusterCapacity()
+// 256 weights x bn tokens, SPLIT pairs of a cluster along K (see gemm_sm100_swap.cuh).
+template <int SPLIT>
+__global__ void __launch_bounds__(hcgemm::kSwapThreads, 1)
+GemmBf16SwapKernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, hcgemm::SwapShape shape)
 {
-    static int cap = -1;
-    if (cap >= 0) return cap;
-    cudaFuncSetAttribute(GemmBf16PairKernel<256, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::Config2<256, 7>::kSmemBytes);
-    cudaFuncSetAttribute(GemmBf16PairKernel<224, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::Config2<224, 7>::kSmemBytes);
-    cudaFuncSetAttribute(GemmBf16PairKernel<192, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::Config2<192, 7>::kSmemBytes);
-    cudaFuncSetAttribute(GemmBf16PairKernel<160, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::Config2<160, 7>::kSmemBytes);
-    cudaFuncSetAttribute(GemmBf16PairKernel<128, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::Config2<128, 7>::kSmemBytes);
-    cudaFuncSetAttribute(GemmBf16PairStagedKernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::Config2<256, 6, true>::kSmemBytes);
-    cudaFuncSetAttribute(GemmBf16PairWideKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::ConfigWide<4>::kSmemBytes);
+    hcgemm::GemmMainLoopSwap<SPLIT>(&tmW, &tmX, shape);
+}
+
+template <int SPLIT> int SwapCapacityOf()
+{
+    if (cudaFuncSetAttribute(GemmBf16SwapKernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) { cudaGetLastError(); return 0; }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * 148, 1, 1);
-    cfg.blockDim = dim3(hcgemm::kThreads, 1, 1);
-    cfg.dynamicSmemBytes = hcgemm::Config2<256, 7>::kSmemBytes;
+    cfg.gridDim = dim3(2 * SPLIT * 148, 1, 1);
+    cfg.blockDim = dim3(hcgemm::kSwapThreads, 1, 1);
+    cfg.dynamicSmemBytes = hcgemm::SwapSmemBytes(256);
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[0].val.clusterDim.x = 2 * SPLIT; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, GemmBf16PairKernel<256, 7>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
-    cap = n;
-    HCCL_INFO("GEMM CTA pairs resident at once: %d", cap);
-    return cap;
+    if (cudaOccupancyMaxActiveClusters(&n, GemmBf16SwapKernel<SPLIT>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+    HCCL_INFO("GEMM clusters of %d CTAs resident at once: %d", 2 * SPLIT, n);
+    return n;
 }
+// Clusters of 2^log2Pairs CTA pairs that can be resident at once (0 when the query fails).
+int SwapCapacity(int log2Pairs)
+{
+    static const int cap[3] = {SwapCapacityOf<1>(), SwapCapacityOf<2>(), SwapCapacityOf<4>()};
+    return cap[log2Pairs];
+}
+
 }  // namespace
 
 HcclResult MakeTensorMap2dBf16(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, uint64_t ldElems, uint32_t boxRows, uint32_t boxCols)
@@ -113,7 +102,7 @@ HcclResult MakeTensorMap2dBf16(CUtensorMap *map, const void *base, uint64_t rows
 // partitions and a panel that both halves of the chip read occupies both, so the budget is about half the nominal 126 MB.
 // HCOMM_GEMM_GM or HcommGemmSetTuning override the choice.
 namespace {
-std::atomic<int> g_forceGm{-1}, g_forceBn{-1};
+std::atomic<int> g_forceGm{-1}, g_forceBn{-1}, g_forceSplit{0};
 }
 int PairGroupRows(int K)
 {
@@ -170,172 +159,124 @@ uint32_t *GemmErrorFlag()
 
 namespace {
 
-// One launch of the CTA-pair kernel with tile width bn and rasterisation group gm.
-HcclResult LaunchPairGemm(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, int bn, int gm, void *stream)
+// Tile of the CTA-pair kernels for a shape: tokens per tile and pairs that share a tile along K for the one with exchanged
+// operands (gemm_sm100_swap.cuh), or 256 x 512 (gemm_sm100_2sm_wide.cuh).  The estimate below, in nanoseconds, was fitted to
+// about 120 timings (M 1 .. 8192, N 1024 .. 128256, K 1024 .. 28672) and agrees with nearly all of them within 10 %:
+//   * a 64-deep step of a 256 x bn tile takes 48 + 1.28 bn ns on the tensor core at the clock that a GPU under such load
+//     holds, but never less than its operands (16 KB of weights, 128 bytes per token and CTA) at 120 bytes per ns and SM;
+//   * tiles come in whole waves of the clusters that fit at once (74 of two CTAs, 33 of four, 15 of eight);
+//   * all operand traffic passes L2 at 13.5 TB/s, every operand comes from HBM once at 6.5 TB/s, a tenth less when only a
+//     few SMs ask for it;
+//   * a launch costs 3 us, emptying the accumulator 6 ns per token, exchanging partial sums 1.5 us and 8 ns per token; a
+//     further wave of clusters that share tiles starts from nothing, 3 us;
+//   * a 256 x 512 tile moves a quarter less operand data than two of 256 x 256, and under the power cap that sets the clock:
+//     690 ns a step against 752, but 4 us in which nothing overlaps the emptying of its one accumulator.
+// Examples, us, against the fixed choice before (128 x 256 tiles of one CTA below 256 rows or at ragged ones):
+// 16 x 8192 x 28672 32/2 71 (165), 96 x 3584 x 8192 96/4 15 (51), 777 x 4096 x 14336 224/1 82 (97), 33 x 128256 x 4096
+// 64/1 165 (185), 5003 x 8192 x 3584 224/1 210 (235).  Half a second into a run at the power cap 8192 x 28672 x 8192 takes
+// 2929 with 256 x 512 and 3149 with 256 x 256 tiles (from a cool start 2988 and 2783), 8192 x 3584 x 8192 414 and 395.
+struct PairTile { int bn, split; };      // bn = 512: the 256 x 512 kernel
+PairTile PickPairTile(int M, int N, int K, const int (&cap)[3])
 {
-    CUtensorMap tmA, tmB;
-    CHK_RET(MakeTensorMap2dBf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, hcgemm::kBlockM, hcgemm::kBlockK));
-    CHK_RET(MakeTensorMap2dBf16(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, bn == hcgemm::kWideN ? 128u : (uint32_t)(bn / 2), hcgemm::kBlockK));
-    hcgemm::GemmShape shape;
-    shape.M = M; shape.N = N; shape.K = K;
-    shape.tilesM = M / hcgemm::kPairM;
-    shape.tilesN = N / bn;
-    shape.errFlag = GemmErrorFlag();
-    shape.phase = nullptr;
-    hcgemm::StoreBf16 epi{(__nv_bfloat16 *)C, ldc, M, N};
-    const int clusters = std::min(PairClusterCapacity(), shape.tilesM * shape.tilesN);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * clusters, 1, 1);
-    cfg.blockDim = dim3(hcgemm::kThreads, 1, 1);
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
-    static const bool stagedEpilogue = [] { const char *e = getenv("HCOMM_GEMM_STAGED"); return e && e[0] == '1'; }();
-    if (stagedEpilogue && ldc % 8 == 0 && bn == 256) {
-        cfg.dynamicSmemBytes = hcgemm::Config2<256, 6, true>::kSmemBytes;
-        hcgemm::StoreBf16Staged sepi{(__nv_bfloat16 *)C, ldc};
-        cudaError_t e2 = cudaLaunchKernelEx(&cfg, GemmBf16PairStagedKernel<256>, tmA, tmB, shape, sepi, gm);
-        if (e2 != cudaSuccess) { HCCL_ERROR("GemmBf16 (CTA pairs, staged epilogue) launch failed: %s", cudaGetErrorString(e2)); return HCCL_E_RUNTIME; }
-        return HCCL_SUCCESS;
-    }
-    cudaError_t e;
-    switch (bn) {
-        case hcgemm::kWideN: {
-            CUtensorMap tmC;            // result tiles leave through TMA stores: boxes of 32 rows x 64 columns
-            CHK_RET(MakeTensorMap2dBf16(&tmC, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64));
-            cfg.dynamicSmemBytes = hcgemm::ConfigWide<4>::kSmemBytes;
-            cfg.blockDim = dim3(hcgemm::kWideThreads, 1, 1);
-            e = cudaLaunchKernelEx(&cfg, GemmBf16PairWideKernel, tmA, tmB, tmC, shape, gm);
-            break;
+    PairTile best{32, 1};
+    double bestNs = 0;
+    const double kBlocks = (K + hcgemm::kBlockK - 1) / hcgemm::kBlockK, tilesW = (N + hcgemm::kPairM - 1) / hcgemm::kPairM;
+    const double hbmNs = 2.0 * ((double)M * K + (double)N * K + (double)M * N) / 6500.0;
+    for (int si = 0; si < 3; ++si) {
+        const int split = 1 << si;
+        if (cap[si] <= 0 || (split > 1 && kBlocks < 4 * split)) continue;
+        for (int bn = 256; bn >= 32; bn -= 32) {
+            if (bn - 32 >= M) continue;                             // a narrower tile holds every token
+            const double tiles = tilesW * ((M + bn - 1) / bn), x = std::min(bn, M);
+            const double waves = std::ceil(tiles / cap[si]), active = std::min(tiles, (double)cap[si]) * split / cap[0];
+            const double step = std::max(48 + 1.28 * bn, (16384 + 64 * x) / 120);
+            const double loop = std::max(waves * std::ceil(kBlocks / split) * step, tiles * kBlocks * (32768 + 128 * x) / 13500);
+            const double ns = std::max(loop, hbmNs / (0.9 + 0.1 * std::min(1.0, active))) + 3000 + 6 * x + (split > 1 ? 1500 + 8 * x + (waves - 1) * 3000 : 0);
+            if (bestNs == 0 || ns < bestNs) { bestNs = ns; best = {bn, split}; }
         }
-        case 256: cfg.dynamicSmemBytes = hcgemm::Config2<256, 7>::kSmemBytes; e = cudaLaunchKernelEx(&cfg, GemmBf16PairKernel<256, 7>, tmA, tmB, shape, epi, gm); break;
-        case 224: cfg.dynamicSmemBytes = hcgemm::Config2<224, 7>::kSmemBytes; e = cudaLaunchKernelEx(&cfg, GemmBf16PairKernel<224, 7>, tmA, tmB, shape, epi, gm); break;
-        case 192: cfg.dynamicSmemBytes = hcgemm::Config2<192, 7>::kSmemBytes; e = cudaLaunchKernelEx(&cfg, GemmBf16PairKernel<192, 7>, tmA, tmB, shape, epi, gm); break;
-        case 160: cfg.dynamicSmemBytes = hcgemm::Config2<160, 7>::kSmemBytes; e = cudaLaunchKernelEx(&cfg, GemmBf16PairKernel<160, 7>, tmA, tmB, shape, epi, gm); break;
-        default: cfg.dynamicSmemBytes = hcgemm::Config2<128, 7>::kSmemBytes; e = cudaLaunchKernelEx(&cfg, GemmBf16PairKernel<128, 7>, tmA, tmB, shape, epi, gm); break;
+    }
+    if (cap[0] > 0) {
+        const double tiles = (double)((M + hcgemm::kPairM - 1) / hcgemm::kPairM) * ((N + hcgemm::kWideN - 1) / hcgemm::kWideN);
+        if (std::max(std::ceil(tiles / cap[0]) * (kBlocks * 690 + 4000), hbmNs) + 3000 < bestNs) best = {hcgemm::kWideN, 1};
+    }
+    return best;
+}
+
+cudaLaunchConfig_t PairConfig(cudaLaunchAttribute *at, int clusters, int clusterCtas, int threads, int smemBytes, void *stream)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(clusters * clusterCtas, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smemBytes;
+    cfg.stream = (cudaStream_t)stream;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = clusterCtas; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cfg;
+}
+
+HcclResult LaunchSwapGemm(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, const PairTile &tile, void *stream)
+{
+    CUtensorMap tmW, tmX;
+    CHK_RET(MakeTensorMap2dBf16(&tmW, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, hcgemm::kBlockM, hcgemm::kBlockK));
+    CHK_RET(MakeTensorMap2dBf16(&tmX, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)(tile.bn / 2), hcgemm::kBlockK));
+    hcgemm::SwapShape g;
+    g.M = M; g.N = N; g.K = K;
+    g.tilesW = (N + hcgemm::kPairM - 1) / hcgemm::kPairM;
+    g.tilesT = (M + tile.bn - 1) / tile.bn;
+    g.bn = tile.bn; g.stages = hcgemm::SwapStages(tile.bn);
+    g.group = PairGroupRows(K);
+    g.C = (__nv_bfloat16 *)C; g.ldc = ldc;
+    g.errFlag = GemmErrorFlag();
+    const int tiles = g.tilesW * g.tilesT;
+    cudaLaunchAttribute at[2];
+    const cudaLaunchConfig_t cfg = PairConfig(at, tile.split > 1 ? tiles : std::min(SwapCapacity(0), tiles), 2 * tile.split, hcgemm::kSwapThreads,
+                                              hcgemm::SwapSmemBytes(tile.bn), stream);
+    cudaError_t e;
+    switch (tile.split) {
+        case 4: e = cudaLaunchKernelEx(&cfg, GemmBf16SwapKernel<4>, tmW, tmX, g); break;
+        case 2: e = cudaLaunchKernelEx(&cfg, GemmBf16SwapKernel<2>, tmW, tmX, g); break;
+        default: e = cudaLaunchKernelEx(&cfg, GemmBf16SwapKernel<1>, tmW, tmX, g); break;
     }
     if (e != cudaSuccess) {
-        HCCL_ERROR("GemmBf16 (CTA pairs) launch failed: %s", cudaGetErrorString(e));
+        HCCL_ERROR("GemmBf16 (tiles of %d tokens, %d CTA pairs along K) launch failed: %s", tile.bn, tile.split, cudaGetErrorString(e));
         return HCCL_E_RUNTIME;
     }
     return HCCL_SUCCESS;
 }
 
-// Tile width and rasterisation group of the CTA-pair kernel for a shape.  The wave model (PickPairTileWidth) and the
-// group rule (PairGroupRows) decide.  With HCOMM_GEMM_AUTOTUNE=1 a large shape seen for the first time is also timed
-// once with the candidates around that choice on the caller's stream - interleaved rounds, medians - and the fastest
-// is kept for the process.  It is off by default: on a GPU at its power cap the variants differ mostly through the
-// clock they leave the chip at (the cycle counts of the 256- and 224-wide variants are within 1 % for every group size;
-// the DRAM traffic, 4 to 10 GB for the benchmark's projections, sets the power), and timings of a few launches each
-// were not stable enough to rank them - repeated runs of one process kept different winners.
-// Never done while the stream is being captured into a graph, nor when a width or group is forced.
-struct ShapeKey {
-    int M, N, K;
-    bool operator<(const ShapeKey &o) const { return M != o.M ? M < o.M : (N != o.N ? N < o.N : K < o.K); }
-};
-std::mutex g_tuneMu;
-std::map<ShapeKey, std::pair<int, int>> g_tuned;
-
-// HCOMM_GEMM_WIDE=0 keeps the tiles at 256 columns or fewer.
-bool WideTilesEnabled()
+HcclResult LaunchWideGemm(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, void *stream)
 {
-    static const bool on = [] { const char *e = getenv("HCOMM_GEMM_WIDE"); return !(e && e[0] == '0'); }();
-    return on;
+    CUtensorMap tmA, tmB, tmC;            // result tiles leave through TMA stores: boxes of 32 rows x 64 columns
+    CHK_RET(MakeTensorMap2dBf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, hcgemm::kBlockM, hcgemm::kBlockK));
+    CHK_RET(MakeTensorMap2dBf16(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 128u, hcgemm::kBlockK));
+    CHK_RET(MakeTensorMap2dBf16(&tmC, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64));
+    hcgemm::GemmShape shape;
+    shape.M = M; shape.N = N; shape.K = K;
+    shape.tilesM = (M + hcgemm::kPairM - 1) / hcgemm::kPairM;
+    shape.tilesN = (N + hcgemm::kWideN - 1) / hcgemm::kWideN;
+    shape.errFlag = GemmErrorFlag();
+    shape.phase = nullptr;
+    static const bool ready = cudaFuncSetAttribute(GemmBf16PairWideKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::ConfigWide<4>::kSmemBytes) == cudaSuccess;
+    if (!ready) { cudaGetLastError(); HCCL_ERROR("GemmBf16: no shared memory for 256 x 512 tiles"); return HCCL_E_RUNTIME; }
+    // a wave of 74 such tiles loads the fewest panels at 12 rows x 6 columns
+    const int rows = PairGroupRows(K), group = g_forceGm.load() > 0 || rows >= 16 ? rows : 12;
+    cudaLaunchAttribute at[2];
+    const cudaLaunchConfig_t cfg = PairConfig(at, std::min(SwapCapacity(0), shape.tilesM * shape.tilesN), 2, hcgemm::kWideThreads, hcgemm::ConfigWide<4>::kSmemBytes, stream);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, GemmBf16PairWideKernel, tmA, tmB, tmC, shape, group);
+    if (e != cudaSuccess) { HCCL_ERROR("GemmBf16 (256 x 512 tiles) launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
+    return HCCL_SUCCESS;
 }
 
-bool AutotuneEnabled()
+PairTile ChoosePairTile(int M, int N, int K)
 {
-    static const bool on = [] { const char *e = getenv("HCOMM_GEMM_AUTOTUNE"); return e && e[0] == '1'; }();
-    return on;
-}
-
-void PairChoice(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, void *stream, int *bnOut, int *gmOut)
-{
-    const int pairs = PairClusterCapacity();
-    int bn0 = PickPairTileWidth(M / hcgemm::kPairM, N, pairs), gm0 = PairGroupRows(K);
-    // 256 x 512 tiles (a quarter less operand traffic, one accumulator) when N allows and whole waves of them cost at most
-    // 5 % more columns than the best narrower width; a wave of 74 such tiles loads the fewest panels at 12 rows x 6 columns
-    if (N % hcgemm::kWideN == 0 && WideTilesEnabled()) {
-        const long rowBlocks = M / hcgemm::kPairM;
-        const long wide = (rowBlocks * (N / hcgemm::kWideN) + pairs - 1) / pairs * hcgemm::kWideN;
-        const long narrow = (rowBlocks * (N / bn0) + pairs - 1) / pairs * bn0;
-        const int forcedBn = ForcedPairTileWidth();
-        if (forcedBn == hcgemm::kWideN || (forcedBn == 0 && wide * 100 <= narrow * 105)) {
-            *bnOut = hcgemm::kWideN;
-            *gmOut = g_forceGm.load() > 0 ? g_forceGm.load() : (gm0 >= 16 ? 16 : 12);
-            return;
-        }
-    }
-    *bnOut = bn0; *gmOut = gm0;
-    const bool forced = ForcedPairTileWidth() > 0 || g_forceGm.load() > 0;
-    const double flops = 2.0 * M * N * K;
-    if (forced || !AutotuneEnabled() || flops < 2e11) return;
-    const ShapeKey key{M, N, K};
-    {
-        std::lock_guard<std::mutex> lk(g_tuneMu);
-        auto it = g_tuned.find(key);
-        if (it != g_tuned.end()) { *bnOut = it->second.first; *gmOut = it->second.second; return; }
-    }
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing((cudaStream_t)stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { cudaGetLastError(); return; }
-    // candidates: widths whose whole-wave cost is within 15 % of the best, each with the group halved, kept and doubled
-    struct Cand { int bn, gm; float best; };
-    std::vector<Cand> cands;
-    const int rowBlocks = M / hcgemm::kPairM;
-    long bestCost = 0;
-    for (int bn = 256; bn >= 128; bn -= 32) {
-        if (N % bn) continue;
-        const long tiles = (long)rowBlocks * (N / bn), cost = (tiles + pairs - 1) / pairs * bn;
-        if (!bestCost || cost < bestCost) bestCost = cost;
-    }
-    for (int bn = 256; bn >= 128; bn -= 32) {
-        if (N % bn) continue;
-        const long tiles = (long)rowBlocks * (N / bn), cost = (tiles + pairs - 1) / pairs * bn;
-        if (cost * 100 > bestCost * 115) continue;
-        for (int gm : {gm0 / 2, gm0, gm0 * 2})
-            if (gm >= 2 && gm <= 32) cands.push_back({bn, gm, 1e30f});
-    }
-    if (cands.size() < 2) return;
-    // Five rounds over all candidates, two back-to-back launches each; the first round only warms up (module load, L2,
-    // clocks).  Odd rounds walk the list backwards so that a drift over a round does not favour one end of it, and a
-    // candidate's figure is the median of its four counted rounds, not its luckiest one.
-    cudaEvent_t ev[2];
-    if (cudaEventCreate(&ev[0]) != cudaSuccess || cudaEventCreate(&ev[1]) != cudaSuccess) { cudaGetLastError(); return; }
-    bool ok = true;
-    const int nc = (int)cands.size();
-    std::vector<std::vector<float>> samples(nc);
-    for (int round = 0; round < 5 && ok; ++round) {
-        for (int i = 0; i < nc && ok; ++i) {
-            const int ci = (round & 1) ? nc - 1 - i : i;
-            const Cand &cd = cands[ci];
-            cudaEventRecord(ev[0], (cudaStream_t)stream);
-            for (int rep = 0; rep < 2 && ok; ++rep)
-                if (LaunchPairGemm(A, B, C, M, N, K, lda, ldb, ldc, cd.bn, cd.gm, stream) != HCCL_SUCCESS) ok = false;
-            cudaEventRecord(ev[1], (cudaStream_t)stream);
-            if (!ok || cudaEventSynchronize(ev[1]) != cudaSuccess) { cudaGetLastError(); ok = false; break; }
-            float ms = 0;
-            cudaEventElapsedTime(&ms, ev[0], ev[1]);
-            if (round > 0) samples[ci].push_back(ms * 0.5f);
-        }
-    }
-    cudaEventDestroy(ev[0]);
-    cudaEventDestroy(ev[1]);
-    if (!ok) return;
-    for (int i = 0; i < nc; ++i) {
-        std::sort(samples[i].begin(), samples[i].end());
-        cands[i].best = samples[i].empty() ? 1e30f : 0.5f * (samples[i][(samples[i].size() - 1) / 2] + samples[i][samples[i].size() / 2]);
-    }
-    const Cand *win = &cands[0];
-    for (auto &cd : cands)
-        if (cd.best < win->best) win = &cd;
-    HCCL_INFO("GEMM %d x %d x %d: tile width %d, group %d chosen by measurement (%.3f ms; model said %d / %d)", M, N, K, win->bn, win->gm, win->best, bn0, gm0);
-    {
-        std::lock_guard<std::mutex> lk(g_tuneMu);
-        g_tuned[key] = {win->bn, win->gm};
-    }
-    *bnOut = win->bn; *gmOut = win->gm;
+    const int cap[3] = {SwapCapacity(0), SwapCapacity(1), SwapCapacity(2)};
+    PairTile t = PickPairTile(M, N, K, cap);
+    const int bn = ForcedPairTileWidth(), split = g_forceSplit.load(), kBlocks = (K + hcgemm::kBlockK - 1) / hcgemm::kBlockK;
+    if (bn >= hcgemm::kWideN) t = {hcgemm::kWideN, 1};
+    else if (bn > 0) t.bn = std::min(256, std::max(32, bn / 32 * 32));
+    if (t.bn <= 256 && (split == 1 || split == 2 || split == 4) && split <= kBlocks && cap[split / 2] > 0) t.split = split;
+    return t;
 }
 
 }  // namespace
@@ -348,11 +289,12 @@ HcclResult GemmBf16(const void *A, const void *B, void *C, int M, int N, int K, 
         return HCCL_E_PARA;
     }
     static const bool pairEnabled = [] { const char *e = getenv("HCOMM_GEMM_PAIR"); return !(e && e[0] == '0'); }();
-    if (pairEnabled && M % hcgemm::kPairM == 0 && N % 128 == 0 && PairClusterCapacity() > 0) {
-        int bn = 0, gm = 0;
-        PairChoice(A, B, C, M, N, K, lda, ldb, ldc, stream, &bn, &gm);
-        return LaunchPairGemm(A, B, C, M, N, K, lda, ldb, ldc, bn, gm, stream);
+    if (pairEnabled && SwapCapacity(0) > 0) {
+        const PairTile tile = ChoosePairTile(M, N, K);
+        return tile.bn == hcgemm::kWideN ? LaunchWideGemm(A, B, C, M, N, K, lda, ldb, ldc, stream)
+                                         : LaunchSwapGemm(A, B, C, M, N, K, lda, ldb, ldc, tile, stream);
     }
+    // without CTA pairs (HCOMM_GEMM_PAIR=0, or a device that cannot hold a cluster): one CTA per 128-row tile
     const int BN = (N % 256 == 0 || N >= 2048) ? 256 : 128;
     CUtensorMap tmA, tmB;
     CHK_RET(MakeTensorMap2dBf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, hcgemm::kBlockM, hcgemm::kBlockK));
@@ -397,13 +339,24 @@ extern "C" void HcommGemmSetTuning(int groupRows, int tileWidth)
     hc::g_forceGm.store(groupRows > 0 ? groupRows : 0);
     hc::g_forceBn.store(tileWidth > 0 ? tileWidth : 0);
 }
-// Tile width and rasterisation group the measurement at first use chose for a shape (0 / 0: none was made).
-extern "C" void HcommGemmGetTuned(int M, int N, int K, int *tileWidth, int *groupRows)
+// CTA pairs (1, 2 or 4) that share a tile along K; 0 = automatic.
+extern "C" void HcommGemmSetSplit(int pairsAlongK)
 {
-    std::lock_guard<std::mutex> lk(hc::g_tuneMu);
-    auto it = hc::g_tuned.find(hc::ShapeKey{M, N, K});
-    if (tileWidth) *tileWidth = it == hc::g_tuned.end() ? 0 : it->second.first;
-    if (groupRows) *groupRows = it == hc::g_tuned.end() ? 0 : it->second.second;
+    hc::g_forceSplit.store(pairsAlongK);
+}
+// The rule behind the automatic choice, for a device that holds cap1, cap2 and cap4 clusters of 1, 2 and 4 CTA pairs at once.
+extern "C" void HcommToolGemmTile(int M, int N, int K, int cap1, int cap2, int cap4, int *tileWidth, int *pairsAlongK)
+{
+    const int cap[3] = {cap1, cap2, cap4};
+    const hc::PairTile t = hc::PickPairTile(M, N, K, cap);
+    if (tileWidth) *tileWidth = t.bn;
+    if (pairsAlongK) *pairsAlongK = t.split;
+}
+// Kept for callers of earlier versions, which could time a shape at its first use: no measurement is made (0 / 0).
+extern "C" void HcommGemmGetTuned(int, int, int, int *tileWidth, int *groupRows)
+{
+    if (tileWidth) *tileWidth = 0;
+    if (groupRows) *groupRows = 0;
 }
 extern "C" int HcommGemmTakeError(void)
 {

@@ -36,7 +36,7 @@ template <int STAGES = 4> struct ConfigWide {
     static_assert(kSmemBytes <= 227 * 1024, "shared memory per CTA");
 };
 
-// g.tilesM counts 256-row blocks, g.tilesN 512-column blocks; N a multiple of 512.  The B tensor map has 128-row boxes,
+// g.tilesM counts 256-row blocks, g.tilesN 512-column blocks; the edges may be ragged (TMA fills with zeros and clips).  The B tensor map has 128-row boxes,
 // the C tensor map boxes of 32 rows x 64 columns with the 128-byte swizzle.
 template <int STAGES, typename TileOrder>
 __device__ __forceinline__ void GemmMainLoopPairWide(const CUtensorMap *tmA, const CUtensorMap *tmB, const CUtensorMap *tmC, const GemmShape &g, TileOrder order)
@@ -172,7 +172,7 @@ __device__ __forceinline__ void GemmMainLoopPairWide(const CUtensorMap *tmA, con
                 }
                 FenceProxyAsyncShared();                        // my writes, before the copy engine reads them
                 __syncwarp();
-                if (lane == 0) {
+                if (lane == 0 && row0 < g.M && nb * kWideN + c < g.N) {     // the store itself leaves out what lies beyond M and N
                     TmaStore2d(tmC, slab, nb * kWideN + c, row0);
                     TmaStoreCommit();
                 }

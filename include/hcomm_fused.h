@@ -25,11 +25,13 @@ extern "C" {
 
 /* C[M,N] = A[M,K] * B[N,K]^T on the current device.  N, K and ldc multiples of 8, C 16-byte aligned. */
 int HcommGemmBf16(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, void *stream);
-/* Tuning overrides of the CTA-pair GEMM kernels (0 = automatic): rasterisation group in 256-row blocks, tile width (128..256, multiple of 32). */
+/* Tuning overrides of the CTA-pair GEMM kernels (0 = automatic): rasterisation group in 256-row blocks; tile width in rows of A
+ * for the plain GEMM (32..256, rounded down to a multiple of 32; 512: tiles of 256 rows of A x 512 rows of B), in columns for
+ * the fused kernels (128..256, multiple of 32). */
 void HcommGemmSetTuning(int groupRows, int tileWidth);
-/* With HCOMM_GEMM_AUTOTUNE=1, large shapes (2 * M * N * K >= 2e11) seen for the first time are timed once with the candidate
- * tile widths and groups on the caller's stream (not while it is being captured) and the fastest is kept for the process.
- * Returns what was chosen for a shape, 0 / 0 if nothing was measured. */
+/* CTA pairs (1, 2 or 4) that share a tile of the plain GEMM along K; 0 = automatic. */
+void HcommGemmSetSplit(int pairsAlongK);
+/* Kept for callers of earlier versions, which could time a shape at its first use: no measurement is made, always 0 / 0. */
 void HcommGemmGetTuned(int M, int N, int K, int *tileWidth, int *groupRows);
 /* Reads and clears the "a bounded wait expired inside a GEMM kernel" flag of the current device (0 = none). */
 int HcommGemmTakeError(void);

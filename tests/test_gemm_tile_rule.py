@@ -1,0 +1,41 @@
+"""The rule that picks the plain GEMM's tile, on the CPU: every shape gets a tile that the kernels take."""
+import ctypes
+
+import pytest
+
+from hcomm_b200 import _lib
+
+CAPS = [(74, 33, 15), (74, 0, 0), (8, 4, 2), (1, 0, 0)]
+
+
+def pick(m, n, k, caps):
+    bn, split = ctypes.c_int(), ctypes.c_int()
+    _lib.load().HcommToolGemmTile(m, n, k, *caps, ctypes.byref(bn), ctypes.byref(split))
+    return bn.value, split.value
+
+
+@pytest.mark.parametrize("caps", CAPS)
+def test_every_shape_gets_a_tile_that_the_kernel_takes(caps):
+    sizes = [8, 64, 72, 136, 256, 264, 1000, 1024, 3584, 4096, 5000, 8192, 28672, 128256]
+    for m in [1, 2, 15, 31, 32, 33, 64, 65, 96, 127, 128, 200, 255, 256, 257, 300, 777, 1024, 5003, 8192, 100000]:
+        for n in sizes:
+            for k in sizes:
+                bn, split = pick(m, n, k, caps)
+                assert split in (1, 2, 4) and (split == 1 or caps[split // 2] > 0), (m, n, k, split)
+                if bn == 512:
+                    assert split == 1
+                    continue
+                assert 32 <= bn <= 256 and bn % 32 == 0, (m, n, k, bn)
+                assert bn - 32 < m, "a tile with a whole step of empty columns"
+                assert split == 1 or (k + 63) // 64 >= 4 * split, "a part of K that is hardly a step"
+
+
+def test_known_choices():
+    caps = (74, 33, 15)
+    assert pick(16, 8192, 28672, caps) == (32, 2)       # 32 tiles: two pairs each, so that enough SMs ask for the weights
+    assert pick(16, 28672, 8192, caps) == (32, 1)       # 112 tiles keep the chip busy as they are
+    assert pick(96, 3584, 8192, caps) == (96, 4)        # 14 tiles, a deep K
+    assert pick(33, 128256, 4096, caps) == (64, 1)      # one tile across all tokens: every weight is fetched once
+    assert pick(8192, 28672, 8192, caps) == (512, 1)    # 25 full waves: the least operand traffic
+    assert pick(777, 14336, 4096, caps) == (160, 1)     # 800 columns of work for 777 tokens
+    assert pick(8192, 3584, 8192, caps) == (224, 1)     # seven full waves instead of eight of 256 columns

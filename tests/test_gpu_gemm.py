@@ -54,3 +54,32 @@ def test_wide_tile_kernel_matches_fp32_reference(m, n, k, group):
     err = (out.float() - ref).abs().max().item()
     assert err <= 1e-2 * max(ref.abs().max().item(), 1.0), f"max abs err {err}"
     assert out_full[:, n:].abs().max().item() == 0
+
+
+@pytest.mark.parametrize("width,split", [(32, 1), (32, 4), (96, 1), (96, 2), (224, 1), (224, 4), (256, 1), (256, 2), (256, 4), (512, 1)])
+@pytest.mark.parametrize("m,n,k", [(1, 136, 264), (33, 264, 512), (200, 1000, 520), (257, 776, 1032), (700, 2048, 320)])
+def test_gemm_tiles_and_parts_of_k(m, n, k, width, split):
+    # rows and columns around the edges of the tiles, K not a multiple of the 64-wide step or of the parts of a split,
+    # a result inside a wider matrix whose other columns must stay as they are, and bit-equal results from run to run
+    from hcomm_b200 import _lib
+    from hcomm_b200.ops.gemm import gemm_bf16, take_kernel_error
+    lib = _lib.load()
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(n, k, device="cuda") * 0.05).to(torch.bfloat16)
+    full = torch.full((2, m, n + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    lib.HcommGemmSetTuning(0, width)
+    lib.HcommGemmSetSplit(split)
+    try:
+        for i in range(2):
+            gemm_bf16(a, b, full[i][:, :n])
+        torch.cuda.synchronize()
+    finally:
+        lib.HcommGemmSetTuning(0, 0)
+        lib.HcommGemmSetSplit(0)
+    assert take_kernel_error() == 0
+    assert torch.equal(full[0], full[1]) and bool((full[:, :, n:] == 7.0).all())
+    ref = a.double() @ b.double().t()
+    # one rounding to bf16 (half a step, 2^-9) and fp32 sums of k products (k * 2^-24 of the sum of magnitudes)
+    bound = 2.0 ** -8 * ref.abs() + k * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t())
+    assert bool(((full[0][:, :n].double() - ref).abs() <= bound).all())
