@@ -69,6 +69,7 @@ __device__ __forceinline__ void GemmMainLoopPairWide(const CUtensorMap *tmA, con
         TmemAlloc2(&st->tmemBase, Cfg::kTmemCols);
         TmemRelinquish2();
     }
+    GridDependentsLaunch();
     TcFenceBefore();
     __syncthreads();
     ClusterSync();
@@ -80,6 +81,7 @@ __device__ __forceinline__ void GemmMainLoopPairWide(const CUtensorMap *tmA, con
         if (ElectOne()) {
             uint32_t it = 0;
             bool alive = true;
+            GridDependencyWait();           // up to here a CTA may run beside the tail of the kernel in front; all it writes follows its loads
             for (int t = firstTile; t < numTiles && alive; t += tileStep) {
                 int mb, nb;
                 order(t, g, &mb, &nb);

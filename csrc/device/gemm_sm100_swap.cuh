@@ -114,6 +114,7 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
         TmemAlloc2(&st->tmemBase, 512);
         TmemRelinquish2();
     }
+    GridDependentsLaunch();
     TcFenceBefore();
     __syncthreads();
     ClusterSync();          // every barrier of the cluster is initialised before anything signals it
@@ -126,6 +127,7 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
             int s = 0;
             uint32_t ph = 0;
             bool alive = true;
+            GridDependencyWait();           // up to here a CTA may run beside the tail of the kernel in front; all it writes follows its loads
             for (int t = firstTile; t < numTiles && alive; t += tileStep) {
                 int wb, tb;
                 order(t, &wb, &tb);

@@ -28,6 +28,12 @@ __device__ __forceinline__ bool ElectOne()
     return pred != 0;
 }
 
+// Programmatic dependent launch (a launch with the stream-serialization attribute; without it both do nothing).  Wait: until
+// the grids in front have completed and their writes are visible - before the first access to memory that they may touch.
+// Launch: the grid behind may start to take the SMs that this one leaves; its own Wait still holds it back from memory.
+__device__ __forceinline__ void GridDependencyWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void GridDependentsLaunch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------------- mbarrier
 
 __device__ __forceinline__ void MbarInit(uint64_t *bar, uint32_t count)

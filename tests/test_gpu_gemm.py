@@ -83,3 +83,30 @@ def test_gemm_tiles_and_parts_of_k(m, n, k, width, split):
     # one rounding to bf16 (half a step, 2^-9) and fp32 sums of k products (k * 2^-24 of the sum of magnitudes)
     bound = 2.0 ** -8 * ref.abs() + k * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t())
     assert bool(((full[0][:, :n].double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("m,h,i", [(16, 1024, 4096), (300, 1024, 2048), (2048, 8192, 8192)])
+def test_back_to_back_calls_see_each_others_results(m, h, i):
+    # a chain in which every call reads what the call in front wrote and overwrites what it read: the launches overlap,
+    # the accesses must not
+    from hcomm_b200.ops.gemm import gemm_bf16, take_kernel_error
+    torch.manual_seed(m)
+    up = (torch.randn(i, h, device="cuda") / h ** 0.5).to(torch.bfloat16)
+    down = (torch.randn(h, i, device="cuda") / i ** 0.5).to(torch.bfloat16)
+    x0 = torch.randn(m, h, device="cuda").to(torch.bfloat16)
+
+    def chain(wait):
+        x, y = x0.clone(), torch.empty(m, i, device="cuda", dtype=torch.bfloat16)
+        for _ in range(6):
+            gemm_bf16(x, up, y)
+            if wait:
+                torch.cuda.synchronize()
+            gemm_bf16(y, down, x)
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return x
+    want = chain(True)
+    for _ in range(3):
+        assert torch.equal(chain(False), want)
+    assert take_kernel_error() == 0
