@@ -10,15 +10,17 @@
 //                     one cross-rank barrier, the per-expert offsets of this rank's own experts for its grouped GEMM
 //   dispatch (N CTAs) every CTA reads the owners' count tables and derives, for each expert, where this rank's rows
 //                     start in the owner's receive buffer (rows are grouped by expert, inside an expert by source rank);
-//                     one warp per token: load 7168 bf16, per 128-value block absmax -> scale -> e4m3, lanes 0..k-1
-//                     claim the rows of the token's k experts in parallel (local atomics), then the k rows, scales and
-//                     origins leave back to back; each CTA ends with one cross-rank barrier with its namesakes
-// Combine, rank r (owner of experts) - two ordinary launches:
-//   send  one warp per received row: the bf16 expert output goes to slot (token, k) of the token's rank; cross-rank barrier
-//   sum   one warp per local token: out = sum_k gate[k] * slot(token, k) over the k that were sent, fp32 accumulation
+//                     the CTA's threads claim the rows of its tokens' experts in parallel (atomics on the row cursors),
+//                     then its warps quantise 512 values of a token at a time and store them to the token's k rows;
+//                     each CTA ends with one cross-rank barrier with its namesakes
+// Combine, rank r (owner of experts) - two ordinary launches, one when there is a single rank:
+//   send  one warp per row received from ANOTHER rank: the bf16 expert output goes to slot (token, k) of the token's rank;
+//         cross-rank barrier
+//   sum   out = sum_k gate[k] * row(token, k) over the k that were sent, fp32 accumulation in the order of k; a row whose
+//         expert lives on the token's own rank is read where the expert wrote it (dispatch noted which row that is)
 //
 // Device scratch (beyond inputs and outputs): numExperts u32 row cursors (second half of a 2 * numExperts table), cleared
-// by the route launch.
+// by the route launch; the local row of every (token, k).
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -58,7 +60,13 @@ struct MoeParams {
     const float *gates;
     __nv_bfloat16 *out;
     uint32_t *overflow;                   // device word: rows that did not fit the receive capacity
+    uint32_t *localRow;                   // [maxTokens * topk]: row of (token, k) in this rank's receive buffer, kNoRow when it went elsewhere
+    int segsPerItem;                      // sum: 256-column segments that a warp takes at a time
+    int countsLaunch;                     // sum: this launch is the whole operator (single rank) and advances the launch state
 };
+constexpr uint32_t kNoRow = 0xffffffffu;
+
+#define MOE_ARGS const MoeParams &p = (table != nullptr) ? table[blockIdx.y] : byval
 
 __device__ __forceinline__ uint32_t *Counts(const MoeParams &p, int rank) { return (uint32_t *)(p.peerBuf[rank] + p.lay.offCounts); }
 __device__ __forceinline__ uint8_t *Rows(const MoeParams &p, int rank) { return (uint8_t *)(p.peerBuf[rank] + p.lay.offRows); }
@@ -70,167 +78,216 @@ __device__ __forceinline__ __nv_bfloat16 *Comb(const MoeParams &p, int rank) { r
 // (masked) or the owner's receive capacity was exhausted; combine leaves such rows out of the sum
 __device__ __forceinline__ uint8_t *Valid(const MoeParams &p, int rank) { return (uint8_t *)(p.peerBuf[rank] + p.lay.offValid); }
 
-// Dispatch, first launch (one CTA per rank): routing histogram, counts published to the experts' owners, one cross-rank
-// barrier, the offsets of this rank's own experts, row cursors cleared for the second launch.
-__global__ void __launch_bounds__(1024) MoeRouteKernel(const MoeParams *table)
+// Streamed once, not worth a line of L1.  Data that peers wrote has landed in this GPU's memory before the kernel began.
+__device__ __forceinline__ uint4 LdStream16(const void *p)
 {
-    const MoeParams &p = table[blockIdx.y];
+    uint4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+// Exclusive prefix sums of v over the CTA's threads (a multiple of 32, at most 1024); warpSums: one word per warp.
+__device__ __forceinline__ uint32_t BlockExclusiveScan(uint32_t v, uint32_t *warpSums)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) warpSums[warp] = x;
+    __syncthreads();
+    uint32_t below = 0;
+    for (int w = 0; w < warps; ++w) below += w < warp ? warpSums[w] : 0u;
+    return below + x - v;
+}
+
+// Dispatch, first launch (one CTA per rank): routing histogram, counts published to the experts' owners, one cross-rank
+// barrier, the offsets of this rank's own experts, row cursors cleared for the second launch.  Bound by latency and by
+// shared-memory atomics: 32768 choices 10.5 us (28 with one histogram and a serial prefix), 512 choices 6 (12).
+__global__ void __launch_bounds__(1024) MoeRouteKernel(const __grid_constant__ MoeParams byval, const MoeParams *table)
+{
+    MOE_ARGS;
     const CommDev *d = p.dev;
     const LaunchState ls = KernelBegin(d);
     const int n = d->nRanks, me = d->rank;
     const int E = p.lay.numExperts, El = E / n, K = p.lay.topk;
     const int tid = threadIdx.x;
-    __shared__ uint32_t sHist[kMaxExperts], sTot[kMaxExperts];
+    // four histograms, warps dealt over them: neighbouring lanes often hold the same expert and would queue for its counter
+    __shared__ uint32_t sHist[4][kMaxExperts], sWarp[32];
     uint32_t *cursor = p.scratch + E;
-    for (int e = tid; e < E; e += blockDim.x) { sHist[e] = 0; cursor[e] = 0; }
-    __syncthreads();
-    for (int i = tid; i < p.numTokens * K; i += blockDim.x) {
-        int e = p.topkIdx[i];
-        if (e >= 0 && e < E) atomicAdd(&sHist[e], 1u);
+    for (int e = tid; e < E; e += blockDim.x) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) sHist[h][e] = 0;
+        cursor[e] = 0;
     }
     __syncthreads();
-    for (int e = tid; e < E; e += blockDim.x) Counts(p, e / El)[me * El + (e % El)] = sHist[e];
-    CrossRankBarrier(d, ls.epoch0 + 1);
+    uint32_t *hist = sHist[(tid >> 5) & 3];
+    const int total = p.numTokens * K, stride = blockDim.x;
+    for (int i = tid; i < total; i += 8 * stride) {         // eight loads in flight
+        int e[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) e[u] = i + u * stride < total ? p.topkIdx[i + u * stride] : -1;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (e[u] >= 0 && e[u] < E) atomicAdd(&hist[e[u]], 1u);
+    }
+    __syncthreads();
+    for (int e = tid; e < E; e += blockDim.x) Counts(p, e / El)[me * El + (e % El)] = sHist[0][e] + sHist[1][e] + sHist[2][e] + sHist[3][e];
+    if (n > 1) CrossRankBarrier(d, ls.epoch0 + 1);
+    else __syncthreads();
     // the offsets of my own experts for the grouped GEMM that follows (the table may be overwritten by a peer's next
     // dispatch as soon as the second launch's barrier is passed, so derive them now): one thread per local expert sums
-    // its column, thread 0 turns the sums into a prefix
-    for (int el = tid; el < El; el += blockDim.x) {
+    // its column.  Every entry is clamped to the receive capacity: a grouped GEMM that walks [off[el], off[el + 1]) never
+    // leaves the buffer.
+    uint32_t sum = 0;
+    if (tid < El) {
         const volatile uint32_t *c = Counts(p, me);
-        uint32_t sum = 0;
-        for (int s = 0; s < n; ++s) sum += c[s * El + el];
-        sTot[el] = sum;
+        for (int s = 0; s < n; ++s) sum += c[s * El + tid];
     }
-    __syncthreads();
-    if (tid == 0) {
-        // every entry is clamped to the receive capacity: a grouped GEMM that walks [off[el], off[el + 1]) never leaves the buffer
-        const uint32_t capRows = (uint32_t)p.lay.maxRecvRows;
-        uint32_t acc = 0;
-        uint32_t *off = ExpertOffsets(p, me);
-        for (int el = 0; el < El; ++el) {
-            off[el] = acc < capRows ? acc : capRows;
-            acc += sTot[el];
-        }
-        off[El] = acc < capRows ? acc : capRows;
-    }
+    const uint32_t before = BlockExclusiveScan(sum, sWarp), capRows = (uint32_t)p.lay.maxRecvRows;
+    uint32_t *off = ExpertOffsets(p, me);
+    if (tid < El) off[tid] = before < capRows ? before : capRows;
+    if (tid == El - 1) off[El] = before + sum < capRows ? before + sum : capRows;
     KernelEnd(d, ls, 1, 0);
 }
 
 // Dispatch, second launch (any number of CTAs, an ordinary launch that can share the GPU with expert GEMMs): every CTA
-// derives from the owners' count tables where this rank's rows of each expert start, then quantises and sends its
-// tokens, one warp per token, and meets its namesakes on the other ranks once all of its rows are on their way.
-__global__ void __launch_bounds__(512) MoeDispatchKernel(const MoeParams *table)
+// derives from the owners' count tables where this rank's rows of each expert start, claims the rows of its tokens, then
+// quantises and sends them, and meets its namesakes on the other ranks once all of its rows are on their way.
+// Bound by memory and, about as much, by the instructions of 16 divisions and k stores per 32 bytes: 4096 x 7168 to 8 experts
+// each take 69 us (86 with one warp per token), 46 at HBM rate; 64 tokens 9 us (39).  A CTA owns whole tokens and its 16 warps share them in
+// pieces of 512 values, so that few tokens still occupy many warps and the claims cost one round of atomics per CTA, not one
+// per token.
+constexpr int kClaims = 512;           // (token, k) pairs that a CTA claims at a time: one per thread
+__global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constant__ MoeParams byval, const MoeParams *table)
 {
-    const MoeParams &p = table[blockIdx.y];
+    MOE_ARGS;
     const CommDev *d = p.dev;
     const LaunchState ls = KernelBegin(d);
     const int n = d->nRanks, me = d->rank;
     const int E = p.lay.numExperts, El = E / n, K = p.lay.topk, H = p.lay.hidden;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int warpsPerCta = blockDim.x >> 5;
-    __shared__ uint32_t sBase[kMaxExperts], sTot[kMaxExperts];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    __shared__ uint32_t sBase[kMaxExperts], sWarp[16];
+    __shared__ uint8_t *sRow[kClaims];
+    __shared__ float *sScale[kClaims];
     uint32_t *cursor = p.scratch + E;
+    const int t0 = (int)((int64_t)p.numTokens * blockIdx.x / gridDim.x), t1 = (int)((int64_t)p.numTokens * (blockIdx.x + 1) / gridDim.x);
+    const int segs = H / 512, perRound = kClaims / K;
+
+    // the first piece of this warp is on its way while the rows are being found
+    uint4 a = make_uint4(0, 0, 0, 0), b = a;
+    const int firstItems = (t1 - t0 < perRound ? t1 - t0 : perRound) * segs;
+    if (warp < firstItems) {
+        const __nv_bfloat16 *src = p.x + (size_t)t0 * H + (size_t)warp * 512 + lane * 16;     // pieces of consecutive tokens are consecutive in x
+        a = LdStream16(src); b = LdStream16(src + 8);
+    }
 
     // where do my rows of expert e start at its owner?  before them: all rows of the owner's earlier experts,
-    // and the rows of this expert that come from lower ranks.  One thread per expert fetches that expert's n
-    // counts from the owner (independent loads, one NVLink round trip), then the prefix runs on shared memory.
-    for (int e = tid; e < E; e += blockDim.x) {
-        const int owner = e / El, el = e % El;
-        const volatile uint32_t *c = Counts(p, owner);
-        uint32_t total = 0, below = 0;
-        for (int s = 0; s < n; ++s) {
-            const uint32_t v = c[s * El + el];
-            total += v;
-            if (s < me) below += v;
+    // and the rows of this expert that come from lower ranks.  Every thread fetches the n counts of two experts
+    // from their owner (independent loads, one NVLink round trip), then the prefix runs inside the CTA.
+    {
+        uint32_t tot[2] = {0, 0}, below[2] = {0, 0};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int e = 2 * tid + j;
+            if (e < E) {
+                const volatile uint32_t *c = Counts(p, e / El) + e % El;
+                for (int s = 0; s < n; ++s) {
+                    const uint32_t v = c[s * El];
+                    tot[j] += v;
+                    if (s < me) below[j] += v;
+                }
+            }
         }
-        sTot[e] = total;
-        sBase[e] = below;
+        const uint32_t before = BlockExclusiveScan(tot[0] + tot[1], sWarp);
+        if (2 * tid < E) sBase[2 * tid] = before;
+        if (2 * tid + 1 < E) sBase[2 * tid + 1] = before + tot[0];
+        __syncthreads();
+        uint32_t base[2] = {0, 0};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int e = 2 * tid + j;
+            if (e < E) base[j] = sBase[e] - sBase[e / El * El] + below[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            if (2 * tid + j < E) sBase[2 * tid + j] = base[j];
+        __syncthreads();
     }
-    __syncthreads();
-    for (int e = tid; e < E; e += blockDim.x) {
-        const int first = (e / El) * El;
-        uint32_t base = 0;
-        for (int e2 = first; e2 < e; ++e2) base += sTot[e2];
-        sBase[e] += base;       // only this thread touches sBase[e]; sTot is read-only here
-    }
-    __syncthreads();
 
-    // quantise and send, one warp per token
-    const int chunks = H / 16;                       // 16 values (32 bytes in, 16 bytes out) per lane step
-    const int blocksPerRow = H / kBlock;
-    for (int t = blockIdx.x * warpsPerCta + warp; t < p.numTokens; t += gridDim.x * warpsPerCta) {
-        // lane k claims the row of the token's k-th expert while the other lanes already load the token
-        int myExpert = -1;
-        uint32_t mySlot = 0xffffffffu;
-        if (lane < K) {
-            myExpert = p.topkIdx[t * K + lane];
-            if (myExpert >= 0 && myExpert < E) {
-                mySlot = sBase[myExpert] + atomicAdd(&cursor[myExpert], 1u);
-                if (mySlot >= (uint32_t)p.lay.maxRecvRows) { atomicAdd(p.overflow, 1u); mySlot = 0xffffffffu; }
+    for (int r0 = t0; r0 < t1; r0 += perRound) {
+        const int tokens = t1 - r0 < perRound ? t1 - r0 : perRound;
+        if (tid < tokens * K) {
+            const size_t tk = (size_t)r0 * K + tid;
+            const int e = p.topkIdx[tk];
+            uint32_t slot = kNoRow, local = kNoRow;
+            if (e >= 0 && e < E) {
+                slot = sBase[e] + atomicAdd(&cursor[e], 1u);
+                if (slot >= (uint32_t)p.lay.maxRecvRows) { atomicAdd(p.overflow, 1u); slot = kNoRow; }
             }
-            Valid(p, me)[t * K + lane] = mySlot != 0xffffffffu ? 1 : 0;
+            Valid(p, me)[tk] = slot != kNoRow ? 1 : 0;
+            sRow[tid] = nullptr;
+            if (slot != kNoRow) {
+                const int owner = e / El;
+                sRow[tid] = Rows(p, owner) + (size_t)slot * H;
+                sScale[tid] = Scales(p, owner) + (size_t)slot * (H / kBlock);
+                Origin(p, owner)[slot] = ((uint64_t)me << 32) | (uint32_t)tk;
+                if (owner == me) local = slot;
+            }
+            p.localRow[tk] = local;
         }
-        const __nv_bfloat16 *src = p.x + (size_t)t * H;
-        uint4 q[16];                                 // up to 16 chunks per lane: hidden <= 8192; fully unrolled so that they stay in registers
-        float sc[16];
+        __syncthreads();
+        const int items = tokens * segs;
+        const __nv_bfloat16 *src = p.x + (size_t)r0 * H + lane * 16;
+        if (r0 != t0 && warp < items) { a = LdStream16(src + (size_t)warp * 512); b = LdStream16(src + (size_t)warp * 512 + 8); }
+        for (int it = warp; it < items; it += warps) {
+            const uint4 ca = a, cb = b;
+            if (it + warps < items) { a = LdStream16(src + (size_t)(it + warps) * 512); b = LdStream16(src + (size_t)(it + warps) * 512 + 8); }
+            // the largest magnitude of the lane's 16 values (a maximum of bf16 values is exact in bf16)
+            const uint4 cur[2] = {ca, cb};
+            const __nv_bfloat162 *x2 = (const __nv_bfloat162 *)cur;
+            __nv_bfloat162 m2 = __habs2(x2[0]);
 #pragma unroll
-        for (int nq = 0; nq < 16; ++nq) {
-            const int c = lane + 32 * nq;
-            if (c >= chunks) break;
-            const uint4 a = *(const uint4 *)(src + c * 16), b = *(const uint4 *)(src + c * 16 + 8);
-            float v[16];
-            const __nv_bfloat162 *pa = (const __nv_bfloat162 *)&a, *pb = (const __nv_bfloat162 *)&b;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float2 fa = __bfloat1622float2(pa[j]), fb = __bfloat1622float2(pb[j]);
-                v[2 * j] = fa.x; v[2 * j + 1] = fa.y; v[8 + 2 * j] = fb.x; v[8 + 2 * j + 1] = fb.y;
-            }
-            float amax = 0.f;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(v[j]));
+            for (int j = 1; j < 8; ++j) m2 = __hmax2(m2, __habs2(x2[j]));
+            float amax = fmaxf(0.f, fmaxf(__low2float(m2), __high2float(m2)));
             // the 8 lanes that share a 128-value block sit next to each other
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
             const float scale = fmaxf(amax, 1e-4f) / 448.0f;   // values are divided (not multiplied by a reciprocal): bit-exact with x / scale
-            sc[nq] = scale;
             uint32_t w[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * j] / scale, v[4 * j + 1] / scale), __NV_SATFINITE, __NV_E4M3);
-                __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * j + 2] / scale, v[4 * j + 3] / scale), __NV_SATFINITE, __NV_E4M3);
+                const float2 f0 = __bfloat1622float2(x2[2 * j]), f1 = __bfloat1622float2(x2[2 * j + 1]);
+                const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(f0.x / scale, f0.y / scale), __NV_SATFINITE, __NV_E4M3);
+                const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(f1.x / scale, f1.y / scale), __NV_SATFINITE, __NV_E4M3);
                 w[j] = (uint32_t)lo | ((uint32_t)hi << 16);
             }
-            q[nq] = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-        // the token's rows leave back to back: nothing but stores between the first and the last
-        for (int k = 0; k < K; ++k) {
-            const int e = __shfl_sync(0xffffffffu, myExpert, k);
-            const uint32_t slot = __shfl_sync(0xffffffffu, mySlot, k);
-            if (slot == 0xffffffffu) continue;
-            const int owner = e / El;
-            uint8_t *row = Rows(p, owner) + (size_t)slot * H;
-            float *srow = Scales(p, owner) + (size_t)slot * blocksPerRow;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int c = lane + 32 * i;
-                if (c >= chunks) break;
-                *(uint4 *)(row + c * 16) = q[i];
-                if ((lane & 7) == 0) srow[c / 8] = sc[i];
+            const uint4 q = make_uint4(w[0], w[1], w[2], w[3]);
+            const int tok = it / segs, seg = it - tok * segs, c0 = tok * K;
+            for (int k = 0; k < K; ++k) {
+                uint8_t *row = sRow[c0 + k];
+                if (!row) continue;
+                *(uint4 *)(row + seg * 512 + lane * 16) = q;
+                if ((lane & 7) == 0) sScale[c0 + k][seg * 4 + (lane >> 3)] = scale;
             }
-            if (lane == 0) Origin(p, owner)[slot] = ((uint64_t)me << 32) | (uint32_t)(t * K + k);
         }
+        __syncthreads();        // the claims of the next round overwrite these
     }
     // all rows of this CTA are on their way; once every local CTA has passed its barrier (= the kernel has ended) all
     // CTAs of all ranks have sent
-    CrossRankBarrier(d, ls.epoch0 + 1);
+    if (n > 1) CrossRankBarrier(d, ls.epoch0 + 1);
     KernelEnd(d, ls, 1);
 }
 
-// Combine, first launch: every expert output row goes home, into slot (token, k) of the token's rank; each CTA then
-// meets its namesakes on the other ranks.  When the kernel has ended on a rank, every rank's rows for it have landed.
-__global__ void __launch_bounds__(512) MoeCombineSendKernel(const MoeParams *table)
+// Combine, first launch: every expert output row of another rank's token goes home, into slot (token, k) of that rank; each
+// CTA then meets its namesakes on the other ranks.  When the kernel has ended on a rank, every rank's rows for it have landed.
+__global__ void __launch_bounds__(512) MoeCombineSendKernel(const __grid_constant__ MoeParams byval, const MoeParams *table)
 {
-    const MoeParams &p = table[blockIdx.y];
+    MOE_ARGS;
     const CommDev *d = p.dev;
     const LaunchState ls = KernelBegin(d);
     const int n = d->nRanks, me = d->rank;
@@ -241,6 +298,7 @@ __global__ void __launch_bounds__(512) MoeCombineSendKernel(const MoeParams *tab
     for (int r = blockIdx.x * warpsPerCta + warp; r < rows; r += gridDim.x * warpsPerCta) {
         const uint64_t o = Origin(p, me)[r];
         const int src = (int)(o >> 32);
+        if (src == me) continue;                     // the sum reads it where it is
         const uint32_t tk = (uint32_t)o;
         const uint4 *in = (const uint4 *)(p.y + (size_t)r * H);
         uint4 *dst = (uint4 *)(Comb(p, src) + (size_t)tk * H);
@@ -259,41 +317,56 @@ __global__ void __launch_bounds__(512) MoeCombineSendKernel(const MoeParams *tab
     KernelEnd(d, ls, 1);
 }
 
-// Combine, second launch (local): gate-weighted sum of the K landing slots of every local token, fp32 accumulation.
-__global__ void __launch_bounds__(512) MoeCombineSumKernel(const MoeParams *table)
+// Combine, second launch (local): gate-weighted sum of the K rows of every local token, fp32 accumulation in the order of k.
+// Bound by memory: 2 k H bytes in, 2 H out per token; 3001 x 7168, 8 experts each, a tenth masked, 75 us (205 with every row
+// copied to its slot first), 54 at HBM rate; 64 tokens 7 us (13 + 43).  A warp takes segsPerItem segments of 256 columns of a token; lane k
+// finds the k-th row's address, and every lane keeps the loads of eight rows of a segment in flight.
+constexpr int kSumThreads = 256, kSumCtasPerSm = 3;     // 85 registers a thread: eight addresses and gates of rows beside their loads
+__global__ void __launch_bounds__(kSumThreads, kSumCtasPerSm) MoeCombineSumKernel(const __grid_constant__ MoeParams byval, const MoeParams *table)
 {
-    const MoeParams &p = table[blockIdx.y];
-    const int me = p.dev->rank;
-    const int K = p.lay.topk, H = p.lay.hidden;
+    MOE_ARGS;
+    const CommDev *d = p.dev;
+    LaunchState ls = {};
+    if (p.countsLaunch) ls = KernelBegin(d);
+    const int me = d->rank, K = p.lay.topk, H = p.lay.hidden;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warpsPerCta = blockDim.x >> 5;
-    const int vecs = H / 8;
-    for (int t = blockIdx.x * warpsPerCta + warp; t < p.numTokens; t += gridDim.x * warpsPerCta) {
-        float g[16];
-        bool live[16];
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            live[k] = k < K && Valid(p, me)[t * K + k] != 0;
-            g[k] = live[k] ? p.gates[t * K + k] : 0.f;
+    const int segs = H / 256, perToken = (segs + p.segsPerItem - 1) / p.segsPerItem;
+    const int items = p.numTokens * perToken;
+    for (int it = blockIdx.x * warpsPerCta + warp; it < items; it += gridDim.x * warpsPerCta) {
+        const int t = it / perToken, seg0 = (it - t * perToken) * p.segsPerItem;
+        const int seg1 = seg0 + p.segsPerItem < segs ? seg0 + p.segsPerItem : segs;
+        uint64_t mine = 0;                          // address of row (t, lane); zero when nothing was sent: the slot then holds an older step's row
+        float myGate = 0.f;
+        if (lane < K) {
+            const size_t tk = (size_t)t * K + lane;
+            const uint32_t row = p.localRow[tk];
+            if (row != kNoRow) mine = (uint64_t)(p.y + (size_t)row * H);
+            else if (Valid(p, me)[tk] != 0) mine = (uint64_t)(Comb(p, me) + tk * H);
+            myGate = p.gates[tk];
         }
-        for (int v = lane; v < vecs; v += 32) {
+        const uint32_t live = __ballot_sync(0xffffffffu, mine != 0);
+        for (int seg = seg0; seg < seg1; ++seg) {
+            const uint32_t col = seg * 512 + lane * 16;         // bytes
             float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            // eight rows of this column at a time: eight independent loads in flight (fully unrolled: registers, not local memory)
 #pragma unroll
             for (int kb = 0; kb < 16; kb += 8) {
                 if (kb >= K) break;
                 uint4 pk[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    if (live[kb + k]) pk[k] = Ld16Volatile((const char *)(Comb(p, me) + ((size_t)t * K + kb + k) * H) + (size_t)v * 16);
+                for (int k = 0; k < 8; ++k) {
+                    const uint64_t row = __shfl_sync(0xffffffffu, mine, kb + k);
+                    if (live >> (kb + k) & 1u) pk[k] = LdStream16((const char *)row + col);
+                }
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
-                    if (!live[kb + k]) continue;            // nothing was sent for this (token, k): the slot holds an older step's row
+                    const float g = __shfl_sync(0xffffffffu, myGate, kb + k);
+                    if (!(live >> (kb + k) & 1u)) continue;
                     const __nv_bfloat162 *ph = (const __nv_bfloat162 *)&pk[k];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         float2 f = __bfloat1622float2(ph[j]);
-                        acc[2 * j] += g[kb + k] * f.x;
-                        acc[2 * j + 1] += g[kb + k] * f.y;
+                        acc[2 * j] += g * f.x;
+                        acc[2 * j + 1] += g * f.y;
                     }
                 }
             }
@@ -304,9 +377,10 @@ __global__ void __launch_bounds__(512) MoeCombineSumKernel(const MoeParams *tabl
                 __nv_bfloat162 h = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
                 pw[j] = *(uint32_t *)&h;
             }
-            *(uint4 *)((char *)(p.out + (size_t)t * H) + (size_t)v * 16) = outv;
+            *(uint4 *)((char *)(p.out + (size_t)t * H) + col) = outv;
         }
     }
+    if (p.countsLaunch) KernelEnd(d, ls, 1);
 }
 
 struct MoeCtx {
@@ -319,47 +393,64 @@ struct MoeCtx {
     uint32_t *staticScratch = nullptr;   // device address of the built-in counter table on this exchange's GPU
     int device = -1;                     // the GPU this exchange was created on
     uint32_t *overflow = nullptr;
-    MoeParams *devParams = nullptr;
-    int nextParam = 0;
+    uint32_t *localRow = nullptr;        // [maxTokens * topk], see MoeParams
 };
 std::mutex g_mu;
 std::map<void *, MoeCtx *> g_ctx;
 
 uint64_t Align256(uint64_t v) { return (v + 255) & ~255ull; }
 
-// CTAs of the data-moving launches: all SMs unless HCOMM_MOE_CTAS leaves some to kernels running beside them.
-int MoeCtas(int sms)
+// HCOMM_MOE_CTAS: CTAs of the data-moving launches, to leave SMs to kernels running beside them (0 = not set).
+int ForcedMoeCtas()
 {
-    static const int forced = [] { const char *e = getenv("HCOMM_MOE_CTAS"); return e ? atoi(e) : 0; }();
-    return forced > 0 ? std::min(forced, HC_MAX_CTAS) : std::min(sms, HC_MAX_CTAS);
+    static const int forced = [] { const char *e = getenv("HCOMM_MOE_CTAS"); return e ? std::max(0, atoi(e)) : 0; }();
+    return std::min(forced, HC_MAX_CTAS);
 }
-
-// One launch of `kernel` with `ctas` CTAs of `threads` threads (ctas <= 0: the data-moving default).  Ordinary launches:
-// nothing in these kernels waits for another CTA of the same launch.  Ranks that share a GPU (tests) are merged into one
-// cooperative launch, because their kernels wait for each other.
-HcclResult LaunchMoe(MoeCtx *m, void *kernel, const MoeParams &hp, int id, void *stream, int ctas = 0, int threads = 512)
+int MoeSms()
 {
-    Comm *c = m->comm;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+// CTAs of a launch that meets its namesakes on the other ranks: the same number on every rank, whatever it has to do.  A
+// single rank meets nobody: two CTAs per SM, no more than there is work for.
+int MoeCtas(const Comm *c, int sms, int64_t useful)
+{
+    const int forced = ForcedMoeCtas();
+    if (c->nRanks > 1) return forced > 0 ? forced : std::min(sms, HC_MAX_CTAS);
+    return (int)std::max<int64_t>(1, std::min<int64_t>(forced > 0 ? forced : 2 * sms, useful));
+}
+
+// One launch of `kernel` with `ctas` CTAs of `threads` threads.  Ordinary launches: nothing in these kernels waits for
+// another CTA of the same launch.  Ranks that share a GPU (tests) are merged into one cooperative launch with `emuCtas`
+// CTAs per rank, because their kernels wait for each other.
+HcclResult LaunchMoe(MoeCtx *m, void *kernel, const MoeParams &hp, int id, void *stream, int ctas, int emuCtas, int threads)
+{
+    Comm *c = m->comm;
+    const MoeParams *none = nullptr;
     if (c->emuSameDevice && c->nRanks > 1) {
-        const int perRank = ctas > 0 ? ctas : std::max(1, sms / (int)c->nRanks);
         return EmuLaunchGeneric(c->identifier + "#moe" + std::to_string(c->group.id), c->nRanks, c->rank, id, &hp, sizeof(hp), stream,
                                 [=](const void *devTable, uint32_t n, void *st) {
-                                    void *args[] = {(void *)&devTable};
-                                    cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(perRank, n, 1), dim3(threads, 1, 1), args, 0, (cudaStream_t)st);
+                                    MoeParams unused = hp;
+                                    void *args[] = {(void *)&unused, (void *)&devTable};
+                                    cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(emuCtas, n, 1), dim3(threads, 1, 1), args, 0, (cudaStream_t)st);
                                     if (e != cudaSuccess) { HCCL_ERROR("MoE launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
                                     return HCCL_SUCCESS;
                                 });
     }
-    MoeParams *slot = m->devParams + m->nextParam;
-    m->nextParam = (m->nextParam + 1) % 32;
-    if (cudaMemcpyAsync(slot, &hp, sizeof(hp), cudaMemcpyHostToDevice, (cudaStream_t)stream) != cudaSuccess) return HCCL_E_RUNTIME;
-    void *args[] = {(void *)&slot};
-    cudaError_t e = cudaLaunchKernel(kernel, dim3(ctas > 0 ? ctas : MoeCtas(sms), 1, 1), dim3(threads, 1, 1), args, 0, (cudaStream_t)stream);
+    void *args[] = {(void *)&hp, (void *)&none};
+    cudaError_t e = cudaLaunchKernel(kernel, dim3(ctas, 1, 1), dim3(threads, 1, 1), args, 0, (cudaStream_t)stream);
     if (e != cudaSuccess) { HCCL_ERROR("MoE launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
+}
+
+// The two launches of a dispatch; hp.scratch holds the row cursors.
+HcclResult LaunchDispatch(MoeCtx *m, const MoeParams &hp, int routeId, int dispatchId, void *stream)
+{
+    const int sms = MoeSms();
+    CHK_RET(LaunchMoe(m, (void *)MoeRouteKernel, hp, routeId, stream, 1, 1, 1024));
+    return LaunchMoe(m, (void *)MoeDispatchKernel, hp, dispatchId, stream, MoeCtas(m->comm, sms, hp.numTokens), std::max(1, sms / (int)m->comm->nRanks), 512);
 }
 
 }  // namespace
@@ -454,7 +545,8 @@ int HcommMoeCreate(HcclComm comm, int numExperts, int topk, int hidden, int maxT
     cudaMemset(m->scratch, 0, sizeof(uint32_t) * 2 * numExperts);
     cudaMalloc(&m->overflow, sizeof(uint32_t));
     cudaMemset(m->overflow, 0, sizeof(uint32_t));
-    cudaMalloc(&m->devParams, sizeof(MoeParams) * 32);
+    cudaMalloc(&m->localRow, sizeof(uint32_t) * (size_t)maxTokens * topk);
+    cudaMemset(m->localRow, 0xff, sizeof(uint32_t) * (size_t)maxTokens * topk);
     cudaGetDevice(&m->device);
     m->staticScratch = ResolveStaticScratch();       // set-up time, the exchange's GPU is current
     cudaFuncAttributes fa;
@@ -480,7 +572,7 @@ int HcommMoeDestroy(void *handle)
     cudaDeviceSynchronize();
     HcclCommSymWinDeregister(m->win);
     HcommMemFree(m->buf);
-    cudaFree(m->scratch); cudaFree(m->overflow); cudaFree(m->devParams);
+    cudaFree(m->scratch); cudaFree(m->overflow); cudaFree(m->localRow);
     delete m;
     return HCCL_SUCCESS;
 }
@@ -507,6 +599,7 @@ static void FillCommon(MoeCtx *m, MoeParams &hp)
     hp.lay = m->lay;
     hp.scratch = m->scratch;
     hp.overflow = m->overflow;
+    hp.localRow = m->localRow;
 }
 
 int HcommMoeDispatch(void *handle, const void *x, const int32_t *topkIdx, int numTokens, void *stream)
@@ -523,8 +616,7 @@ int HcommMoeDispatch(void *handle, const void *x, const int32_t *topkIdx, int nu
     FillCommon(m, hp);
     hp.x = (const __nv_bfloat16 *)x; hp.topkIdx = topkIdx; hp.numTokens = numTokens;
     ++c->opSeq;
-    CHK_RET(LaunchMoe(m, (void *)MoeRouteKernel, hp, 9100, stream, 1, 1024));
-    return LaunchMoe(m, (void *)MoeDispatchKernel, hp, 9101, stream);
+    return LaunchDispatch(m, hp, 9100, 9101, stream);
 }
 
 int HcommMoeCombine(void *handle, const void *y, const float *gates, void *out, int numTokens, void *stream)
@@ -541,8 +633,16 @@ int HcommMoeCombine(void *handle, const void *y, const float *gates, void *out, 
     FillCommon(m, hp);
     hp.y = (const __nv_bfloat16 *)y; hp.gates = gates; hp.out = (__nv_bfloat16 *)out; hp.numTokens = numTokens;
     ++c->opSeq;
-    CHK_RET(LaunchMoe(m, (void *)MoeCombineSendKernel, hp, 9102, stream));
-    return LaunchMoe(m, (void *)MoeCombineSumKernel, hp, 9104, stream);
+    const int sms = MoeSms(), emuCtas = std::max(1, sms / (int)c->nRanks), segs = m->lay.hidden / 256;
+    if (c->nRanks > 1) CHK_RET(LaunchMoe(m, (void *)MoeCombineSendKernel, hp, 9102, stream, MoeCtas(c, sms, 0), emuCtas, 512));
+    else hp.countsLaunch = 1;
+    // four segments to a warp where that still fills every SM's warps (the row addresses are then found once for all four),
+    // single segments below
+    constexpr int warps = kSumThreads / 32;
+    hp.segsPerItem = (int64_t)numTokens * ((segs + 3) / 4) >= (int64_t)warps * kSumCtasPerSm * sms ? 4 : 1;
+    const int64_t items = (int64_t)numTokens * ((segs + hp.segsPerItem - 1) / hp.segsPerItem);
+    const int forced = ForcedMoeCtas(), most = forced > 0 ? forced : kSumCtasPerSm * sms;
+    return LaunchMoe(m, (void *)MoeCombineSumKernel, hp, 9104, stream, (int)std::max<int64_t>(1, std::min<int64_t>(most, (items + warps - 1) / warps)), emuCtas, kSumThreads);
 }
 
 // ------------------------------------------------------------------ dispatch without any allocation
@@ -588,8 +688,7 @@ int HcommMoeDispatchStaticScratch(void *handle, const void *x, const int32_t *to
     hp.scratch = m->staticScratch;
     hp.x = (const __nv_bfloat16 *)x; hp.topkIdx = topkIdx; hp.numTokens = numTokens;
     ++c->opSeq;
-    CHK_RET(LaunchMoe(m, (void *)MoeRouteKernel, hp, 9105, stream, 1, 1024));
-    return LaunchMoe(m, (void *)MoeDispatchKernel, hp, 9103, stream);
+    return LaunchDispatch(m, hp, 9105, 9103, stream);
 }
 
 // Rows dropped because a rank received more than its capacity since the last call (clears the counter).

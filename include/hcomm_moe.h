@@ -19,7 +19,7 @@ struct MoeLayout {
     uint64_t offOrigin;          // u64 [maxRecvRows]                 (source rank << 32) | (token * topk + k)
     uint64_t offScales;          // f32 [maxRecvRows][hidden / 128]
     uint64_t offRows;            // fp8 e4m3 [maxRecvRows][hidden]
-    uint64_t offCombine;         // bf16 [maxTokens][topk][hidden]    landing area of the combine step
+    uint64_t offCombine;         // bf16 [maxTokens][topk][hidden]    landing area of the combine step: rows from other ranks
     uint64_t totalBytes;
     uint64_t offValid;           // u8 [maxTokens][topk]              1 = dispatch sent this (token, k), 0 = masked or dropped
 };

@@ -135,3 +135,53 @@ def test_masked_experts_and_dropped_rows_stay_out_of_the_sum(capacity_factor, ma
     finally:
         run_ranks(n, lambda r: moes[r].destroy())
         run_ranks(n, lambda r: comms[r].destroy())
+
+
+@pytest.mark.parametrize("experts,topk,hidden,tokens,capacity_factor,masked", [
+    (8, 2, 512, 1, 1.0, False), (8, 16, 512, 33, 1.0, False), (256, 8, 7168, 64, 1.0, True), (1024, 4, 8192, 300, 1.0, True), (64, 6, 2048, 1999, 1.0, False),
+    (16, 4, 1024, 700, 0.4, True)])
+def test_single_rank_rows_are_summed_where_the_experts_wrote_them(experts, topk, hidden, tokens, capacity_factor, masked):
+    """One rank: every row stays local.  Dispatched bytes, offsets and marks against the reference quantiser, the sum bit for
+    bit against fp32 accumulation in the order of k; CTAs with no token, several claim rounds per CTA, one to many segments."""
+    import hcomm_b200 as hb
+    from hcomm_b200.ops.moe import MoeExchange, quantize_e4m3_1x128
+    torch.cuda.set_device(0)
+    comm = hb.Communicator(1, hb.get_root_info(), 0, buffer_mb=8)
+    moe = MoeExchange(comm, experts, topk, hidden, tokens, capacity_factor=capacity_factor)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(tokens)
+        for t in (tokens, max(1, tokens // 3)):         # fewer tokens than the exchange is made for, over older contents
+            x = torch.randn(t, hidden, device="cuda", generator=g).to(torch.bfloat16)
+            # with replacement: several choices of one token may name the same expert
+            idx = torch.randint(0, experts, (t, topk), device="cuda", generator=g).to(torch.int32)
+            if masked:
+                idx[torch.rand(t, topk, device="cuda", generator=g) < 0.2] = -1
+                idx[0, 0] = experts
+            gates = torch.rand(t, topk, device="cuda", generator=g)
+            rec = moe.dispatch(x, idx)
+            torch.cuda.synchronize()
+            inside = (idx >= 0) & (idx < experts)
+            counts = torch.bincount(idx[inside].long(), minlength=experts)
+            want = torch.cat([torch.zeros(1, device="cuda", dtype=torch.int64), counts.cumsum(0)]).clamp(max=moe.layout.maxRecvRows)
+            assert torch.equal(rec.expert_offsets.long(), want)
+            sent, n = moe.sent[:t].bool(), rec.num_rows
+            assert bool((sent <= inside).all()) and int(sent.sum()) == n and moe.overflow() == int(inside.sum()) - n
+            origin = rec.origin[:n]
+            assert torch.equal(origin.sort().values, sent.flatten().nonzero().flatten())
+            expert_of_row = torch.bucketize(torch.arange(n, device="cuda"), want[1:], right=True)
+            assert torch.equal(idx.flatten()[origin].long(), expert_of_row)
+            q, sc = quantize_e4m3_1x128(x)
+            assert torch.equal(rec.rows[:n].view(torch.uint8), q.view(torch.uint8)[origin // topk]) and torch.equal(rec.scales[:n], sc[origin // topk])
+            y = torch.randn(n, hidden, device="cuda", generator=g).to(torch.bfloat16)
+            out = moe.combine(y, gates)
+            row = torch.full((t * topk,), -1, device="cuda", dtype=torch.int64)
+            row[origin] = torch.arange(n, device="cuda")
+            acc = torch.zeros(t, hidden, device="cuda", dtype=torch.float64)
+            for k in range(topk):                       # a fused multiply-add rounds once: the product is exact in fp64, the sum is rounded to fp32
+                r = row.view(t, topk)[:, k]
+                step = (acc + gates[:, k:k + 1].double() * y[r.clamp(min=0)].double()).float().double()
+                acc = torch.where((r >= 0).unsqueeze(1), step, acc)
+            assert torch.equal(out, acc.float().to(torch.bfloat16))
+    finally:
+        moe.destroy()
+        comm.destroy()
