@@ -157,6 +157,54 @@ bool TrySmallLL(Comm *c, const OpDesc &d, const Selection &sel, HcclResult *res)
     return true;
 }
 
+// A communicator of one rank: every data-moving operator is a copy of this rank's block, scaled where the operator scales.
+// Scatter and gather keep the staged kernels and their size limit.  Returns true (and the launch result in *res) when served.
+bool TryLocal(Comm *c, const OpDesc &d, HcclResult *res)
+{
+    if (c->nRanks != 1) return false;
+    const uint64_t esz = DtypeSize(d.dtype);
+    uint64_t count = d.count, from = 0, to = 0;
+    bool reducing = false;
+    switch (d.cmd) {
+        case HCCL_CMD_ALLREDUCE: case HCCL_CMD_REDUCE: reducing = true; break;
+        case HCCL_CMD_REDUCE_SCATTER: case HCCL_CMD_REDUCE_SCATTER_V:
+            reducing = true;
+            if (!d.sendCounts.empty()) { count = d.sendCounts[0]; from = d.sendDispls[0]; }
+            break;
+        case HCCL_CMD_ALLGATHER: case HCCL_CMD_ALLGATHER_V:
+            if (!d.recvCounts.empty()) { count = d.recvCounts[0]; to = d.recvDispls[0]; }
+            break;
+        case HCCL_CMD_ALLTOALL: case HCCL_CMD_ALLTOALLV: case HCCL_CMD_ALLTOALLVC:
+            if (!d.sendCounts.empty()) { count = d.sendCounts[0]; from = d.sendDispls[0]; }
+            if (!d.recvCounts.empty()) to = d.recvDispls[0];
+            break;
+        case HCCL_CMD_BROADCAST: break;
+        default: return false;
+    }
+    if (reducing && !DtypeReducible(d.dtype)) return false;
+    CollArgs a;
+    FillBase(c, d, a);
+    a.in = (const char *)d.in + from * esz;
+    a.out = (char *)d.out + to * esz;
+    a.count = count;
+    if (!reducing || !LocalNeedsType(d.dtype, d.useScale)) {
+        a.dtype = HCCL_DATA_TYPE_UINT8;
+        a.count = count * esz;
+        a.useScale = 0;
+    }
+    // two rounds of the CTAs that fit at once (two of 512 threads per SM: 64 KB of loads in flight); small operands spread in
+    // shares of 32 KB, four 16-byte words per thread
+    static const uint64_t most = 2 * (uint64_t)std::max(1, FastMaxCoResidentCtas(FK_LOCAL, 512, 0));
+    int ctas = (int)std::max<uint64_t>(1, std::min<uint64_t>(most, (count * esz + 32767) / 32768));
+    const int cap = EnvConfig::Get().maxCtas.value, forced = EnvConfig::Get().forceCtas.value;
+    const uint32_t own = __atomic_load_n(&c->ctaLimit, __ATOMIC_RELAXED);
+    if (cap > 0) ctas = std::min(ctas, cap);
+    if (own > 0) ctas = std::min(ctas, (int)own);
+    if (forced > 0) ctas = forced;
+    *res = Launch(c, FK_LOCAL, a, std::max(1, ctas), d.stream);
+    return true;
+}
+
 // -------------------------------------------------------------------------- fast-kernel drivers
 
 // Zero-copy on registered memory: when a buffer lies inside a window registered with HcclCommSymWinRegister (or an
@@ -813,6 +861,8 @@ HcclResult RunOpLocked(Comm *c, const OpDesc &d)
         // the stream engine has no fused scale: a second pass over the result applies it
         if (r == HCCL_SUCCESS && d.useScale) r = c->plat->ScaleAsync(d.out, d.count, d.dtype, d.scale, c->plat->kind() == PlatKind::SIM ? nullptr : d.stream);
         if (r == HCCL_SUCCESS && c->plat->kind() == PlatKind::SIM) r = CommPollDeviceStatus(c);
+    } else if (TryLocal(c, d, &r)) {
+        // a single rank has nobody to meet
     } else if (TrySmallLL(c, d, sel, &r)) {
         // served by the flag-in-data kernel
     } else {

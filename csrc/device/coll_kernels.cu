@@ -25,8 +25,11 @@
 //   AlltoAll(V/VC)      aiv_all_to_all_910b_smalldata.h, aiv_all_to_all_v_910b.h, ..._vc_910b_*.h
 //   Broadcast*          aiv_broadcast_910b_{small,big}data.h
 //   Reduce / Scatter / Gather   A5 aiv_reduce_mesh_1d.h, aiv_scatter_mesh_1d.h (+ gather)
+//   Local               a communicator of one rank (the reference copies with its runtime)
 //   Send / Recv         A5 aiv_send_mesh_1D.h / aiv_recv_mesh_1D.h
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "../alg/ir.h"
 #include "../core/log.h"
@@ -1263,6 +1266,83 @@ __global__ void __launch_bounds__(512) KIrInterp(const __grid_constant__ IrArgs 
     KernelEnd(d, ls, used);
 }
 
+// ----------------------------------------------------------------------------------- single rank
+
+// A communicator of one rank: out = scale * in (or in as it is).  No peer shares the partition of the data, so there is no
+// staging, no window and no barrier, and the CTAs sweep the operand together, lanes side by side whatever the alignment:
+// words of W bytes, the widest that both buffers start on, four loads of each thread in flight.  Bound by HBM: 33.4 M bf16
+// values scaled into another buffer, 134 MB in all, take 29 us in back-to-back calls (79 with the staged two-shot kernel,
+// which kept half as many loads in flight and cut the operand into windows with barriers between them); a copy by the driver
+// takes 25.  One contiguous share per CTA instead of the common sweep cost 2 us.
+template <int BYTES> struct WordOf { using type = typename BitsOf<BYTES>::type; };
+template <> struct WordOf<16> { using type = uint4; };
+template <typename T, int W>
+__device__ __forceinline__ void LocalRange(const char *in, char *out, uint64_t words, bool useScale, float scale)
+{
+    using V = typename WordOf<W>::type;
+    constexpr int N = W / (int)sizeof(T), U = 4;
+    union Word { V v; T e[N]; };
+    const uint64_t hi = words;
+    for (uint64_t i = (uint64_t)blockIdx.x * U * blockDim.x + threadIdx.x; i < hi; i += (uint64_t)gridDim.x * U * blockDim.x) {
+        Word w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (i + u * blockDim.x < hi) w[u].v = ((const V *)in)[i + u * blockDim.x];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i + u * blockDim.x >= hi) continue;
+            if constexpr (!std::is_same<T, uint8_t>::value) {
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    const typename AccOf<T>::type a = Widen<T>(w[u].e[j]);
+                    w[u].e[j] = Narrow<T>(useScale ? ScaleAcc<typename AccOf<T>::type>(a, scale) : a);
+                }
+            }
+            ((V *)out)[i + u * blockDim.x] = w[u].v;
+        }
+    }
+}
+template <typename T, int W>
+__device__ __forceinline__ void LocalMove(const char *in, char *out, uint64_t bytes, bool useScale, float scale)
+{
+    HC_BOUNDS_OR_RETURN(in, bytes);
+    HC_BOUNDS_OR_RETURN(out, bytes);
+    LocalRange<T, W>(in, out, bytes / W, useScale, scale);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x < (bytes % W) / sizeof(T)) {      // ragged end: fewer elements than a word
+        const uint64_t off = bytes / W * W + threadIdx.x * sizeof(T);
+        T v = *(const T *)(in + off);
+        if constexpr (!std::is_same<T, uint8_t>::value) {
+            const typename AccOf<T>::type a = Widen<T>(v);
+            v = Narrow<T>(useScale ? ScaleAcc<typename AccOf<T>::type>(a, scale) : a);
+        }
+        *(T *)(out + off) = v;
+    }
+}
+template <typename T>
+__global__ void __launch_bounds__(512, 2) KLocal(const __grid_constant__ CollArgs byval, const CollArgs *emu)
+{
+    HC_ARGS;
+    // launched with the stream-serialization attribute: resident before the kernel in front has ended, idle until it has
+    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+    const LaunchState ls = KernelBegin(d);
+    const char *in = (const char *)a.in;
+    char *out = (char *)a.out;
+    const uint64_t bytes = a.count * sizeof(T);
+    if (!(std::is_same<T, uint8_t>::value && in == out)) {
+        const uintptr_t both = (uintptr_t)in | (uintptr_t)out;
+        if ((both & 15) == 0) LocalMove<T, 16>(in, out, bytes, a.useScale != 0, a.scale);
+        else if ((both & 7) == 0 && sizeof(T) <= 8) LocalMove<T, 8>(in, out, bytes, a.useScale != 0, a.scale);
+        else if constexpr (sizeof(T) <= 4) {
+            if ((both & 3) == 0) LocalMove<T, 4>(in, out, bytes, a.useScale != 0, a.scale);
+            else if constexpr (sizeof(T) <= 2) {
+                if ((both & 1) == 0) LocalMove<T, 2>(in, out, bytes, a.useScale != 0, a.scale);
+                else if constexpr (sizeof(T) == 1) LocalMove<T, 1>(in, out, bytes, a.useScale != 0, a.scale);
+            }
+        }
+    }
+    KernelEnd(d, ls, 0);
+}
+
 template <typename K> struct KernelOf { K fn; };
 
 template <template <typename> class Dummy = AccOf>
@@ -1327,6 +1407,15 @@ void *KernelFor(int kind, int dtype)
         case FK_SEND: return (void *)KSend;
         case FK_RECV: return (void *)KRecv;
         case FK_BARRIER: return (void *)KBarrier;
+        case FK_LOCAL:
+            switch (dtype) {
+                case HCCL_DATA_TYPE_FP32: return (void *)KLocal<float>;
+                case HCCL_DATA_TYPE_FP16: return (void *)KLocal<__half>;
+                case HCCL_DATA_TYPE_BFP16: return (void *)KLocal<__nv_bfloat16>;
+                case HCCL_DATA_TYPE_FP64: return (void *)KLocal<double>;
+                case HCCL_DATA_TYPE_UINT8: return (void *)KLocal<uint8_t>;
+                default: return nullptr;
+            }
         default: return ReduceKernelFor<>(kind, dtype);
     }
 }
@@ -1358,8 +1447,13 @@ const char *FastKindName(int32_t k)
 {
     static const char *names[] = {"AllReduceOneShot", "AllReduceTwoShot", "AllReduceNvls", "ReduceScatter", "AllGather", "AlltoAll",
                                   "BroadcastPush", "BroadcastTwoShot", "BroadcastNvls", "Reduce", "Scatter", "Gather", "Send", "Recv", "Barrier", "SmallLL",
-                                  "ReduceScatterNvls", "AllGatherNvls", "AllReduceTwoShotWindows", "ReduceScatterWindows", "ReduceScatterInPlace", "AllReduceNvlsPipeline"};
+                                  "ReduceScatterNvls", "AllGatherNvls", "AllReduceTwoShotWindows", "ReduceScatterWindows", "ReduceScatterInPlace", "AllReduceNvlsPipeline", "Local"};
     return (k >= 0 && k < FK_COUNT) ? names[k] : "?";
+}
+
+bool LocalNeedsType(int32_t dtype, bool scaled)
+{
+    return scaled || dtype == HCCL_DATA_TYPE_FP16 || dtype == HCCL_DATA_TYPE_BFP16;
 }
 
 uint32_t FastKindBarriers(int32_t kind, int preBarrier)
@@ -1367,7 +1461,7 @@ uint32_t FastKindBarriers(int32_t kind, int preBarrier)
     uint32_t k = 1;
     switch (kind) {
         case FK_ALLREDUCE_TWOSHOT: case FK_ALLREDUCE_NVLS: case FK_REDUCE: case FK_BROADCAST_NVLS: k = 2; break;   // per window
-        case FK_SEND: case FK_RECV: case FK_SMALL_LL: return 0;
+        case FK_SEND: case FK_RECV: case FK_SMALL_LL: case FK_LOCAL: return 0;
         default: k = 1;
     }
     return k + (preBarrier ? 1 : 0);
@@ -1403,6 +1497,15 @@ HcclResult LaunchFastKernel(const FastLaunch &l)
     // for CTAs of the same launch (shared-GPU emulation, grid.sync in send/recv).
     bool coop = l.emuTable != nullptr;
     if (coop) e = cudaLaunchCooperativeKernel(fn, grid, block, params, 0, (cudaStream_t)l.stream);
+    else if (l.kind == FK_LOCAL) {
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid; cfg.blockDim = block; cfg.stream = (cudaStream_t)l.stream;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        e = cudaLaunchKernelExC(&cfg, fn, params);
+    }
     else e = cudaLaunchKernel(fn, grid, block, params, 0, (cudaStream_t)l.stream);
     if (e != cudaSuccess) {
         HCCL_ERROR("launch of %s (%d CTAs x %d threads, %d ranks) failed: %s", FastKindName(l.kind), l.ctas, l.threads, grid.y, cudaGetErrorString(e));

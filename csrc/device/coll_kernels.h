@@ -36,6 +36,7 @@ enum FastKind : int32_t {
     FK_REDUCE_SCATTER_WIN,      // reduce-scatter of blocks beyond a staging slot: column windows inside one launch
     FK_REDUCE_SCATTER_INPLACE,  // reduce-scatter that reads the peers' registered inputs in place
     FK_ALLREDUCE_NVLS_PIPE,     // in-switch all-reduce of a large unregistered operand: copy-in / reduce / copy-out of different windows overlap
+    FK_LOCAL,                   // single rank: out = scale * in, nothing staged and nobody to meet
     FK_COUNT
 };
 const char *FastKindName(int32_t k);
@@ -108,6 +109,9 @@ void PreloadFastKernels();
 HcclResult LaunchFastKernel(const FastLaunch &l);
 // Barriers a kernel of this kind consumes (the epoch advance), so callers can reason about it.
 uint32_t FastKindBarriers(int32_t kind, int preBarrier);
+// FK_LOCAL: whether a data type changes under it without a scale (16-bit floats pass through fp32, which gives every NaN one
+// form); all others are moved as bytes (launch those with HCCL_DATA_TYPE_UINT8 and the count in bytes).
+bool LocalNeedsType(int32_t dtype, bool scaled);
 // Upper bound of CTAs per rank for which all CTAs of `ranksOnDevice` ranks are co-resident.
 int FastMaxCoResidentCtas(int32_t kind, int threads, int ranksOnDevice);
 

@@ -320,3 +320,64 @@ def test_single_rank_operator_in_a_captured_cuda_graph():
     root = Path(__file__).resolve().parent.parent
     res = subprocess.run([sys.executable, str(root / "examples" / "02_graphs" / "allreduce_cuda_graph_demo.py")], capture_output=True, text=True, timeout=240)
     assert res.returncode == 0 and "5 replays ok" in res.stdout, res.stdout[-2000:] + res.stderr[-3000:]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16, torch.float64, torch.int8, torch.int64])
+@pytest.mark.parametrize("count", [1, 7, 4099, 1000003, 16777219])
+def test_single_rank_operators_move_and_scale(dtype, count):
+    """One rank: every operator is a copy of its block, the scaled all-reduce a product.  Buffers on and off 16 bytes (each
+    width of access), lengths that end inside a word, in place and not; values around a block must stay as they are."""
+    import hcomm_b200 as hb
+    torch.cuda.set_device(0)
+    comm = hb.Communicator(1, hb.get_root_info(), 0, buffer_mb=4)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(count)
+        floating = dtype.is_floating_point
+        for off_in, off_out in ((0, 0), (1, 0), (3, 3), (0, 8)):
+            pad = 16
+            base = (torch.randn(count + pad, device="cuda", generator=g) * 50).to(dtype)
+            if floating:
+                base[off_in] = float("-inf")
+            x = base[off_in:off_in + count]
+            mark = torch.full((count + pad,), 5, device="cuda", dtype=dtype)
+
+            def check(call, want, name):
+                full = mark.clone()
+                out = full[off_out:off_out + count]
+                call(out)
+                torch.cuda.synchronize()
+                assert torch.equal(out, want), (name, off_in, off_out)
+                full[off_out:off_out + count] = 5
+                assert torch.equal(full, mark), name + " wrote outside its block"
+            for op in ("sum", "max"):
+                check(lambda o: comm.all_reduce(x, o, op=op), x, "all_reduce")
+            check(lambda o: comm.all_gather(x, o), x, "all_gather")
+            check(lambda o: comm.reduce_scatter(x, o), x, "reduce_scatter")
+            check(lambda o: comm.all_to_all(x, o), x, "all_to_all")
+            check(lambda o: comm.reduce(x, o), x, "reduce")
+            if count > 4:
+                k = count - 4
+                want = mark[:count].clone()
+                want[2:2 + k] = x[3:3 + k]
+                check(lambda o: comm.all_to_all_v(x, [k], [3], o, [k], [2]), want, "all_to_all_v")
+                want = mark[:count].clone()
+                want[1:1 + k] = x[:k]
+                check(lambda o: comm.all_gather_v(x, o, [k], [1]), want, "all_gather_v")
+                want = mark[:count].clone()
+                want[:k] = x[2:2 + k]
+                check(lambda o: comm.reduce_scatter_v(x, [k], [2], o[:k]), want, "reduce_scatter_v")
+            if floating:
+                scale = 0.3
+                wide = torch.float64 if dtype == torch.float64 else torch.float32
+                want = (x.to(wide) * torch.tensor(scale, dtype=torch.float32, device="cuda").to(wide)).to(dtype)
+                check(lambda o: comm.all_reduce_scaled(x, o, scale), want, "all_reduce_scaled")
+                y = x.clone()
+                comm.all_reduce_scaled(y, y, scale)
+                assert torch.equal(y, want)
+            y = x.clone()
+            comm.all_reduce(y)
+            comm.broadcast(y)
+            assert torch.equal(y, x)
+        assert comm.async_error() == 0
+    finally:
+        comm.destroy()
