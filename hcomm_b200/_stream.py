@@ -1,0 +1,16 @@
+"""The raw handle of the stream that torch currently uses for a tensor's device, on the path of every call.
+
+``torch.cuda.current_stream(device).cuda_stream`` builds a stream object for each query (2.2 us, half the time of a small
+operator's launch); torch's own raw accessor answers in 0.1 us and is used where this torch has it.
+"""
+from __future__ import annotations
+
+import torch
+
+_raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def raw_stream(t: torch.Tensor) -> int:
+    if _raw is not None:
+        return _raw(t.get_device())
+    return torch.cuda.current_stream(t.device).cuda_stream

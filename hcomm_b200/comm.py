@@ -23,7 +23,10 @@ _NP_DTYPES = {
 _OPS = {"sum": _lib.SUM, "prod": _lib.PROD, "max": _lib.MAX, "min": _lib.MIN}
 
 
-def _torch_dtype_code(dt):
+_TORCH_DTYPES = {}         # filled at the first tensor: importing this module does not import torch
+
+
+def _fill_torch_dtypes():
     import torch
     table = {torch.int8: _lib.INT8, torch.int16: _lib.INT16, torch.int32: _lib.INT32, torch.float16: _lib.FP16, torch.float32: _lib.FP32,
              torch.int64: _lib.INT64, torch.uint8: _lib.UINT8, torch.float64: _lib.FP64, torch.bfloat16: _lib.BF16}
@@ -31,7 +34,7 @@ def _torch_dtype_code(dt):
                        ("uint64", _lib.UINT64)):
         if hasattr(torch, name):
             table[getattr(torch, name)] = code
-    return table[dt]
+    _TORCH_DTYPES.update(table)
 
 
 def describe(buf):
@@ -44,8 +47,13 @@ def describe(buf):
     if isinstance(buf, torch.Tensor):
         if not buf.is_contiguous():
             raise ValueError("buffers must be contiguous")
-        stream = torch.cuda.current_stream(buf.device).cuda_stream if buf.is_cuda else None
-        return buf.data_ptr(), buf.numel(), _torch_dtype_code(buf.dtype), stream
+        if not _TORCH_DTYPES:
+            _fill_torch_dtypes()
+        stream = None
+        if buf.is_cuda:
+            from ._stream import raw_stream
+            stream = raw_stream(buf)
+        return buf.data_ptr(), buf.numel(), _TORCH_DTYPES[buf.dtype], stream
     raise TypeError(f"unsupported buffer type {type(buf)}")
 
 

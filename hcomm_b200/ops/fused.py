@@ -11,6 +11,7 @@ import ctypes
 import torch
 
 from .. import _lib
+from .._stream import raw_stream
 from ..comm import Communicator
 
 
@@ -37,7 +38,7 @@ def gemm_reduce_scatter(comm: Communicator, a: torch.Tensor, b: torch.Tensor, ou
         raise ValueError("shape mismatch")
     if out is None:
         out = torch.empty((m // comm.size, n), dtype=torch.bfloat16, device=a.device)
-    stream = torch.cuda.current_stream(a.device).cuda_stream
+    stream = raw_stream(a)
     rc = _lib.load().HcommFusedGemmReduceScatterBf16Mode(ctypes.c_void_p(comm.handle), _ptr(a), _ptr(b), _ptr(out), m, n, k, a.stride(0), b.stride(0),
                                                          out.stride(0), ctypes.c_void_p(stream), MODES[mode])
     _lib.check(rc, "HcommFusedGemmReduceScatterBf16")
@@ -55,7 +56,7 @@ def all_gather_gemm(comm: Communicator, x: torch.Tensor, w: torch.Tensor, out: t
         raise ValueError("shape mismatch or non-contiguous shard")
     if out is None:
         out = torch.empty((ms * comm.size, n), dtype=torch.bfloat16, device=x.device)
-    stream = torch.cuda.current_stream(x.device).cuda_stream
+    stream = raw_stream(x)
     rc = _lib.load().HcommFusedAllGatherGemmBf16Mode(ctypes.c_void_p(comm.handle), _ptr(x), _ptr(w), _ptr(out), ms, n, k, x.stride(0), w.stride(0),
                                                      out.stride(0), ctypes.c_void_p(stream), MODES[mode])
     _lib.check(rc, "HcommFusedAllGatherGemmBf16")

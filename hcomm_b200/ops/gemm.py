@@ -10,6 +10,7 @@ import ctypes
 import torch
 
 from .. import _lib
+from .._stream import raw_stream
 
 
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -24,14 +25,20 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None)
     m, k = a.shape
     n = b.shape[0]
     if out is None:
-        out = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
-    lib = _lib.load()
-    stream = torch.cuda.current_stream(a.device).cuda_stream
-    with torch.cuda.device(a.device):
-        rc = lib.HcommGemmBf16(ctypes.c_void_p(a.data_ptr()), ctypes.c_void_p(b.data_ptr()), ctypes.c_void_p(out.data_ptr()), m, n, k,
-                               a.stride(0), b.stride(0), out.stride(0), ctypes.c_void_p(stream))
-    _lib.check(rc, "HcommGemmBf16")
+        out = a.new_empty((m, n))
+    if torch.cuda.current_device() == a.get_device():
+        _launch(a, b, out, m, n, k)
+    else:
+        with torch.cuda.device(a.device):
+            _launch(a, b, out, m, n, k)
     return out
+
+
+def _launch(a, b, out, m, n, k):
+    ptr = ctypes.c_void_p
+    rc = _lib.load().HcommGemmBf16(ptr(a.data_ptr()), ptr(b.data_ptr()), ptr(out.data_ptr()), m, n, k, a.stride(0), b.stride(0), out.stride(0), ptr(raw_stream(a)))
+    if rc:
+        _lib.check(rc, "HcommGemmBf16")
 
 
 def take_kernel_error() -> int:

@@ -17,6 +17,7 @@ from dataclasses import dataclass
 import torch
 
 from .. import _lib
+from .._stream import raw_stream
 from ..comm import Communicator
 
 
@@ -79,7 +80,7 @@ class MoeExchange:
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor) -> Received:
         assert x.dtype == torch.bfloat16 and x.is_contiguous() and x.shape[1] == self.hidden
         assert topk_idx.dtype == torch.int32 and topk_idx.is_contiguous() and topk_idx.shape == (x.shape[0], self.topk)
-        stream = torch.cuda.current_stream(x.device).cuda_stream
+        stream = raw_stream(x)
         _lib.check(self._lib.HcommMoeDispatch(self._h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(topk_idx.data_ptr()), x.shape[0],
                                               ctypes.c_void_p(stream)), "HcommMoeDispatch")
         return Received(self._rows, self._scales, self._origin, self._offsets)
@@ -90,7 +91,7 @@ class MoeExchange:
         t = gates.shape[0]
         if out is None:
             out = torch.empty((t, self.hidden), dtype=torch.bfloat16, device=y.device)
-        stream = torch.cuda.current_stream(y.device).cuda_stream
+        stream = raw_stream(y)
         _lib.check(self._lib.HcommMoeCombine(self._h, ctypes.c_void_p(y.data_ptr()), ctypes.c_void_p(gates.data_ptr()), ctypes.c_void_p(out.data_ptr()), t,
                                              ctypes.c_void_p(stream)), "HcommMoeCombine")
         return out
