@@ -66,7 +66,11 @@ struct MoeParams {
 };
 constexpr uint32_t kNoRow = 0xffffffffu;
 
-#define MOE_ARGS const MoeParams &p = (table != nullptr) ? table[blockIdx.y] : byval
+// A single rank launches with the stream-serialization attribute: the CTAs are resident before the kernel in front has ended
+// and idle until it has.
+#define MOE_ARGS                                                                            \
+    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory"); \
+    const MoeParams &p = (table != nullptr) ? table[blockIdx.y] : byval
 
 __device__ __forceinline__ uint32_t *Counts(const MoeParams &p, int rank) { return (uint32_t *)(p.peerBuf[rank] + p.lay.offCounts); }
 __device__ __forceinline__ uint8_t *Rows(const MoeParams &p, int rank) { return (uint8_t *)(p.peerBuf[rank] + p.lay.offRows); }
@@ -125,12 +129,12 @@ __global__ void __launch_bounds__(1024) MoeRouteKernel(const __grid_constant__ M
     __syncthreads();
     uint32_t *hist = sHist[(tid >> 5) & 3];
     const int total = p.numTokens * K, stride = blockDim.x;
-    for (int i = tid; i < total; i += 8 * stride) {         // eight loads in flight
-        int e[8];
+    for (int i = tid; i < total; i += 16 * stride) {        // sixteen loads in flight
+        int e[16];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) e[u] = i + u * stride < total ? p.topkIdx[i + u * stride] : -1;
+        for (int u = 0; u < 16; ++u) e[u] = i + u * stride < total ? p.topkIdx[i + u * stride] : -1;
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int u = 0; u < 16; ++u)
             if (e[u] >= 0 && e[u] < E) atomicAdd(&hist[e[u]], 1u);
     }
     __syncthreads();
@@ -318,10 +322,12 @@ __global__ void __launch_bounds__(512) MoeCombineSendKernel(const __grid_constan
 }
 
 // Combine, second launch (local): gate-weighted sum of the K rows of every local token, fp32 accumulation in the order of k.
-// Bound by memory: 2 k H bytes in, 2 H out per token; 3001 x 7168, 8 experts each, a tenth masked, 75 us (205 with every row
-// copied to its slot first), 54 at HBM rate; 64 tokens 7 us (13 + 43).  A warp takes segsPerItem segments of 256 columns of a token; lane k
-// finds the k-th row's address, and every lane keeps the loads of eight rows of a segment in flight.
-constexpr int kSumThreads = 256, kSumCtasPerSm = 3;     // 85 registers a thread: eight addresses and gates of rows beside their loads
+// Bound by memory: 2 k H bytes in, 2 H out per token; 3001 x 7168, 8 experts each, a tenth masked, 58 us (205 with every row
+// copied to its slot first), 54 at HBM rate; 64 tokens 6 us (13 + 43).  A warp takes segsPerItem segments of 256 columns of a token; lane k
+// finds the k-th row's address one item ahead, and every lane keeps the loads of eight rows of a segment in flight.
+constexpr int kSumThreads = 256, kSumCtasPerSm = 2;     // 128 registers a thread: eight addresses and gates of rows beside their loads; three CTAs spill and take 67 us for 58
+// BATCHES: groups of eight rows that K calls for.
+template <int BATCHES>
 __global__ void __launch_bounds__(kSumThreads, kSumCtasPerSm) MoeCombineSumKernel(const __grid_constant__ MoeParams byval, const MoeParams *table)
 {
     MOE_ARGS;
@@ -332,25 +338,37 @@ __global__ void __launch_bounds__(kSumThreads, kSumCtasPerSm) MoeCombineSumKerne
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warpsPerCta = blockDim.x >> 5;
     const int segs = H / 256, perToken = (segs + p.segsPerItem - 1) / p.segsPerItem;
     const int items = p.numTokens * perToken;
-    for (int it = blockIdx.x * warpsPerCta + warp; it < items; it += gridDim.x * warpsPerCta) {
+    const int step = gridDim.x * warpsPerCta;
+    // row, mark and gate of (token of item i, lane): looked up while the item before is being summed
+    uint32_t nextRow = kNoRow;
+    uint8_t nextValid = 0;
+    float nextGate = 0.f;
+    auto lookUp = [&](int i) {
+        if (i < items && lane < K) {
+            const size_t tk = (size_t)(i / perToken) * K + lane;
+            nextRow = p.localRow[tk];
+            nextValid = Valid(p, me)[tk];
+            nextGate = p.gates[tk];
+        }
+    };
+    int it = blockIdx.x * warpsPerCta + warp;
+    lookUp(it);
+    for (; it < items; it += step) {
         const int t = it / perToken, seg0 = (it - t * perToken) * p.segsPerItem;
         const int seg1 = seg0 + p.segsPerItem < segs ? seg0 + p.segsPerItem : segs;
         uint64_t mine = 0;                          // address of row (t, lane); zero when nothing was sent: the slot then holds an older step's row
-        float myGate = 0.f;
         if (lane < K) {
-            const size_t tk = (size_t)t * K + lane;
-            const uint32_t row = p.localRow[tk];
-            if (row != kNoRow) mine = (uint64_t)(p.y + (size_t)row * H);
-            else if (Valid(p, me)[tk] != 0) mine = (uint64_t)(Comb(p, me) + tk * H);
-            myGate = p.gates[tk];
+            if (nextRow != kNoRow) mine = (uint64_t)(p.y + (size_t)nextRow * H);
+            else if (nextValid != 0) mine = (uint64_t)(Comb(p, me) + ((size_t)t * K + lane) * H);
         }
+        const float myGate = nextGate;
+        lookUp(it + step);
         const uint32_t live = __ballot_sync(0xffffffffu, mine != 0);
         for (int seg = seg0; seg < seg1; ++seg) {
             const uint32_t col = seg * 512 + lane * 16;         // bytes
             float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-            for (int kb = 0; kb < 16; kb += 8) {
-                if (kb >= K) break;
+            for (int kb = 0; kb < 8 * BATCHES; kb += 8) {
                 uint4 pk[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
@@ -440,7 +458,13 @@ HcclResult LaunchMoe(MoeCtx *m, void *kernel, const MoeParams &hp, int id, void 
                                 });
     }
     void *args[] = {(void *)&hp, (void *)&none};
-    cudaError_t e = cudaLaunchKernel(kernel, dim3(ctas, 1, 1), dim3(threads, 1, 1), args, 0, (cudaStream_t)stream);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas, 1, 1); cfg.blockDim = dim3(threads, 1, 1); cfg.stream = (cudaStream_t)stream;
+    cfg.attrs = at; cfg.numAttrs = c->nRanks == 1 ? 1 : 0;        // kernels that meet other ranks hold no SM before their turn
+    cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
     if (e != cudaSuccess) { HCCL_ERROR("MoE launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
@@ -553,7 +577,8 @@ int HcommMoeCreate(HcclComm comm, int numExperts, int topk, int hidden, int maxT
     cudaFuncGetAttributes(&fa, MoeRouteKernel);
     cudaFuncGetAttributes(&fa, MoeDispatchKernel);
     cudaFuncGetAttributes(&fa, MoeCombineSendKernel);
-    cudaFuncGetAttributes(&fa, MoeCombineSumKernel);
+    cudaFuncGetAttributes(&fa, MoeCombineSumKernel<1>);
+    cudaFuncGetAttributes(&fa, MoeCombineSumKernel<2>);
     cudaDeviceSynchronize();
     *handle = m;
     if (layoutOut) *layoutOut = L;
@@ -642,7 +667,7 @@ int HcommMoeCombine(void *handle, const void *y, const float *gates, void *out, 
     hp.segsPerItem = (int64_t)numTokens * ((segs + 3) / 4) >= (int64_t)warps * kSumCtasPerSm * sms ? 4 : 1;
     const int64_t items = (int64_t)numTokens * ((segs + hp.segsPerItem - 1) / hp.segsPerItem);
     const int forced = ForcedMoeCtas(), most = forced > 0 ? forced : kSumCtasPerSm * sms;
-    return LaunchMoe(m, (void *)MoeCombineSumKernel, hp, 9104, stream, (int)std::max<int64_t>(1, std::min<int64_t>(most, (items + warps - 1) / warps)), emuCtas, kSumThreads);
+    return LaunchMoe(m, m->lay.topk <= 8 ? (void *)MoeCombineSumKernel<1> : (void *)MoeCombineSumKernel<2>, hp, 9104, stream, (int)std::max<int64_t>(1, std::min<int64_t>(most, (items + warps - 1) / warps)), emuCtas, kSumThreads);
 }
 
 // ------------------------------------------------------------------ dispatch without any allocation
