@@ -60,7 +60,7 @@ struct MoeParams {
     const float *gates;
     __nv_bfloat16 *out;
     uint32_t *overflow;                   // device word: rows that did not fit the receive capacity
-    uint32_t *localRow;                   // [maxTokens * topk]: row of (token, k) in this rank's receive buffer, kNoRow when it went elsewhere
+    uint32_t *localRow;                   // [maxTokens * topk]: 1 + row of (token, k) in this rank's receive buffer, 0 when it went elsewhere or nowhere
     int segsPerItem;                      // sum: 256-column segments that a warp takes at a time
     int countsLaunch;                     // sum: this launch is the whole operator (single rank) and advances the launch state
 };
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constan
         if (tid < tokens * K) {
             const size_t tk = (size_t)r0 * K + tid;
             const int e = p.topkIdx[tk];
-            uint32_t slot = kNoRow, local = kNoRow;
+            uint32_t slot = kNoRow, local = 0;
             if (e >= 0 && e < E) {
                 slot = sBase[e] + atomicAdd(&cursor[e], 1u);
                 if (slot >= (uint32_t)p.lay.maxRecvRows) { atomicAdd(p.overflow, 1u); slot = kNoRow; }
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constan
                 sRow[tid] = Rows(p, owner) + (size_t)slot * H;
                 sScale[tid] = Scales(p, owner) + (size_t)slot * (H / kBlock);
                 Origin(p, owner)[slot] = ((uint64_t)me << 32) | (uint32_t)tk;
-                if (owner == me) local = slot;
+                if (owner == me) local = slot + 1;
             }
             p.localRow[tk] = local;
         }
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kSumThreads, kSumCtasPerSm) MoeCombineSumKerne
     const int items = p.numTokens * perToken;
     const int step = gridDim.x * warpsPerCta;
     // row, mark and gate of (token of item i, lane): looked up while the item before is being summed
-    uint32_t nextRow = kNoRow;
+    uint32_t nextRow = 0;
     uint8_t nextValid = 0;
     float nextGate = 0.f;
     auto lookUp = [&](int i) {
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kSumThreads, kSumCtasPerSm) MoeCombineSumKerne
         const int seg1 = seg0 + p.segsPerItem < segs ? seg0 + p.segsPerItem : segs;
         uint64_t mine = 0;                          // address of row (t, lane); zero when nothing was sent: the slot then holds an older step's row
         if (lane < K) {
-            if (nextRow != kNoRow) mine = (uint64_t)(p.y + (size_t)nextRow * H);
+            if (nextRow != 0) mine = (uint64_t)(p.y + (size_t)(nextRow - 1) * H);
             else if (nextValid != 0) mine = (uint64_t)(Comb(p, me) + ((size_t)t * K + lane) * H);
         }
         const float myGate = nextGate;
@@ -565,12 +565,12 @@ int HcommMoeCreate(HcclComm comm, int numExperts, int topk, int hidden, int maxT
         HcclSymWinGetPeerPointer(m->win, 0, (uint32_t)q, &pp);
         m->peer[q] = (char *)pp;
     }
-    cudaMalloc(&m->scratch, sizeof(uint32_t) * 2 * numExperts);
-    cudaMemset(m->scratch, 0, sizeof(uint32_t) * 2 * numExperts);
-    cudaMalloc(&m->overflow, sizeof(uint32_t));
-    cudaMemset(m->overflow, 0, sizeof(uint32_t));
-    cudaMalloc(&m->localRow, sizeof(uint32_t) * (size_t)maxTokens * topk);
-    cudaMemset(m->localRow, 0xff, sizeof(uint32_t) * (size_t)maxTokens * topk);
+    // one block: the row cursors, the overflow count, the local rows
+    const size_t words = 2 * (size_t)numExperts + 64 + (size_t)maxTokens * topk;
+    cudaMalloc(&m->scratch, sizeof(uint32_t) * words);
+    cudaMemset(m->scratch, 0, sizeof(uint32_t) * words);
+    m->overflow = m->scratch + 2 * numExperts;
+    m->localRow = m->overflow + 64;
     cudaGetDevice(&m->device);
     m->staticScratch = ResolveStaticScratch();       // set-up time, the exchange's GPU is current
     cudaFuncAttributes fa;
@@ -597,7 +597,7 @@ int HcommMoeDestroy(void *handle)
     cudaDeviceSynchronize();
     HcclCommSymWinDeregister(m->win);
     HcommMemFree(m->buf);
-    cudaFree(m->scratch); cudaFree(m->overflow); cudaFree(m->localRow);
+    cudaFree(m->scratch);
     delete m;
     return HCCL_SUCCESS;
 }
