@@ -160,8 +160,8 @@ __global__ void __launch_bounds__(1024) MoeRouteKernel(const __grid_constant__ M
 // Dispatch, second launch (any number of CTAs, an ordinary launch that can share the GPU with expert GEMMs): every CTA
 // derives from the owners' count tables where this rank's rows of each expert start, claims the rows of its tokens, then
 // quantises and sends them, and meets its namesakes on the other ranks once all of its rows are on their way.
-// Bound by memory and, about as much, by the instructions of 16 divisions and k stores per 32 bytes: 4096 x 7168 to 8 experts
-// each take 69 us (86 with one warp per token), 46 at HBM rate; 64 tokens 9 us (39).  A CTA owns whole tokens and its 16 warps share them in
+// Bound by memory, by its scattered 512-byte stores: 4096 x 7168 to 8 experts each take 69 us (86 with one warp per token), 46
+// at HBM rate, and no less with a sixth of the divisions; 64 tokens 9 us (39).  A CTA owns whole tokens and its 16 warps share them in
 // pieces of 512 values, so that few tokens still occupy many warps and the claims cost one round of atomics per CTA, not one
 // per token.
 //
