@@ -191,6 +191,10 @@ bool TryLocal(Comm *c, const OpDesc &d, HcclResult *res)
         a.dtype = HCCL_DATA_TYPE_UINT8;
         a.count = count * esz;
         a.useScale = 0;
+    } else if ((((uintptr_t)a.in | (uintptr_t)a.out) & (esz - 1)) != 0) {
+        RPT_ERR("EI0003", "%s: buffers that do not start on an element of %s", CmdName(d.cmd), DtypeName(d.dtype));
+        *res = HCCL_E_PARA;
+        return true;
     }
     // two rounds of the CTAs that fit at once (two of 512 threads per SM: 64 KB of loads in flight); small operands spread in
     // shares of 32 KB, four 16-byte words per thread

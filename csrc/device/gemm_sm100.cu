@@ -58,11 +58,23 @@ template <int SPLIT> int SwapCapacityOf()
     HCCL_INFO("GEMM clusters of %d CTAs resident at once: %d", 2 * SPLIT, n);
     return n;
 }
-// Clusters of 2^log2Pairs CTA pairs that can be resident at once (0 when the query fails).
+// Clusters of 2^log2Pairs CTA pairs that the current device holds at once (0 when the query fails).  The kernels' shared
+// memory limits are a device's own, so the first call on each device sets them.
 int SwapCapacity(int log2Pairs)
 {
-    static const int cap[3] = {SwapCapacityOf<1>(), SwapCapacityOf<2>(), SwapCapacityOf<4>()};
-    return cap[log2Pairs];
+    constexpr int kDevices = 16;
+    static std::once_flag once[kDevices];
+    static int cap[kDevices][3];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) { cudaGetLastError(); return 0; }
+    std::call_once(once[dev], [dev] {
+        const bool wide = cudaFuncSetAttribute(GemmBf16PairWideKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::ConfigWide<4>::kSmemBytes) == cudaSuccess;
+        if (!wide) cudaGetLastError();
+        cap[dev][0] = wide ? SwapCapacityOf<1>() : 0;
+        cap[dev][1] = SwapCapacityOf<2>();
+        cap[dev][2] = SwapCapacityOf<4>();
+    });
+    return cap[dev][log2Pairs];
 }
 
 }  // namespace
@@ -261,8 +273,6 @@ HcclResult LaunchWideGemm(const void *A, const void *B, void *C, int M, int N, i
     shape.tilesN = (N + hcgemm::kWideN - 1) / hcgemm::kWideN;
     shape.errFlag = GemmErrorFlag();
     shape.phase = nullptr;
-    static const bool ready = cudaFuncSetAttribute(GemmBf16PairWideKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::ConfigWide<4>::kSmemBytes) == cudaSuccess;
-    if (!ready) { cudaGetLastError(); HCCL_ERROR("GemmBf16: no shared memory for 256 x 512 tiles"); return HCCL_E_RUNTIME; }
     // a wave of 74 such tiles loads the fewest panels at 12 rows x 6 columns
     const int rows = PairGroupRows(K), group = g_forceGm.load() > 0 || rows >= 16 ? rows : 12;
     cudaLaunchAttribute at[2];

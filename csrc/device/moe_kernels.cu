@@ -60,7 +60,7 @@ struct MoeParams {
     const __nv_bfloat16 *y;
     const float *gates;
     __nv_bfloat16 *out;
-    uint32_t *overflow;                   // device word: rows that did not fit the receive capacity
+    uint32_t *overflow;                   // device words: rows that did not fit the receive capacity, tokens of the last dispatch
     uint32_t *localRow;                   // [maxTokens * topk]: 1 + row of (token, k) in this rank's receive buffer, 0 when it went elsewhere or nowhere
     int segsPerItem;                      // sum: 256-column segments that a warp takes at a time
     int countsLaunch;                     // sum: this launch is the whole operator (single rank) and advances the launch state
@@ -270,6 +270,7 @@ __global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constan
         __syncthreads();
     }
 
+    if (blockIdx.x == 0 && tid == 0) p.overflow[1] = (uint32_t)p.numTokens;
     for (int r0 = t0; r0 < t1; r0 += perRound) {
         const int tokens = t1 - r0 < perRound ? t1 - r0 : perRound;
         if (tid < tokens * K) {
@@ -391,9 +392,13 @@ __global__ void __launch_bounds__(kSumThreads, kSumCtasPerSm) MoeCombineSumKerne
     uint32_t nextRow = 0;
     uint8_t nextValid = 0;
     float nextGate = 0.f;
+    const int dispatched = (int)p.overflow[1];      // marks and rows of later tokens are an older dispatch's: nothing is added for them
     auto lookUp = [&](int i) {
-        if (i < items && lane < K) {
-            const size_t tk = (size_t)(i / perToken) * K + lane;
+        const int t = i / perToken;
+        nextRow = 0;
+        nextValid = 0;
+        if (i < items && lane < K && t < dispatched) {
+            const size_t tk = (size_t)t * K + lane;
             nextRow = p.localRow[tk];
             nextValid = Valid(p, me)[tk];
             nextGate = p.gates[tk];
@@ -615,7 +620,7 @@ int HcommMoeCreate(HcclComm comm, int numExperts, int topk, int hidden, int maxT
         HcclSymWinGetPeerPointer(m->win, 0, (uint32_t)q, &pp);
         m->peer[q] = (char *)pp;
     }
-    // one block: the row cursors, the overflow count, the local rows
+    // one block: the row cursors, the overflow count and the last dispatch's tokens, the local rows
     const size_t words = 2 * (size_t)numExperts + 64 + (size_t)maxTokens * topk;
     cudaMalloc(&m->scratch, sizeof(uint32_t) * words);
     cudaMemset(m->scratch, 0, sizeof(uint32_t) * words);

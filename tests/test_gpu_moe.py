@@ -185,3 +185,24 @@ def test_single_rank_rows_are_summed_where_the_experts_wrote_them(experts, topk,
     finally:
         moe.destroy()
         comm.destroy()
+
+
+def test_combine_of_more_tokens_than_were_dispatched_adds_nothing_for_the_rest():
+    """The marks and rows of tokens beyond the last dispatch are an older one's, and the experts' output holds none of those
+    rows: their sums are zero, whatever the older dispatch left behind."""
+    import hcomm_b200 as hb
+    from hcomm_b200.ops.moe import MoeExchange
+    torch.cuda.set_device(0)
+    comm = hb.Communicator(1, hb.get_root_info(), 0, buffer_mb=8)
+    moe = MoeExchange(comm, 8, 2, 512, 64)
+    try:
+        x = torch.randn(64, 512, device="cuda").to(torch.bfloat16)
+        idx = torch.randint(0, 8, (64, 2), device="cuda").to(torch.int32)
+        moe.dispatch(x, idx)
+        moe.dispatch(x[:5].contiguous(), idx[:5].contiguous())
+        out = moe.combine(torch.ones(10, 512, device="cuda", dtype=torch.bfloat16), torch.ones(64, 2, device="cuda"))
+        torch.cuda.synchronize()
+        assert bool((out[:5] == 2).all()) and bool((out[5:] == 0).all())
+    finally:
+        moe.destroy()
+        comm.destroy()
