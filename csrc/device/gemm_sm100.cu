@@ -179,6 +179,8 @@ namespace {
 //   * tiles come in whole waves of the clusters that fit at once (74 of two CTAs, 33 of four, 15 of eight);
 //   * all operand traffic passes L2 at 13.5 TB/s, every operand comes from HBM once at 6.5 TB/s, a tenth less when only a
 //     few SMs ask for it;
+//     up to 256 tokens, where weights come from HBM and go to every token tile, a fifth of the L2 time adds to that of HBM
+//     (60 shapes: the choice is 1.4 % off the best on average, 2.3 % without; 40 x 4096 x 4096 64/2 10.5 us, not 32/2 12.1);
 //   * a launch costs 3 us, emptying the accumulator 6 ns per token, exchanging partial sums 1.5 us and 8 ns per token; a
 //     further wave of clusters that share tiles starts from nothing, 3 us;
 //   * a 256 x 512 tile moves a quarter less operand data than two of 256 x 256, and under the power cap that sets the clock:
@@ -202,12 +204,13 @@ PairTile PickPairTile(int M, int N, int K, const int (&cap)[3])
             const double tiles = tilesW * ((M + bn - 1) / bn), x = std::min(bn, M);
             const double waves = std::ceil(tiles / cap[si]), active = std::min(tiles, (double)cap[si]) * split / cap[0];
             const double step = std::max(48 + 1.28 * bn, (16384 + 64 * x) / 120);
-            const double loop = std::max(waves * std::ceil(kBlocks / split) * step, tiles * kBlocks * (32768 + 128 * x) / 13500);
-            const double ns = std::max(loop, hbmNs / (0.9 + 0.1 * std::min(1.0, active))) + 3000 + 6 * x + (split > 1 ? 1500 + 8 * x + (waves - 1) * 3000 : 0);
+            const double l2Ns = tiles * kBlocks * (32768 + 128 * x) / 13500;
+            const double loop = std::max(waves * std::ceil(kBlocks / split) * step, l2Ns);
+            const double ns = std::max(loop, hbmNs / (0.9 + 0.1 * std::min(1.0, active))) + (M <= 256 ? 0.2 * l2Ns : 0) + 3000 + 6 * x + (split > 1 ? 1500 + 8 * x + (waves - 1) * 3000 : 0);
             if (bestNs == 0 || ns < bestNs) { bestNs = ns; best = {bn, split}; }
         }
     }
-    if (cap[0] > 0) {
+    if (cap[0] > 0 && M > 256) {
         const double tiles = (double)((M + hcgemm::kPairM - 1) / hcgemm::kPairM) * ((N + hcgemm::kWideN - 1) / hcgemm::kWideN);
         if (std::max(std::ceil(tiles / cap[0]) * (kBlocks * 690 + 4000), hbmNs) + 3000 < bestNs) best = {hcgemm::kWideN, 1};
     }

@@ -36,6 +36,7 @@ def test_known_choices():
     assert pick(16, 28672, 8192, caps) == (32, 1)       # 112 tiles keep the chip busy as they are
     assert pick(96, 3584, 8192, caps) == (96, 4)        # 14 tiles, a deep K
     assert pick(33, 128256, 4096, caps) == (64, 1)      # one tile across all tokens: every weight is fetched once
+    assert pick(40, 4096, 4096, caps) == (64, 2)        # not two token tiles that both read every weight
     assert pick(8192, 28672, 8192, caps) == (512, 1)    # 25 full waves: the least operand traffic
     assert pick(777, 14336, 4096, caps) == (160, 1)     # 800 columns of work for 777 tokens
     assert pick(8192, 3584, 8192, caps) == (224, 1)     # seven full waves instead of eight of 256 columns
