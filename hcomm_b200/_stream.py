@@ -11,6 +11,9 @@ _raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def raw_stream(t: torch.Tensor) -> int:
+    device = t.get_device()
+    if device < 0:          # the raw accessor takes a negative index for the current device; a host address must not reach a kernel
+        raise ValueError(f"expected a tensor on a CUDA device, but got one on {t.device}")
     if _raw is not None:
-        return _raw(t.get_device())
+        return _raw(device)
     return torch.cuda.current_stream(t.device).cuda_stream
