@@ -74,6 +74,7 @@ __device__ __forceinline__ void GemmMainLoopPairWide(const CUtensorMap *tmA, con
     __syncthreads();
     ClusterSync();
     TcFenceAfter();
+    GridDependencyWait();   // every role, not only the producer: a bounded wait must not run down while the kernel in front still works
     const uint32_t tmemBase = st->tmemBase;
 
     if (warp == 0) {
@@ -81,7 +82,6 @@ __device__ __forceinline__ void GemmMainLoopPairWide(const CUtensorMap *tmA, con
         if (ElectOne()) {
             uint32_t it = 0;
             bool alive = true;
-            GridDependencyWait();           // up to here a CTA may run beside the tail of the kernel in front; all it writes follows its loads
             for (int t = firstTile; t < numTiles && alive; t += tileStep) {
                 int mb, nb;
                 order(t, g, &mb, &nb);

@@ -119,6 +119,7 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
     __syncthreads();
     ClusterSync();          // every barrier of the cluster is initialised before anything signals it
     TcFenceAfter();
+    GridDependencyWait();   // every role, not only the producer: a bounded wait must not run down while the kernel in front still works
     const uint32_t tmemBase = st->tmemBase;
 
     if (warp == 0) {
@@ -127,7 +128,6 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
             int s = 0;
             uint32_t ph = 0;
             bool alive = true;
-            GridDependencyWait();           // up to here a CTA may run beside the tail of the kernel in front; all it writes follows its loads
             for (int t = firstTile; t < numTiles && alive; t += tileStep) {
                 int wb, tb;
                 order(t, &wb, &tb);

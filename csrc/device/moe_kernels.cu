@@ -64,14 +64,17 @@ struct MoeParams {
     uint32_t *localRow;                   // [maxTokens * topk]: 1 + row of (token, k) in this rank's receive buffer, 0 when it went elsewhere or nowhere
     int segsPerItem;                      // sum: 256-column segments that a warp takes at a time
     int countsLaunch;                     // sum: this launch is the whole operator (single rank) and advances the launch state
+    int overlaps;                         // single rank: the kernel behind may take SMs early (see MOE_ARGS)
 };
 constexpr uint32_t kNoRow = 0xffffffffu;
 
 // A single rank launches with the stream-serialization attribute: the CTAs are resident before the kernel in front has ended
-// and idle until it has.
-#define MOE_ARGS                                                                            \
-    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory"); \
-    const MoeParams &p = (table != nullptr) ? table[blockIdx.y] : byval
+// and idle until it has, and the kernel behind may do the same.  Kernels that meet other ranks let nothing start early: what is
+// resident behind them would hold its SMs for as long as a peer is late.
+#define MOE_ARGS                                                                               \
+    const MoeParams &p = (table != nullptr) ? table[blockIdx.y] : byval;                       \
+    if (p.overlaps) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");            \
+    asm volatile("griddepcontrol.wait;" ::: "memory")
 
 __device__ __forceinline__ uint32_t *Counts(const MoeParams &p, int rank) { return (uint32_t *)(p.peerBuf[rank] + p.lay.offCounts); }
 __device__ __forceinline__ uint8_t *Rows(const MoeParams &p, int rank) { return (uint8_t *)(p.peerBuf[rank] + p.lay.offRows); }
@@ -516,7 +519,7 @@ HcclResult LaunchMoe(MoeCtx *m, void *kernel, const MoeParams &hp, int id, void 
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas, 1, 1); cfg.blockDim = dim3(threads, 1, 1); cfg.stream = (cudaStream_t)stream;
-    cfg.attrs = at; cfg.numAttrs = c->nRanks == 1 ? 1 : 0;        // kernels that meet other ranks hold no SM before their turn
+    cfg.attrs = at; cfg.numAttrs = hp.overlaps ? 1 : 0;        // kernels that meet other ranks hold no SM before their turn
     cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
     if (e != cudaSuccess) { HCCL_ERROR("MoE launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
@@ -681,6 +684,7 @@ static void FillCommon(MoeCtx *m, MoeParams &hp)
     hp.scratch = m->scratch;
     hp.overflow = m->overflow;
     hp.localRow = m->localRow;
+    hp.overlaps = m->comm->nRanks == 1;
 }
 
 int HcommMoeDispatch(void *handle, const void *x, const int32_t *topkIdx, int numTokens, void *stream)

@@ -31,6 +31,8 @@ __device__ __forceinline__ bool ElectOne()
 // Programmatic dependent launch (a launch with the stream-serialization attribute; without it both do nothing).  Wait: until
 // the grids in front have completed and their writes are visible - before the first access to memory that they may touch.
 // Launch: the grid behind may start to take the SMs that this one leaves; its own Wait still holds it back from memory.
+// Two rules: bounded waits (MbarWait) come after the Wait, or they count down while the grid in front works; and a grid that
+// meets other ranks never executes Launch, so that nothing sits on SMs for as long as a peer is late.
 __device__ __forceinline__ void GridDependencyWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void GridDependentsLaunch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
