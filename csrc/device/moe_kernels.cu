@@ -19,6 +19,9 @@
 //         cross-rank barrier
 //   sum   out = sum_k gate[k] * row(token, k) over the k that were sent, fp32 accumulation in the order of k; a row whose
 //         expert lives on the token's own rank is read where the expert wrote it (dispatch noted which row that is)
+// Rows of this rank's own tokens go through their slots as well (and a single rank has both launches) when the result may
+// overlap the experts' output, whose rows would otherwise be overwritten before they are read, and once the caller has
+// asked for the address of the slots.
 //
 // Device scratch (beyond inputs and outputs): numExperts u32 row cursors (second half of a 2 * numExperts table), cleared
 // by the route launch; the local row of every (token, k).
@@ -28,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <map>
 
 #include "../comm/comm.h"
@@ -64,6 +68,7 @@ struct MoeParams {
     uint32_t *localRow;                   // [maxTokens * topk]: 1 + row of (token, k) in this rank's receive buffer, 0 when it went elsewhere or nowhere
     int segsPerItem;                      // sum: 256-column segments that a warp takes at a time
     int countsLaunch;                     // sum: this launch is the whole operator (single rank) and advances the launch state
+    int allThroughSlots;                  // combine: rows of this rank's own tokens go through the landing area too
     int overlaps;                         // single rank: the kernel behind may take SMs early (see MOE_ARGS)
 };
 constexpr uint32_t kNoRow = 0xffffffffu;
@@ -339,7 +344,7 @@ __global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constan
     KernelEnd(d, ls, 1);
 }
 
-// Combine, first launch: every expert output row of another rank's token goes home, into slot (token, k) of that rank; each
+// Combine, first launch: every expert output row of another rank's token (all rows with allThroughSlots) goes home, into slot (token, k) of that rank; each
 // CTA then meets its namesakes on the other ranks.  When the kernel has ended on a rank, every rank's rows for it have landed.
 __global__ void __launch_bounds__(512) MoeCombineSendKernel(const __grid_constant__ MoeParams byval, const MoeParams *table)
 {
@@ -354,7 +359,7 @@ __global__ void __launch_bounds__(512) MoeCombineSendKernel(const __grid_constan
     for (int r = blockIdx.x * warpsPerCta + warp; r < rows; r += gridDim.x * warpsPerCta) {
         const uint64_t o = Origin(p, me)[r];
         const int src = (int)(o >> 32);
-        if (src == me) continue;                     // the sum reads it where it is
+        if (src == me && !p.allThroughSlots) continue;       // the sum reads it where it is
         const uint32_t tk = (uint32_t)o;
         const uint4 *in = (const uint4 *)(p.y + (size_t)r * H);
         uint4 *dst = (uint4 *)(Comb(p, src) + (size_t)tk * H);
@@ -402,7 +407,7 @@ __global__ void __launch_bounds__(kSumThreads, kSumCtasPerSm) MoeCombineSumKerne
         nextValid = 0;
         if (i < items && lane < K && t < dispatched) {
             const size_t tk = (size_t)t * K + lane;
-            nextRow = p.localRow[tk];
+            nextRow = p.allThroughSlots ? 0u : p.localRow[tk];
             nextValid = Valid(p, me)[tk];
             nextGate = p.gates[tk];
         }
@@ -468,6 +473,7 @@ struct MoeCtx {
     int device = -1;                     // the GPU this exchange was created on
     uint32_t *overflow = nullptr;
     uint32_t *localRow = nullptr;        // [maxTokens * topk], see MoeParams
+    std::atomic<bool> slotsAsked{false}; // HcommMoeGetBuffers has handed out the landing area: combine fills all of it
 };
 std::mutex g_mu;
 std::map<void *, MoeCtx *> g_ctx;
@@ -671,7 +677,10 @@ int HcommMoeGetBuffers(void *handle, void **rows, void **scales, void **origin, 
     if (scales) *scales = b + m->lay.offScales;
     if (origin) *origin = b + m->lay.offOrigin;
     if (expertOffsets) *expertOffsets = b + m->lay.offExpertOffsets;
-    if (combine) *combine = b + m->lay.offCombine;
+    if (combine) {
+        *combine = b + m->lay.offCombine;
+        m->slotsAsked.store(true);
+    }
     return HCCL_SUCCESS;
 }
 
@@ -706,6 +715,12 @@ int HcommMoeDispatch(void *handle, const void *x, const int32_t *topkIdx, int nu
 
 int HcommMoeCombine(void *handle, const void *y, const float *gates, void *out, int numTokens, void *stream)
 {
+    // how many rows y has is not known here: as many as can be received
+    return HcommMoeCombineRows(handle, y, handle ? (uint64_t)((MoeCtx *)handle)->lay.maxRecvRows : 0, gates, out, numTokens, stream);
+}
+
+int HcommMoeCombineRows(void *handle, const void *y, uint64_t yRows, const float *gates, void *out, int numTokens, void *stream)
+{
     MoeCtx *m = (MoeCtx *)handle;
     if (!m || !y || !gates || !out) return HCCL_E_PTR;
     if (numTokens < 0 || numTokens > m->lay.maxTokens) return HCCL_E_PARA;
@@ -718,9 +733,16 @@ int HcommMoeCombine(void *handle, const void *y, const float *gates, void *out, 
     FillCommon(m, hp);
     hp.y = (const __nv_bfloat16 *)y; hp.gates = gates; hp.out = (__nv_bfloat16 *)out; hp.numTokens = numTokens;
     ++c->opSeq;
+    const uintptr_t yBegin = (uintptr_t)y, yEnd = yBegin + yRows * m->lay.hidden * 2;
+    const uintptr_t outBegin = (uintptr_t)out, outEnd = outBegin + (uint64_t)numTokens * m->lay.hidden * 2;
+    hp.allThroughSlots = m->slotsAsked.load() || (outBegin < yEnd && yBegin < outEnd);
     const int sms = MoeSms(), emuCtas = std::max(1, sms / (int)c->nRanks), segs = m->lay.hidden / 256;
-    if (c->nRanks > 1) CHK_RET(LaunchMoe(m, (void *)MoeCombineSendKernel, hp, 9102, stream, MoeCtas(c, sms, 0), emuCtas, 512));
-    else hp.countsLaunch = 1;
+    if (c->nRanks > 1 || hp.allThroughSlots) {
+        const int forced = ForcedMoeCtas();
+        CHK_RET(LaunchMoe(m, (void *)MoeCombineSendKernel, hp, 9102, stream, forced > 0 ? forced : std::min(sms, HC_MAX_CTAS), emuCtas, 512));
+    } else {
+        hp.countsLaunch = 1;
+    }
     // four segments to a warp where that still fills every SM's warps (the row addresses are then found once for all four),
     // single segments below
     constexpr int warps = kSumThreads / 32;

@@ -66,8 +66,8 @@ class MoeExchange:
         self.layout = MoeLayout()
         _lib.check(self._lib.HcommMoeCreate(ctypes.c_void_p(comm.handle), num_experts, topk, hidden, max_tokens, ctypes.c_float(capacity_factor),
                                             ctypes.byref(self._h), ctypes.byref(self.layout)), "HcommMoeCreate")
-        ptrs = [ctypes.c_void_p() for _ in range(5)]
-        _lib.check(self._lib.HcommMoeGetBuffers(self._h, *[ctypes.byref(p) for p in ptrs]), "HcommMoeGetBuffers")
+        ptrs = [ctypes.c_void_p() for _ in range(4)]          # not the landing area: combine then reads local rows where y holds them
+        _lib.check(self._lib.HcommMoeGetBuffers(self._h, *[ctypes.byref(p) for p in ptrs], None), "HcommMoeGetBuffers")
         dev = torch.device("cuda", torch.cuda.current_device())
         cap, epr = self.layout.maxRecvRows, num_experts // comm.size
         self._rows = _view(ptrs[0].value, (cap, hidden), torch.uint8, dev).view(torch.float8_e4m3fn)
@@ -92,8 +92,8 @@ class MoeExchange:
         if out is None:
             out = torch.empty((t, self.hidden), dtype=torch.bfloat16, device=y.device)
         stream = raw_stream(y)
-        _lib.check(self._lib.HcommMoeCombine(self._h, ctypes.c_void_p(y.data_ptr()), ctypes.c_void_p(gates.data_ptr()), ctypes.c_void_p(out.data_ptr()), t,
-                                             ctypes.c_void_p(stream)), "HcommMoeCombine")
+        _lib.check(self._lib.HcommMoeCombineRows(self._h, ctypes.c_void_p(y.data_ptr()), ctypes.c_uint64(y.shape[0]), ctypes.c_void_p(gates.data_ptr()),
+                                                 ctypes.c_void_p(out.data_ptr()), t, ctypes.c_void_p(stream)), "HcommMoeCombineRows")
         return out
 
     def overflow(self) -> int:

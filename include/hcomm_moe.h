@@ -19,7 +19,8 @@ struct MoeLayout {
     uint64_t offOrigin;          // u64 [maxRecvRows]                 (source rank << 32) | (token * topk + k)
     uint64_t offScales;          // f32 [maxRecvRows][hidden / 128]
     uint64_t offRows;            // fp8 e4m3 [maxRecvRows][hidden]
-    uint64_t offCombine;         // bf16 [maxTokens][topk][hidden]    landing area of the combine step: rows from other ranks
+    uint64_t offCombine;         // bf16 [maxTokens][topk][hidden]    landing area of the combine step: rows from other ranks, from all
+                                 //                                   once HcommMoeGetBuffers has been asked for its address
     uint64_t totalBytes;
     uint64_t offValid;           // u8 [maxTokens][topk]              1 = dispatch sent this (token, k), 0 = masked or dropped
 };
@@ -31,12 +32,17 @@ typedef struct MoeLayout MoeLayout;
  * and maps its peers'.  numExperts a multiple of the rank count (<= 1024), topk <= 16, hidden a multiple of 512 (<= 8192). */
 int HcommMoeCreate(HcclComm comm, int numExperts, int topk, int hidden, int maxTokens, float capacityFactor, void **handle, MoeLayout *layoutOut);
 int HcommMoeDestroy(void *handle);
-/* Local addresses of the receive-side arrays (valid after a dispatch on the same stream). */
+/* Local addresses of the receive-side arrays (valid after a dispatch on the same stream; any may be NULL).  Asking for
+ * `combine` makes every later HcommMoeCombine place the row of each (token, k) that was sent in that area, those of this
+ * rank's own experts as well; until then these are summed where y holds them, which is faster. */
 int HcommMoeGetBuffers(void *handle, void **rows, void **scales, void **origin, void **expertOffsets, void **combine);
 /* x: bf16 [numTokens][hidden]; topkIdx: int32 [numTokens][topk], an index outside [0, numExperts) masks that choice. */
 int HcommMoeDispatch(void *handle, const void *x, const int32_t *topkIdx, int numTokens, void *stream);
-/* y: bf16 expert outputs in receive-row order; gates: f32 [numTokens][topk]; out: bf16 [numTokens][hidden]. */
+/* y: bf16 expert outputs in receive-row order; gates: f32 [numTokens][topk]; out: bf16 [numTokens][hidden], which may lie
+ * inside y.  HcommMoeCombineRows is told how many rows the memory at y has room for; HcommMoeCombine assumes the receive
+ * capacity, and takes a result that starts behind a shorter y for one inside it (same result, a pass more). */
 int HcommMoeCombine(void *handle, const void *y, const float *gates, void *out, int numTokens, void *stream);
+int HcommMoeCombineRows(void *handle, const void *y, uint64_t yRows, const float *gates, void *out, int numTokens, void *stream);
 /* Rows dropped because a rank received more than its capacity since the last call (clears the counter). */
 int HcommMoeTakeOverflow(void *handle);
 

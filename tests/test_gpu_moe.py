@@ -206,3 +206,75 @@ def test_combine_of_more_tokens_than_were_dispatched_adds_nothing_for_the_rest()
     finally:
         moe.destroy()
         comm.destroy()
+
+
+@pytest.mark.parametrize("n", [1, 2])
+@pytest.mark.parametrize("hidden,tokens", [(512, 5), (1024, 300)])
+def test_result_inside_the_experts_output_and_rows_in_the_landing_area(n, hidden, tokens):
+    """A result that overlaps the experts' output overwrites rows that other tokens still need: the sum is the one that a
+    result elsewhere gets, wherever in y it lies.  And a caller that asks for the landing area finds every row that was sent
+    in its slot (token, k), those of its own rank's experts too."""
+    import ctypes
+    import hcomm_b200 as hb
+    from hcomm_b200 import _lib
+    from hcomm_b200.ops.moe import MoeExchange, _view
+    experts, topk = 8, 4
+    info = hb.get_root_info()
+
+    def init(r):
+        torch.cuda.set_device(0)
+        return hb.Communicator(n, info, r, buffer_mb=8)
+    comms = run_ranks(n, init)
+    moes = run_ranks(n, lambda r: (torch.cuda.set_device(0), MoeExchange(comms[r], experts, topk, hidden, tokens, capacity_factor=2.0))[1])
+    try:
+        g = torch.Generator(device="cuda").manual_seed(hidden)
+        xs = [torch.randn(tokens, hidden, device="cuda", generator=g).to(torch.bfloat16) for _ in range(n)]
+        idx = [torch.rand(tokens, experts, device="cuda", generator=g).topk(topk, dim=1).indices.to(torch.int32).contiguous() for _ in range(n)]
+        gates = [torch.rand(tokens, topk, device="cuda", generator=g) for _ in range(n)]
+        idx[0][::3, 1] = -1
+        want, slots = [None] * n, [None] * n
+
+        def plain(r):
+            torch.cuda.set_device(0)
+            rec = moes[r].dispatch(xs[r], idx[r])
+            torch.cuda.synchronize()
+            y = rec.dequantized().to(torch.bfloat16)
+            want[r] = moes[r].combine(y, gates[r])
+            torch.cuda.synchronize()
+        run_ranks(n, plain)
+
+        for where in ("start", "middle", "end"):
+            def inside(r):
+                torch.cuda.set_device(0)
+                rec = moes[r].dispatch(xs[r], idx[r])
+                torch.cuda.synchronize()
+                rows = rec.num_rows
+                y = torch.zeros(max(rows, tokens) + tokens, hidden, device="cuda", dtype=torch.bfloat16)
+                y[:rows] = rec.dequantized(rows).to(torch.bfloat16)
+                at = {"start": 0, "middle": rows // 3, "end": max(0, rows - tokens)}[where]
+                out = moes[r].combine(y, gates[r], out=y[at:at + tokens])
+                torch.cuda.synchronize()
+                assert torch.equal(out, want[r]), where
+            run_ranks(n, inside)
+
+        def asked(r):
+            torch.cuda.set_device(0)
+            ptr = ctypes.c_void_p()
+            assert _lib.load().HcommMoeGetBuffers(moes[r]._h, None, None, None, None, ctypes.byref(ptr)) == 0
+            rec = moes[r].dispatch(xs[r], idx[r])
+            torch.cuda.synchronize()
+            out = moes[r].combine(rec.dequantized().to(torch.bfloat16), gates[r])
+            torch.cuda.synchronize()
+            assert torch.equal(out, want[r])
+            slots[r] = _view(ptr.value, (tokens, topk, hidden), torch.bfloat16, torch.device("cuda", 0)).clone()
+        run_ranks(n, asked)
+        for r in range(n):
+            q = moes[r].sent[:tokens].bool()
+            # every expert here returns the dequantised token, so each slot that was sent holds it
+            from hcomm_b200.ops.moe import quantize_e4m3_1x128
+            f8, sc = quantize_e4m3_1x128(xs[r])
+            row = (f8.float().view(tokens, -1, 128) * sc.unsqueeze(-1)).view(tokens, 1, hidden).to(torch.bfloat16)
+            assert bool(q.any()) and torch.equal(slots[r][q], row.expand(-1, topk, -1)[q])
+    finally:
+        run_ranks(n, lambda r: moes[r].destroy())
+        run_ranks(n, lambda r: comms[r].destroy())
