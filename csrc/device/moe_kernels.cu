@@ -478,6 +478,36 @@ struct MoeCtx {
 std::mutex g_mu;
 std::map<void *, MoeCtx *> g_ctx;
 
+// Where an exchange's own device block comes from; a test puts failing functions in their place.
+struct DeviceBlocks {
+    cudaError_t (*take)(void **, size_t);
+    cudaError_t (*clear)(void *, int, size_t);
+    cudaError_t (*give)(void *);
+};
+// One block: the row cursors, the overflow count and the last dispatch's tokens, the local rows.  On failure nothing is kept.
+HcclResult MakeScratch(const DeviceBlocks &from, MoeCtx *m, int numExperts, int maxTokens, int topk)
+{
+    const size_t bytes = sizeof(uint32_t) * (2 * (size_t)numExperts + 64 + (size_t)maxTokens * topk);
+    void *block = nullptr;
+    cudaError_t e = from.take(&block, bytes);
+    if (e != cudaSuccess || !block) {
+        HCCL_ERROR("MoE exchange: no device memory for its %zu bytes of counters and row numbers: %s", bytes, cudaGetErrorString(e));
+        cudaGetLastError();
+        return HCCL_E_MEMORY;
+    }
+    e = from.clear(block, 0, bytes);
+    if (e != cudaSuccess) {
+        HCCL_ERROR("MoE exchange: clearing its counters failed: %s", cudaGetErrorString(e));
+        cudaGetLastError();
+        from.give(block);
+        return HCCL_E_RUNTIME;
+    }
+    m->scratch = (uint32_t *)block;
+    m->overflow = m->scratch + 2 * numExperts;
+    m->localRow = m->overflow + 64;
+    return HCCL_SUCCESS;
+}
+
 uint64_t Align256(uint64_t v) { return (v + 255) & ~255ull; }
 
 // HCOMM_MOE_CTAS: CTAs of the data-moving launches, to leave SMs to kernels running beside them (0 = not set).
@@ -621,20 +651,16 @@ int HcommMoeCreate(HcclComm comm, int numExperts, int topk, int hidden, int maxT
     L.totalBytes = off;
     HcclResult r = (HcclResult)HcommMemAlloc(&m->buf, L.totalBytes);
     if (r != HCCL_SUCCESS) { delete m; return r; }
+    r = MakeScratch({[](void **p, size_t n) { return cudaMalloc(p, n); }, cudaMemset, cudaFree}, m, numExperts, maxTokens, topk);
+    if (r != HCCL_SUCCESS) { HcommMemFree(m->buf); delete m; return r; }
     cudaMemset(m->buf, 0, L.offOrigin);
     r = HcclCommSymWinRegister(comm, m->buf, L.totalBytes, &m->win, 0);
-    if (r != HCCL_SUCCESS) { HcommMemFree(m->buf); delete m; return r; }
+    if (r != HCCL_SUCCESS) { cudaFree(m->scratch); HcommMemFree(m->buf); delete m; return r; }
     for (int q = 0; q < n; ++q) {
         void *pp = nullptr;
         HcclSymWinGetPeerPointer(m->win, 0, (uint32_t)q, &pp);
         m->peer[q] = (char *)pp;
     }
-    // one block: the row cursors, the overflow count and the last dispatch's tokens, the local rows
-    const size_t words = 2 * (size_t)numExperts + 64 + (size_t)maxTokens * topk;
-    cudaMalloc(&m->scratch, sizeof(uint32_t) * words);
-    cudaMemset(m->scratch, 0, sizeof(uint32_t) * words);
-    m->overflow = m->scratch + 2 * numExperts;
-    m->localRow = m->overflow + 64;
     cudaGetDevice(&m->device);
     m->staticScratch = ResolveStaticScratch();       // set-up time, the exchange's GPU is current
     cudaFuncAttributes fa;
@@ -796,6 +822,29 @@ int HcommMoeDispatchStaticScratch(void *handle, const void *x, const int32_t *to
     hp.x = (const __nv_bfloat16 *)x; hp.topkIdx = topkIdx; hp.numTokens = numTokens;
     ++c->opSeq;
     return LaunchDispatch(m, hp, 9105, 9103, stream);
+}
+
+// An exchange's device block from stand-in allocators in host memory: failing 0 = none, 1 = taking it, 2 = clearing it.
+// *blocksLeft: blocks taken and not given back.  Returns what HcommMoeCreate would; on success the parts' offsets in words.
+int HcommToolMoeScratch(int numExperts, int maxTokens, int topk, int failing, int *blocksLeft, uint64_t *overflowAt, uint64_t *localRowAt)
+{
+    static thread_local int fail, taken;
+    fail = failing;
+    taken = 0;
+    const DeviceBlocks host = {[](void **p, size_t n) { if (fail == 1) return cudaErrorMemoryAllocation; ++taken; *p = malloc(n); return *p ? cudaSuccess : cudaErrorMemoryAllocation; },
+                               [](void *p, int v, size_t n) { if (fail == 2) return cudaErrorUnknown; memset(p, v, n); return cudaSuccess; },
+                               [](void *p) { --taken; free(p); return cudaSuccess; }};
+    MoeCtx m;
+    const HcclResult r = MakeScratch(host, &m, numExperts, maxTokens, topk);
+    if (blocksLeft) *blocksLeft = taken;
+    if (r == HCCL_SUCCESS) {
+        if (overflowAt) *overflowAt = (uint64_t)(m.overflow - m.scratch);
+        if (localRowAt) *localRowAt = (uint64_t)(m.localRow - m.scratch);
+        free(m.scratch);
+    } else if (m.scratch || m.overflow || m.localRow) {
+        return HCCL_E_INTERNAL;             // a part of a block that is not there
+    }
+    return r;
 }
 
 // Rows dropped because a rank received more than its capacity since the last call (clears the counter).
