@@ -234,17 +234,23 @@ cudaLaunchConfig_t PairConfig(cudaLaunchAttribute *at, int clusters, int cluster
     return cfg;
 }
 
+hcgemm::SwapShape ShapeOf(int M, int N, int K, int bn)
+{
+    hcgemm::SwapShape g = {};
+    g.M = M; g.N = N; g.K = K;
+    g.tilesW = (N + hcgemm::kPairM - 1) / hcgemm::kPairM;
+    g.tilesT = (M + bn - 1) / bn;
+    g.bn = bn; g.stages = hcgemm::SwapStages(bn);
+    g.group = std::min(PairGroupRows(K), g.tilesW);     // a group that the caller forces may be any number
+    return g;
+}
+
 HcclResult LaunchSwapGemm(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, const PairTile &tile, void *stream)
 {
     CUtensorMap tmW, tmX;
     CHK_RET(MakeTensorMap2dBf16(&tmW, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, hcgemm::kBlockM, hcgemm::kBlockK));
     CHK_RET(MakeTensorMap2dBf16(&tmX, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)(tile.bn / 2), hcgemm::kBlockK));
-    hcgemm::SwapShape g;
-    g.M = M; g.N = N; g.K = K;
-    g.tilesW = (N + hcgemm::kPairM - 1) / hcgemm::kPairM;
-    g.tilesT = (M + tile.bn - 1) / tile.bn;
-    g.bn = tile.bn; g.stages = hcgemm::SwapStages(tile.bn);
-    g.group = PairGroupRows(K);
+    hcgemm::SwapShape g = ShapeOf(M, N, K, tile.bn);
     g.C = (__nv_bfloat16 *)C; g.ldc = ldc;
     g.errFlag = GemmErrorFlag();
     const int tiles = g.tilesW * g.tilesT;
@@ -368,6 +374,13 @@ extern "C" void HcommToolGemmTile(int M, int N, int K, int cap1, int cap2, int c
     const hc::PairTile t = hc::PickPairTile(M, N, K, cap);
     if (tileWidth) *tileWidth = t.bn;
     if (pairsAlongK) *pairsAlongK = t.split;
+}
+// The blocks (256 weights, tileWidth tokens) of tile t of the GEMM with exchanged operands; returns the number of tiles.
+extern "C" int HcommToolGemmOrder(int M, int N, int K, int tileWidth, int t, int *weightBlock, int *tokenBlock)
+{
+    const hcgemm::SwapShape g = hc::ShapeOf(M, N, K, tileWidth);
+    if (t >= 0 && t < g.tilesW * g.tilesT) hcgemm::SwapOrder(g, t, weightBlock, tokenBlock);
+    return g.tilesW * g.tilesT;
 }
 // Kept for callers of earlier versions, which could time a shape at its first use: no measurement is made (0 / 0).
 extern "C" void HcommGemmGetTuned(int, int, int, int *tileWidth, int *groupRows)

@@ -35,11 +35,21 @@ struct SwapShape {
     int M, N, K;
     int tilesW, tilesT;      // blocks of 256 weights, of bn tokens
     int bn, stages;
-    int group;               // weight blocks per rasterisation group
+    int group;               // weight blocks per rasterisation group, 1 .. tilesW
     __nv_bfloat16 *C;
     int ldc;
     uint32_t *errFlag;
 };
+
+// Tile t's block of weights and of tokens: walks the weight blocks of a group for one token block, then for the next, so that
+// the pairs in flight share both operands' panels in L2.
+__host__ __device__ inline void SwapOrder(const SwapShape &g, int t, int *wb, int *tb)
+{
+    const int perGroup = g.group * g.tilesT, gi = t / perGroup, rem = t % perGroup;
+    const int left = g.tilesW - gi * g.group, here = left < g.group ? left : g.group;
+    *tb = rem / here;
+    *wb = gi * g.group + rem % here;
+}
 
 __host__ __device__ constexpr int SwapStageBytes(int bn) { return (kBlockM + bn / 2) * kBlockK * 2; }
 constexpr int kSwapFixedSmem = 8 * kSwapSlab + (int)sizeof(SwapState) + 1024 /* alignment slack */;
@@ -91,13 +101,6 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
     const int kBlocks = (g.K + kBlockK - 1) / kBlockK;
     const int kFirst = kBlocks * part / SPLIT, kLast = kBlocks * (part + 1) / SPLIT;
     const int firstTile = (int)ClusterId(), tileStep = (int)NumClusters();
-    // walk the weight blocks of a group for one token block, then the next: the pairs in flight share both operands' panels in L2
-    auto order = [&](int t, int *wb, int *tb) {
-        const int perGroup = g.group * g.tilesT, gi = t / perGroup, rem = t % perGroup;
-        const int left = g.tilesW - gi * g.group, here = left < g.group ? left : g.group;
-        *tb = rem / here;
-        *wb = gi * g.group + rem % here;
-    };
 
     if (threadIdx.x < (unsigned)g.stages) {
         MbarInit(&st->full[threadIdx.x], 1);
@@ -130,7 +133,7 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
             bool alive = true;
             for (int t = firstTile; t < numTiles && alive; t += tileStep) {
                 int wb, tb;
-                order(t, &wb, &tb);
+                SwapOrder(g, t, &wb, &tb);
                 const int wRow = (wb * 2 + half) * kBlockM, xRow = tb * g.bn + half * (g.bn / 2);
                 for (int kb = kFirst; kb < kLast; ++kb) {
                     if (!MbarWait(&st->empty[s], ph ^ 1, &st->abort)) { alive = false; break; }
@@ -182,7 +185,7 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
         bool alive = true;
         for (int t = firstTile; t < numTiles && alive; t += tileStep, ++tileIter) {
             int wb, tb;
-            order(t, &wb, &tb);
+            SwapOrder(g, t, &wb, &tb);
             const uint32_t acc = tileIter & 1, accPh = (tileIter >> 1) & 1;
             if (!MbarWait(&st->tmemFull[acc], accPh, &st->abort)) { alive = false; break; }
             TcFenceAfter();
@@ -226,7 +229,7 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
         // landed and all MMAs that read them have finished.
         const int q = warp & 3, odd = (warp - 2) >> 2;
         int wb, tb;
-        order(firstTile, &wb, &tb);
+        SwapOrder(g, firstTile, &wb, &tb);
         const int tokens = g.M - tb * g.bn < g.bn ? g.M - tb * g.bn : g.bn;
         if (MbarWait(&st->tmemFull[0], 0, &st->abort)) {
             TcFenceAfter();
@@ -246,7 +249,7 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
     ClusterSync();
     if constexpr (SPLIT > 1) {
         int wb, tb;
-        order(firstTile, &wb, &tb);
+        SwapOrder(g, firstTile, &wb, &tb);
         const int t0 = tb * g.bn, tokens = g.M - t0 < g.bn ? g.M - t0 : g.bn;
         const int per = (tokens + SPLIT - 1) / SPLIT, lo = part * per, hi = lo + per < tokens ? lo + per : tokens;
         const int n = wb * kPairM + half * kBlockM + lane * 4;

@@ -25,7 +25,8 @@ extern "C" {
 
 /* C[M,N] = A[M,K] * B[N,K]^T on the current device.  N, K and ldc multiples of 8, C 16-byte aligned. */
 int HcommGemmBf16(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, void *stream);
-/* Tuning overrides of the CTA-pair GEMM kernels (0 = automatic): rasterisation group in 256-row blocks; tile width in rows of A
+/* Tuning overrides of the CTA-pair GEMM kernels (0 = automatic): rasterisation group in blocks of 256 rows (of
+ * B in the plain GEMM, of A where its tiles are 256 x 512 and in the fused kernels; more blocks than there are count as all); tile width in rows of A
  * for the plain GEMM (32..256, rounded down to a multiple of 32; 512: tiles of 256 rows of A x 512 rows of B), in columns for
  * the fused kernels (128..256, multiple of 32). */
 void HcommGemmSetTuning(int groupRows, int tileWidth);

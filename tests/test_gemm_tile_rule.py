@@ -40,3 +40,23 @@ def test_known_choices():
     assert pick(8192, 28672, 8192, caps) == (512, 1)    # 25 full waves: the least operand traffic
     assert pick(777, 14336, 4096, caps) == (160, 1)     # 800 columns of work for 777 tokens
     assert pick(8192, 3584, 8192, caps) == (224, 1)     # seven full waves instead of eight of 256 columns
+
+
+@pytest.mark.parametrize("group", [0, 1, 3, 1000, 1 << 28, 1 << 30, 2147483647])
+@pytest.mark.parametrize("m,n,width", [(1000, 5000, 256), (33, 128256, 64), (700, 256, 32), (8192, 8, 224)])
+def test_every_tile_is_walked_once_whatever_group_is_asked_for(m, n, width, group):
+    lib = _lib.load()
+    wb, tb = ctypes.c_int(), ctypes.c_int()
+    lib.HcommGemmSetTuning(group, 0)
+    try:
+        total = lib.HcommToolGemmOrder(m, n, 4096, width, -1, None, None)
+        blocks_w, blocks_t = -(-n // 256), -(-m // width)
+        assert total == blocks_w * blocks_t
+        seen = set()
+        for t in range(total):
+            lib.HcommToolGemmOrder(m, n, 4096, width, t, ctypes.byref(wb), ctypes.byref(tb))
+            assert 0 <= wb.value < blocks_w and 0 <= tb.value < blocks_t
+            seen.add((wb.value, tb.value))
+        assert len(seen) == total
+    finally:
+        lib.HcommGemmSetTuning(0, 0)

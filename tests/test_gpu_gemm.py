@@ -110,3 +110,21 @@ def test_back_to_back_calls_see_each_others_results(m, h, i):
     for _ in range(3):
         assert torch.equal(chain(False), want)
     assert take_kernel_error() == 0
+
+
+@pytest.mark.parametrize("width", [32, 256, 512])
+def test_oversized_raster_group(width):
+    from hcomm_b200 import _lib
+    from hcomm_b200.ops.gemm import gemm_bf16, take_kernel_error
+    lib = _lib.load()
+    a = torch.randn(1000, 256, device="cuda").to(torch.bfloat16)
+    b = torch.randn(776, 256, device="cuda").to(torch.bfloat16)
+    lib.HcommGemmSetTuning(0, width)
+    want = gemm_bf16(a, b)
+    try:
+        lib.HcommGemmSetTuning(1 << 30, width)          # times the number of token blocks this is no 32-bit number
+        got = gemm_bf16(a, b)
+        torch.cuda.synchronize()
+    finally:
+        lib.HcommGemmSetTuning(0, 0)
+    assert take_kernel_error() == 0 and torch.equal(got, want)
