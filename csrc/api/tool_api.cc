@@ -9,6 +9,7 @@
 #include "../alg/templates.h"
 #include "../core/env.h"
 #include "../core/log.h"
+#include "../core/per_device.h"
 #include "../plat/platform.h"
 #include "../topo/nvml_topo.h"
 #include "../topo/rank_graph.h"
@@ -141,6 +142,16 @@ int HcommToolSelect(int cmd, uint32_t nRanks, uint64_t bytes, int dtype, int op,
     if (r != HCCL_SUCCESS) { Out(out, outLen, "not supported"); return (int)r; }
     Out(out, outLen, sel.name);
     return 0;
+}
+
+// A series of questions to a per-device value: call i is made on devices[i], where the device would answer answers[i] (0 or
+// less: the query fails).  values[i] is what the caller gets; returns how often a device was asked.
+int HcommToolPerDevice(int calls, const int *devices, const int *answers, int *values)
+{
+    PerDevice<int> kept;
+    int asked = 0;
+    for (int i = 0; i < calls; ++i) values[i] = kept.Get(devices[i], [&](int *v) { ++asked; *v = answers[i]; return *v > 0; });
+    return asked;
 }
 
 // Simulator ranks of this process lose their next n flag writes (a message that the test drops): the peers' waits

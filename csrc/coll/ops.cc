@@ -17,6 +17,7 @@
 #include "../core/env.h"
 #include "../core/log.h"
 #include "../core/nvtx_range.h"
+#include "../core/per_device.h"
 #include "../device/coll_kernels.h"
 #include "../device/emu_launch.h"
 #include "exec.h"
@@ -198,7 +199,9 @@ bool TryLocal(Comm *c, const OpDesc &d, HcclResult *res)
     }
     // two rounds of the CTAs that fit at once (two of 512 threads per SM: 64 KB of loads in flight); small operands spread in
     // shares of 32 KB, four 16-byte words per thread
-    static const uint64_t most = 2 * (uint64_t)std::max(1, FastMaxCoResidentCtas(FK_LOCAL, 512, 0));
+    static PerDevice<int> resident;
+    const int fit = resident.Get(c->device, [](int *n) { return (*n = FastMaxCoResidentCtas(FK_LOCAL, 512, 0)) > 0; });
+    const uint64_t most = 2 * (uint64_t)std::max(1, fit);
     int ctas = (int)std::max<uint64_t>(1, std::min<uint64_t>(most, (count * esz + 32767) / 32768));
     const int cap = EnvConfig::Get().maxCtas.value, forced = EnvConfig::Get().forceCtas.value;
     const uint32_t own = __atomic_load_n(&c->ctaLimit, __ATOMIC_RELAXED);

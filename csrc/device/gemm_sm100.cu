@@ -8,6 +8,7 @@
 #include <mutex>
 
 #include "../core/log.h"
+#include "../core/per_device.h"
 #include "gemm_api.h"
 #include "gemm_sm100.cuh"
 #include "gemm_sm100_2sm_wide.cuh"
@@ -42,9 +43,22 @@ GemmBf16SwapKernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     hcgemm::GemmMainLoopSwap<SPLIT>(&tmW, &tmX, shape);
 }
 
-template <int SPLIT> int SwapCapacityOf()
+// What the plain GEMM's kernels find on a device: clusters of 1, 2 and 4 CTA pairs that it holds at once, 0 where a kernel
+// cannot run, and whether the kernels without pairs have their shared memory.
+struct GemmLimits {
+    int cap[3];
+    bool single;
+};
+template <typename Kernel> bool AllowShared(Kernel *kernel, int bytes)
 {
-    if (cudaFuncSetAttribute(GemmBf16SwapKernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) { cudaGetLastError(); return 0; }
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+template <int SPLIT> bool ClustersAtOnce(int *n)
+{
+    *n = 0;
+    if (!AllowShared(GemmBf16SwapKernel<SPLIT>, 227 * 1024)) return false;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * SPLIT * 148, 1, 1);
     cfg.blockDim = dim3(hcgemm::kSwapThreads, 1, 1);
@@ -53,28 +67,23 @@ template <int SPLIT> int SwapCapacityOf()
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2 * SPLIT; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, GemmBf16SwapKernel<SPLIT>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
-    HCCL_INFO("GEMM clusters of %d CTAs resident at once: %d", 2 * SPLIT, n);
-    return n;
+    if (cudaOccupancyMaxActiveClusters(n, GemmBf16SwapKernel<SPLIT>, &cfg) != cudaSuccess) { cudaGetLastError(); *n = 0; return false; }
+    HCCL_INFO("GEMM clusters of %d CTAs resident at once: %d", 2 * SPLIT, *n);
+    return true;
 }
-// Clusters of 2^log2Pairs CTA pairs that the current device holds at once (0 when the query fails).  The kernels' shared
-// memory limits are a device's own, so the first call on each device sets them.
-int SwapCapacity(int log2Pairs)
+// The limits of the current device: shared memory limits are a device's own, so its first call sets them.
+GemmLimits Limits()
 {
-    constexpr int kDevices = 16;
-    static std::once_flag once[kDevices];
-    static int cap[kDevices][3];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) { cudaGetLastError(); return 0; }
-    std::call_once(once[dev], [dev] {
-        const bool wide = cudaFuncSetAttribute(GemmBf16PairWideKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::ConfigWide<4>::kSmemBytes) == cudaSuccess;
-        if (!wide) cudaGetLastError();
-        cap[dev][0] = wide ? SwapCapacityOf<1>() : 0;
-        cap[dev][1] = SwapCapacityOf<2>();
-        cap[dev][2] = SwapCapacityOf<4>();
+    static PerDevice<GemmLimits> limits;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return {}; }
+    return limits.Get(dev, [](GemmLimits *l) {
+        const bool wide = AllowShared(GemmBf16PairWideKernel, hcgemm::ConfigWide<4>::kSmemBytes);
+        const bool one = ClustersAtOnce<1>(&l->cap[0]), two = ClustersAtOnce<2>(&l->cap[1]), four = ClustersAtOnce<4>(&l->cap[2]);
+        if (!wide) l->cap[0] = 0;
+        l->single = AllowShared(GemmBf16Kernel<256>, hcgemm::Config<256>::kSmemBytes) && AllowShared(GemmBf16Kernel<128>, hcgemm::Config<128>::kSmemBytes);
+        return wide && one && two && four && l->single;
     });
-    return cap[dev][log2Pairs];
 }
 
 }  // namespace
@@ -255,7 +264,7 @@ HcclResult LaunchSwapGemm(const void *A, const void *B, void *C, int M, int N, i
     g.errFlag = GemmErrorFlag();
     const int tiles = g.tilesW * g.tilesT;
     cudaLaunchAttribute at[2];
-    const cudaLaunchConfig_t cfg = PairConfig(at, tile.split > 1 ? tiles : std::min(SwapCapacity(0), tiles), 2 * tile.split, hcgemm::kSwapThreads,
+    const cudaLaunchConfig_t cfg = PairConfig(at, tile.split > 1 ? tiles : std::min(Limits().cap[0], tiles), 2 * tile.split, hcgemm::kSwapThreads,
                                               hcgemm::SwapSmemBytes(tile.bn), stream);
     cudaError_t e;
     switch (tile.split) {
@@ -285,15 +294,14 @@ HcclResult LaunchWideGemm(const void *A, const void *B, void *C, int M, int N, i
     // a wave of 74 such tiles loads the fewest panels at 12 rows x 6 columns
     const int rows = PairGroupRows(K), group = g_forceGm.load() > 0 || rows >= 16 ? rows : 12;
     cudaLaunchAttribute at[2];
-    const cudaLaunchConfig_t cfg = PairConfig(at, std::min(SwapCapacity(0), shape.tilesM * shape.tilesN), 2, hcgemm::kWideThreads, hcgemm::ConfigWide<4>::kSmemBytes, stream);
+    const cudaLaunchConfig_t cfg = PairConfig(at, std::min(Limits().cap[0], shape.tilesM * shape.tilesN), 2, hcgemm::kWideThreads, hcgemm::ConfigWide<4>::kSmemBytes, stream);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, GemmBf16PairWideKernel, tmA, tmB, tmC, shape, group);
     if (e != cudaSuccess) { HCCL_ERROR("GemmBf16 (256 x 512 tiles) launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
 
-PairTile ChoosePairTile(int M, int N, int K)
+PairTile ChoosePairTile(int M, int N, int K, const int (&cap)[3])
 {
-    const int cap[3] = {SwapCapacity(0), SwapCapacity(1), SwapCapacity(2)};
     PairTile t = PickPairTile(M, N, K, cap);
     const int bn = ForcedPairTileWidth(), split = g_forceSplit.load(), kBlocks = (K + hcgemm::kBlockK - 1) / hcgemm::kBlockK;
     if (bn >= hcgemm::kWideN) t = {hcgemm::kWideN, 1};
@@ -312,8 +320,9 @@ HcclResult GemmBf16(const void *A, const void *B, void *C, int M, int N, int K, 
         return HCCL_E_PARA;
     }
     static const bool pairEnabled = [] { const char *e = getenv("HCOMM_GEMM_PAIR"); return !(e && e[0] == '0'); }();
-    if (pairEnabled && SwapCapacity(0) > 0) {
-        const PairTile tile = ChoosePairTile(M, N, K);
+    const GemmLimits limits = Limits();
+    if (pairEnabled && limits.cap[0] > 0) {
+        const PairTile tile = ChoosePairTile(M, N, K, limits.cap);
         return tile.bn == hcgemm::kWideN ? LaunchWideGemm(A, B, C, M, N, K, lda, ldb, ldc, stream)
                                          : LaunchSwapGemm(A, B, C, M, N, K, lda, ldb, ldc, tile, stream);
     }
@@ -332,12 +341,8 @@ HcclResult GemmBf16(const void *A, const void *B, void *C, int M, int N, int K, 
     int grid = std::min(GemmSmCount(), shape.tilesM * shape.tilesN);
     cudaError_t e;
     if (BN == 256) {
-        static bool attr = false;
-        if (!attr) { cudaFuncSetAttribute(GemmBf16Kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::Config<256>::kSmemBytes); attr = true; }
         GemmBf16Kernel<256><<<grid, hcgemm::kThreads, hcgemm::Config<256>::kSmemBytes, (cudaStream_t)stream>>>(tmA, tmB, shape, epi);
     } else {
-        static bool attr = false;
-        if (!attr) { cudaFuncSetAttribute(GemmBf16Kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, hcgemm::Config<128>::kSmemBytes); attr = true; }
         GemmBf16Kernel<128><<<grid, hcgemm::kThreads, hcgemm::Config<128>::kSmemBytes, (cudaStream_t)stream>>>(tmA, tmB, shape, epi);
     }
     e = cudaGetLastError();
