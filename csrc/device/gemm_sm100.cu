@@ -182,16 +182,21 @@ namespace {
 
 // Tile of the CTA-pair kernels for a shape: tokens per tile and pairs that share a tile along K for the one with exchanged
 // operands (gemm_sm100_swap.cuh), or 256 x 512 (gemm_sm100_2sm_wide.cuh).  The estimate below, in nanoseconds, was fitted to
-// about 120 timings (M 1 .. 8192, N 1024 .. 128256, K 1024 .. 28672) and agrees with nearly all of them within 10 %:
+// timings of every tile at about 1600 shapes (M 1 .. 65536, N 8 .. 128256, K 64 .. 28672):
 //   * a 64-deep step of a 256 x bn tile takes 48 + 1.28 bn ns on the tensor core at the clock that a GPU under such load
 //     holds, but never less than its operands (16 KB of weights, 128 bytes per token and CTA) at 120 bytes per ns and SM;
 //   * tiles come in whole waves of the clusters that fit at once (74 of two CTAs, 33 of four, 15 of eight);
-//   * all operand traffic passes L2 at 13.5 TB/s, every operand comes from HBM once at 6.5 TB/s, a tenth less when only a
+//   * a tile's accumulator is emptied while the next tile is multiplied, in 1 us and 0.5 for every 64 tokens begun.  Where K is
+//     shallow neither hides the other: measured, the two add up like the sides of a right angle (256 tokens, K of 64 / 256 /
+//     512: 2.7 / 3.1 / 4.2 us a tile; multiplying alone 0.4 / 1.5 / 3.0), which makes wide tiles the better ones:
+//     65536 x 4096 x 64 takes 119 us with 512/1, 310 with 64/1;
+//   * all operand traffic passes L2 at 13.5 TB/s, half as much again where K is no multiple of 64, so that rows straddle
+//     128-byte lines (seen from the third wave on: 16384 x 4096 x 1000 512/1 107 us, 256/1 122), every operand comes from HBM once at 6.5 TB/s, a tenth less when only a
 //     few SMs ask for it;
 //     up to 256 tokens, where weights come from HBM and go to every token tile, a fifth of the L2 time adds to that of HBM
-//     (60 shapes: the choice is 1.4 % off the best on average, 2.3 % without; 40 x 4096 x 4096 64/2 10.5 us, not 32/2 12.1);
-//   * a launch costs 3 us, emptying the accumulator 6 ns per token, exchanging partial sums 1.5 us and 8 ns per token; a
-//     further wave of clusters that share tiles starts from nothing, 3 us;
+//     (40 x 4096 x 4096 64/2 10.5 us, not 32/2 12.1);
+//   * a launch costs 3 us, emptying the last accumulator 6 ns per token, exchanging partial sums 1.5 us and 8 ns per token.
+//     Tiles are shared along K only where their clusters all fit at once: a further wave starts from nothing;
 //   * a 256 x 512 tile moves a quarter less operand data than two of 256 x 256, and under the power cap that sets the clock:
 //     690 ns a step against 752, but 4 us in which nothing overlaps the emptying of its one accumulator.
 // Examples, us, against the fixed choice before (128 x 256 tiles of one CTA below 256 rows or at ragged ones):
@@ -204,6 +209,7 @@ PairTile PickPairTile(int M, int N, int K, const int (&cap)[3])
     PairTile best{32, 1};
     double bestNs = 0;
     const double kBlocks = (K + hcgemm::kBlockK - 1) / hcgemm::kBlockK, tilesW = (N + hcgemm::kPairM - 1) / hcgemm::kPairM;
+    const double straddle = K % hcgemm::kBlockK ? 1.5 : 1;
     const double hbmNs = 2.0 * ((double)M * K + (double)N * K + (double)M * N) / 6500.0;
     for (int si = 0; si < 3; ++si) {
         const int split = 1 << si;
@@ -212,16 +218,19 @@ PairTile PickPairTile(int M, int N, int K, const int (&cap)[3])
             if (bn - 32 >= M) continue;                             // a narrower tile holds every token
             const double tiles = tilesW * ((M + bn - 1) / bn), x = std::min(bn, M);
             const double waves = std::ceil(tiles / cap[si]), active = std::min(tiles, (double)cap[si]) * split / cap[0];
+            if (split > 1 && waves > 1) continue;
             const double step = std::max(48 + 1.28 * bn, (16384 + 64 * x) / 120);
-            const double l2Ns = tiles * kBlocks * (32768 + 128 * x) / 13500;
-            const double loop = std::max(waves * std::ceil(kBlocks / split) * step, l2Ns);
-            const double ns = std::max(loop, hbmNs / (0.9 + 0.1 * std::min(1.0, active))) + (M <= 256 ? 0.2 * l2Ns : 0) + 3000 + 6 * x + (split > 1 ? 1500 + 8 * x + (waves - 1) * 3000 : 0);
+            const double multiply = std::ceil(kBlocks / split) * step, empty = 1000 + 500 * std::ceil(x / 64);
+            const double l2Ns = tiles * kBlocks * (32768 + 128 * x) / 13500 * (M > 256 && waves > 2 ? straddle : 1);
+            const double loop = std::max(waves > 1 ? waves * std::max(multiply, std::sqrt(0.94 * multiply * multiply + empty * empty)) : multiply, l2Ns);
+            const double ns = std::max(loop, hbmNs / (0.9 + 0.1 * std::min(1.0, active))) + (M <= 256 ? 0.2 * l2Ns : 0) + 3000 + 6 * x + (split > 1 ? 1500 + 8 * x : 0);
             if (bestNs == 0 || ns < bestNs) { bestNs = ns; best = {bn, split}; }
         }
     }
     if (cap[0] > 0 && M > 256) {
         const double tiles = (double)((M + hcgemm::kPairM - 1) / hcgemm::kPairM) * ((N + hcgemm::kWideN - 1) / hcgemm::kWideN);
-        if (std::max(std::ceil(tiles / cap[0]) * (kBlocks * 690 + 4000), hbmNs) + 3000 < bestNs) best = {hcgemm::kWideN, 1};
+        const double waves = std::ceil(tiles / cap[0]), l2Ns = tiles * kBlocks * 98304 / 13500 * (waves > 2 ? straddle : 0);
+        if (std::max({waves * (kBlocks * 690 + 4000), l2Ns, hbmNs}) + 3000 < bestNs) best = {hcgemm::kWideN, 1};
     }
     return best;
 }

@@ -42,6 +42,19 @@ def test_known_choices():
     assert pick(8192, 3584, 8192, caps) == (224, 1)     # seven full waves instead of eight of 256 columns
 
 
+def test_shallow_k_takes_wide_tiles():
+    caps = (74, 33, 15)
+    # emptying the accumulators bounds these: measured 119 us (310 with 64 tokens), 7.6 (21 with 32), 11.8 (36 with 32), 10.1 (15.5)
+    assert pick(65536, 4096, 64, caps) == (512, 1)
+    assert pick(8192, 1024, 64, caps) == (512, 1)
+    assert pick(1000, 14336, 64, caps) == (512, 1)
+    assert pick(16384, 512, 136, caps)[0] >= 160
+    # operands whose rows straddle lines, many waves: 107 us (122 with 256)
+    assert pick(16384, 4096, 1000, caps) == (512, 1)
+    # 48 clusters of four would come in two waves: 95.7 us with 128/1, 112 with 192/2
+    assert pick(1101, 4096, 14336, caps)[1] == 1
+
+
 @pytest.mark.parametrize("group", [0, 1, 3, 1000, 1 << 28, 1 << 30, 2147483647])
 @pytest.mark.parametrize("m,n,width", [(1000, 5000, 256), (33, 128256, 64), (700, 256, 32), (8192, 8, 224)])
 def test_every_tile_is_walked_once_whatever_group_is_asked_for(m, n, width, group):
