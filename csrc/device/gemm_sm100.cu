@@ -203,13 +203,22 @@ namespace {
 // 16 x 8192 x 28672 32/2 71 (165), 96 x 3584 x 8192 96/4 15 (51), 777 x 4096 x 14336 224/1 82 (97), 33 x 128256 x 4096
 // 64/1 165 (185), 5003 x 8192 x 3584 224/1 210 (235).  Half a second into a run at the power cap 8192 x 28672 x 8192 takes
 // 2929 with 256 x 512 and 3149 with 256 x 256 tiles (from a cool start 2988 and 2783), 8192 x 3584 x 8192 414 and 395.
-struct PairTile { int bn, split; };      // bn = 512: the 256 x 512 kernel
+// Results of at most 128 columns fill less than half of a tile's 256 weights, and all clusters read the same few lines of B at
+// the same time, which costs each step some ns for every cluster beyond 30.  The kernel without pairs (128 x 128 tiles, one
+// per SM) is the better one there from 2048 rows and up to a K of 1024, beyond 148 tiles up to 512: 16384 x 8 x 256 5.1 us (6.9
+// with the best exchanged tile), 8192 x 64 x 512 5.2 (6.1), 5956 x 24 x 936 7.8 (8.2); but 2048 x 64 x 1000 8.8 (6.4) where
+// few clusters do, 65536 x 8 x 1000 49 (38).  Below 2048 rows the exchanged tiles are ahead by a tenth and more.
+struct PairTile {
+    int bn, split;              // bn = 512: the 256 x 512 kernel
+    bool single;                // the kernel without pairs, bn columns
+};
 PairTile PickPairTile(int M, int N, int K, const int (&cap)[3])
 {
-    PairTile best{32, 1};
+    PairTile best{32, 1, false};
     double bestNs = 0;
     const double kBlocks = (K + hcgemm::kBlockK - 1) / hcgemm::kBlockK, tilesW = (N + hcgemm::kPairM - 1) / hcgemm::kPairM;
     const double straddle = K % hcgemm::kBlockK ? 1.5 : 1;
+    const bool few = N <= 128 && (N < 64 || K % hcgemm::kBlockK);       // from 64 columns on, lines of B that do not straddle suffice
     const double hbmNs = 2.0 * ((double)M * K + (double)N * K + (double)M * N) / 6500.0;
     for (int si = 0; si < 3; ++si) {
         const int split = 1 << si;
@@ -219,18 +228,24 @@ PairTile PickPairTile(int M, int N, int K, const int (&cap)[3])
             const double tiles = tilesW * ((M + bn - 1) / bn), x = std::min(bn, M);
             const double waves = std::ceil(tiles / cap[si]), active = std::min(tiles, (double)cap[si]) * split / cap[0];
             if (split > 1 && waves > 1) continue;
-            const double step = std::max(48 + 1.28 * bn, (16384 + 64 * x) / 120);
+            const double crowd = few ? (K <= 1024 ? 4 : 2) * std::max(0.0, std::min(tiles, (double)cap[si]) - 30) : 0;
+            const double step = std::max(48 + 1.28 * bn, (16384 + 64 * x) / 120) + crowd;
             const double multiply = std::ceil(kBlocks / split) * step, empty = 1000 + 500 * std::ceil(x / 64);
             const double l2Ns = tiles * kBlocks * (32768 + 128 * x) / 13500 * (M > 256 && waves > 2 ? straddle : 1);
             const double loop = std::max(waves > 1 ? waves * std::max(multiply, std::sqrt(0.94 * multiply * multiply + empty * empty)) : multiply, l2Ns);
             const double ns = std::max(loop, hbmNs / (0.9 + 0.1 * std::min(1.0, active))) + (M <= 256 ? 0.2 * l2Ns : 0) + 3000 + 6 * x + (split > 1 ? 1500 + 8 * x : 0);
-            if (bestNs == 0 || ns < bestNs) { bestNs = ns; best = {bn, split}; }
+            if (bestNs == 0 || ns < bestNs) { bestNs = ns; best = {bn, split, false}; }
         }
     }
     if (cap[0] > 0 && M > 256) {
         const double tiles = (double)((M + hcgemm::kPairM - 1) / hcgemm::kPairM) * ((N + hcgemm::kWideN - 1) / hcgemm::kWideN);
         const double waves = std::ceil(tiles / cap[0]), l2Ns = tiles * kBlocks * 98304 / 13500 * (waves > 2 ? straddle : 0);
-        if (std::max({waves * (kBlocks * 690 + 4000), l2Ns, hbmNs}) + 3000 < bestNs) best = {hcgemm::kWideN, 1};
+        if (std::max({waves * (kBlocks * 690 + 4000), l2Ns, hbmNs}) + 3000 < bestNs) best = {hcgemm::kWideN, 1, false};
+    }
+    const double rows = (M + hcgemm::kBlockM - 1) / hcgemm::kBlockM, sms = 2.0 * cap[0];
+    if (N <= 128 && M >= 2048 && K <= (rows <= sms ? 1024 : 512)) {
+        const double tile = std::max(kBlocks * (K % hcgemm::kBlockK ? 240 : 200), 700.0);
+        if (std::max(std::ceil(rows / sms) * tile, hbmNs) + 2900 < bestNs) best = {128, 1, true};
     }
     return best;
 }
@@ -313,8 +328,9 @@ PairTile ChoosePairTile(int M, int N, int K, const int (&cap)[3])
 {
     PairTile t = PickPairTile(M, N, K, cap);
     const int bn = ForcedPairTileWidth(), split = g_forceSplit.load(), kBlocks = (K + hcgemm::kBlockK - 1) / hcgemm::kBlockK;
-    if (bn >= hcgemm::kWideN) t = {hcgemm::kWideN, 1};
-    else if (bn > 0) t.bn = std::min(256, std::max(32, bn / 32 * 32));
+    if (bn >= hcgemm::kWideN) t = {hcgemm::kWideN, 1, false};
+    else if (bn > 0) { t.bn = std::min(256, std::max(32, bn / 32 * 32)); t.single = false; }
+    if (split > 0) t.single = false;
     if (t.bn <= 256 && (split == 1 || split == 2 || split == 4) && split <= kBlocks && cap[split / 2] > 0) t.split = split;
     return t;
 }
@@ -332,10 +348,11 @@ HcclResult GemmBf16(const void *A, const void *B, void *C, int M, int N, int K, 
     const GemmLimits limits = Limits();
     if (pairEnabled && limits.cap[0] > 0) {
         const PairTile tile = ChoosePairTile(M, N, K, limits.cap);
-        return tile.bn == hcgemm::kWideN ? LaunchWideGemm(A, B, C, M, N, K, lda, ldb, ldc, stream)
-                                         : LaunchSwapGemm(A, B, C, M, N, K, lda, ldb, ldc, tile, stream);
+        if (!tile.single)
+            return tile.bn == hcgemm::kWideN ? LaunchWideGemm(A, B, C, M, N, K, lda, ldb, ldc, stream)
+                                             : LaunchSwapGemm(A, B, C, M, N, K, lda, ldb, ldc, tile, stream);
     }
-    // without CTA pairs (HCOMM_GEMM_PAIR=0, or a device that cannot hold a cluster): one CTA per 128-row tile
+    // one CTA per 128-row tile: few columns, HCOMM_GEMM_PAIR=0, or a device that cannot hold a cluster
     const int BN = (N % 256 == 0 || N >= 2048) ? 256 : 128;
     CUtensorMap tmA, tmB;
     CHK_RET(MakeTensorMap2dBf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, hcgemm::kBlockM, hcgemm::kBlockK));
@@ -388,6 +405,13 @@ extern "C" void HcommToolGemmTile(int M, int N, int K, int cap1, int cap2, int c
     const hc::PairTile t = hc::PickPairTile(M, N, K, cap);
     if (tileWidth) *tileWidth = t.bn;
     if (pairsAlongK) *pairsAlongK = t.split;
+}
+// Which kernel that rule takes: 0 exchanged operands, 1 tiles of 256 x 512, 2 without pairs.
+extern "C" int HcommToolGemmKernel(int M, int N, int K, int cap1, int cap2, int cap4)
+{
+    const int cap[3] = {cap1, cap2, cap4};
+    const hc::PairTile t = hc::PickPairTile(M, N, K, cap);
+    return t.single ? 2 : t.bn == hcgemm::kWideN ? 1 : 0;
 }
 // The blocks (256 weights, tileWidth tokens) of tile t of the GEMM with exchanged operands; returns the number of tiles.
 extern "C" int HcommToolGemmOrder(int M, int N, int K, int tileWidth, int t, int *weightBlock, int *tokenBlock)

@@ -55,6 +55,16 @@ def test_shallow_k_takes_wide_tiles():
     assert pick(1101, 4096, 14336, caps)[1] == 1
 
 
+def test_few_columns_of_many_rows_run_without_pairs():
+    caps = (74, 33, 15)
+    kernel = _lib.load().HcommToolGemmKernel
+    assert kernel(16384, 8, 256, *caps) == 2 and kernel(8192, 64, 512, *caps) == 2 and kernel(65536, 8, 64, *caps) == 2
+    assert kernel(5956, 24, 936, *caps) == 2
+    # too few rows, too deep a K, too many columns
+    assert kernel(1000, 8, 256, *caps) == 0 and kernel(16384, 8, 4096, *caps) == 0 and kernel(65536, 8, 1000, *caps) == 0
+    assert kernel(16384, 136, 256, *caps) != 2 and kernel(8192, 28672, 8192, *caps) == 1
+
+
 @pytest.mark.parametrize("group", [0, 1, 3, 1000, 1 << 28, 1 << 30, 2147483647])
 @pytest.mark.parametrize("m,n,width", [(1000, 5000, 256), (33, 128256, 64), (700, 256, 32), (8192, 8, 224)])
 def test_every_tile_is_walked_once_whatever_group_is_asked_for(m, n, width, group):

@@ -128,3 +128,22 @@ def test_oversized_raster_group(width):
     finally:
         lib.HcommGemmSetTuning(0, 0)
     assert take_kernel_error() == 0 and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("m,n,k", [(4097, 8, 64), (12800, 128, 8), (5003, 72, 136), (8192, 24, 1000), (19000, 8, 72), (40001, 64, 512)])
+def test_few_columns_of_many_rows(m, n, k):
+    # the kernel without pairs is the one that runs here; rows of a longer pitch in, a result inside a wider matrix
+    from hcomm_b200 import _lib
+    from hcomm_b200.ops.gemm import gemm_bf16, take_kernel_error
+    assert _lib.load().HcommToolGemmKernel(m, n, k, 74, 33, 15) == 2
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a = torch.randn(m, k + 8, device="cuda", generator=g).to(torch.bfloat16)[:, :k]
+    b = (torch.randn(n, k, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    full = torch.full((m, n + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm_bf16(a, b, full[:, :n])
+    torch.cuda.synchronize()
+    assert take_kernel_error() == 0 and bool((full[:, n:] == 7.0).all())
+    ref = a.double() @ b.double().t()
+    # one rounding to bf16 (half a step, 2^-9) and fp32 sums of k products (k * 2^-24 of the sum of magnitudes)
+    bound = 2.0 ** -8 * ref.abs() + k * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t())
+    assert bool(((full[:, :n].double() - ref).abs() <= bound).all())
