@@ -11,6 +11,7 @@
 #include "../core/per_device.h"
 #include "gemm_api.h"
 #include "gemm_sm100.cuh"
+#include "gemm_sm100_2sm.cuh"
 #include "gemm_sm100_2sm_wide.cuh"
 #include "gemm_sm100_swap.cuh"
 
@@ -33,6 +34,13 @@ __global__ void __launch_bounds__(hcgemm::kWideThreads, 1)
 GemmBf16PairWideKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC, hcgemm::GemmShape shape, int gm)
 {
     hcgemm::GemmMainLoopPairWide<4>(&tmA, &tmB, &tmC, shape, hcgemm::GroupedOrder{shape.tilesM < gm ? shape.tilesM : gm});
+}
+
+// 256 x 224 tiles with the tokens as rows (see gemm_sm100_2sm.cuh).
+__global__ void __launch_bounds__(hcgemm::kThreads, 1)
+GemmBf16Pair224Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, hcgemm::GemmShape shape, hcgemm::StoreBf16 epi, int gm)
+{
+    hcgemm::GemmMainLoopPair<224, 7>(&tmA, &tmB, shape, hcgemm::GroupedOrder{shape.tilesM < gm ? shape.tilesM : gm}, epi);
 }
 
 // 256 weights x bn tokens, SPLIT pairs of a cluster along K (see gemm_sm100_swap.cuh).
@@ -78,7 +86,7 @@ GemmLimits Limits()
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return {}; }
     return limits.Get(dev, [](GemmLimits *l) {
-        const bool wide = AllowShared(GemmBf16PairWideKernel, hcgemm::ConfigWide<4>::kSmemBytes);
+        const bool wide = AllowShared(GemmBf16PairWideKernel, hcgemm::ConfigWide<4>::kSmemBytes) && AllowShared(GemmBf16Pair224Kernel, hcgemm::Config2<224, 7>::kSmemBytes);
         const bool one = ClustersAtOnce<1>(&l->cap[0]), two = ClustersAtOnce<2>(&l->cap[1]), four = ClustersAtOnce<4>(&l->cap[2]);
         if (!wide) l->cap[0] = 0;
         l->single = AllowShared(GemmBf16Kernel<256>, hcgemm::Config<256>::kSmemBytes) && AllowShared(GemmBf16Kernel<128>, hcgemm::Config<128>::kSmemBytes);
@@ -208,13 +216,19 @@ namespace {
 // per SM) is the better one there from 2048 rows and up to a K of 1024, beyond 148 tiles up to 512: 16384 x 8 x 256 5.1 us (6.9
 // with the best exchanged tile), 8192 x 64 x 512 5.2 (6.1), 5956 x 24 x 936 7.8 (8.2); but 2048 x 64 x 1000 8.8 (6.4) where
 // few clusters do, 65536 x 8 x 1000 49 (38).  Below 2048 rows the exchanged tiles are ahead by a tenth and more.
+// Layers are often a multiple of 224 wide (3584, 7168, 14336, 28672) and batches a multiple of 256 tokens.  Tiles of 256 tokens x
+// 224 weights, the roles not exchanged, then come out whole where 256 weights x any number of tokens leaves part of a wave
+// empty: 512 x 14336 x 8192 91 us (101 with 512/1), 256 x 14336 x 8192 52.8 (56), half a second into a run at the power cap
+// 2048 x 14336 x 8192 373 (390).  With a shallower K its result, stored by the lanes at a row stride, holds it up: 4096 x
+// 14336 x 1000 146 (111 with 256/1); the line is a K of 4096.
+enum class GemmKernel { EXCHANGED = 0, WIDE = 1, SINGLE = 2, ROWS224 = 3 };     // SINGLE: without pairs
 struct PairTile {
-    int bn, split;              // bn = 512: the 256 x 512 kernel
-    bool single;                // the kernel without pairs, bn columns
+    int bn, split;              // WIDE: bn = 512
+    GemmKernel kernel;
 };
 PairTile PickPairTile(int M, int N, int K, const int (&cap)[3])
 {
-    PairTile best{32, 1, false};
+    PairTile best{32, 1, GemmKernel::EXCHANGED};
     double bestNs = 0;
     const double kBlocks = (K + hcgemm::kBlockK - 1) / hcgemm::kBlockK, tilesW = (N + hcgemm::kPairM - 1) / hcgemm::kPairM;
     const double straddle = K % hcgemm::kBlockK ? 1.5 : 1;
@@ -234,18 +248,26 @@ PairTile PickPairTile(int M, int N, int K, const int (&cap)[3])
             const double l2Ns = tiles * kBlocks * (32768 + 128 * x) / 13500 * (M > 256 && waves > 2 ? straddle : 1);
             const double loop = std::max(waves > 1 ? waves * std::max(multiply, std::sqrt(0.94 * multiply * multiply + empty * empty)) : multiply, l2Ns);
             const double ns = std::max(loop, hbmNs / (0.9 + 0.1 * std::min(1.0, active))) + (M <= 256 ? 0.2 * l2Ns : 0) + 3000 + 6 * x + (split > 1 ? 1500 + 8 * x : 0);
-            if (bestNs == 0 || ns < bestNs) { bestNs = ns; best = {bn, split, false}; }
+            if (bestNs == 0 || ns < bestNs) { bestNs = ns; best = {bn, split, GemmKernel::EXCHANGED}; }
         }
     }
     if (cap[0] > 0 && M > 256) {
         const double tiles = (double)((M + hcgemm::kPairM - 1) / hcgemm::kPairM) * ((N + hcgemm::kWideN - 1) / hcgemm::kWideN);
         const double waves = std::ceil(tiles / cap[0]), l2Ns = tiles * kBlocks * 98304 / 13500 * (waves > 2 ? straddle : 0);
-        if (std::max({waves * (kBlocks * 690 + 4000), l2Ns, hbmNs}) + 3000 < bestNs) best = {hcgemm::kWideN, 1, false};
+        const double ns = std::max({waves * (kBlocks * 690 + 4000), l2Ns, hbmNs}) + 3000;
+        if (ns < bestNs) { bestNs = ns; best = {hcgemm::kWideN, 1, GemmKernel::WIDE}; }
+    }
+    if (cap[0] > 0 && M % hcgemm::kPairM == 0 && N % 224 == 0 && N % 128 == 0 && K >= 4096) {
+        const double tiles = (double)(M / hcgemm::kPairM) * (N / 224), waves = std::ceil(tiles / cap[0]);
+        const double multiply = kBlocks * (48 + 1.28 * 224), l2Ns = tiles * kBlocks * (32768 + 128 * 224) / 13500;
+        // by three hundredths, less is chance
+        if ((std::max({waves * std::max(multiply, std::sqrt(0.94 * multiply * multiply + 3000.0 * 3000.0)), l2Ns, hbmNs}) + 3000 + 6 * 224) / 0.97 < bestNs)
+            best = {224, 1, GemmKernel::ROWS224};
     }
     const double rows = (M + hcgemm::kBlockM - 1) / hcgemm::kBlockM, sms = 2.0 * cap[0];
     if (N <= 128 && M >= 2048 && K <= (rows <= sms ? 1024 : 512)) {
         const double tile = std::max(kBlocks * (K % hcgemm::kBlockK ? 240 : 200), 700.0);
-        if (std::max(std::ceil(rows / sms) * tile, hbmNs) + 2900 < bestNs) best = {128, 1, true};
+        if (std::max(std::ceil(rows / sms) * tile, hbmNs) + 2900 < bestNs) best = {128, 1, GemmKernel::SINGLE};
     }
     return best;
 }
@@ -324,13 +346,33 @@ HcclResult LaunchWideGemm(const void *A, const void *B, void *C, int M, int N, i
     return HCCL_SUCCESS;
 }
 
+HcclResult LaunchPair224Gemm(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, void *stream)
+{
+    CUtensorMap tmA, tmB;
+    CHK_RET(MakeTensorMap2dBf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, hcgemm::kBlockM, hcgemm::kBlockK));
+    CHK_RET(MakeTensorMap2dBf16(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 224u / 2, hcgemm::kBlockK));
+    hcgemm::GemmShape shape;
+    shape.M = M; shape.N = N; shape.K = K;
+    shape.tilesM = M / hcgemm::kPairM;
+    shape.tilesN = N / 224;
+    shape.errFlag = GemmErrorFlag();
+    shape.phase = nullptr;
+    const hcgemm::StoreBf16 epi{(__nv_bfloat16 *)C, ldc, M, N};
+    cudaLaunchAttribute at[2];
+    cudaLaunchConfig_t cfg = PairConfig(at, std::min(Limits().cap[0], shape.tilesM * shape.tilesN), 2, hcgemm::kThreads, hcgemm::Config2<224, 7>::kSmemBytes, stream);
+    cfg.numAttrs = 1;           // the loop is the fused kernels', which do not wait for a kernel in front: an ordinary launch
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, GemmBf16Pair224Kernel, tmA, tmB, shape, epi, PairGroupRows(K));
+    if (e != cudaSuccess) { HCCL_ERROR("GemmBf16 (256 x 224 tiles) launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
+    return HCCL_SUCCESS;
+}
+
 PairTile ChoosePairTile(int M, int N, int K, const int (&cap)[3])
 {
     PairTile t = PickPairTile(M, N, K, cap);
     const int bn = ForcedPairTileWidth(), split = g_forceSplit.load(), kBlocks = (K + hcgemm::kBlockK - 1) / hcgemm::kBlockK;
-    if (bn >= hcgemm::kWideN) t = {hcgemm::kWideN, 1, false};
-    else if (bn > 0) { t.bn = std::min(256, std::max(32, bn / 32 * 32)); t.single = false; }
-    if (split > 0) t.single = false;
+    if (bn >= hcgemm::kWideN) t = {hcgemm::kWideN, 1, GemmKernel::WIDE};
+    else if (bn > 0) t = {std::min(256, std::max(32, bn / 32 * 32)), t.split, GemmKernel::EXCHANGED};
+    else if (split > 0 && t.kernel != GemmKernel::WIDE) t.kernel = GemmKernel::EXCHANGED;
     if (t.bn <= 256 && (split == 1 || split == 2 || split == 4) && split <= kBlocks && cap[split / 2] > 0) t.split = split;
     return t;
 }
@@ -348,9 +390,9 @@ HcclResult GemmBf16(const void *A, const void *B, void *C, int M, int N, int K, 
     const GemmLimits limits = Limits();
     if (pairEnabled && limits.cap[0] > 0) {
         const PairTile tile = ChoosePairTile(M, N, K, limits.cap);
-        if (!tile.single)
-            return tile.bn == hcgemm::kWideN ? LaunchWideGemm(A, B, C, M, N, K, lda, ldb, ldc, stream)
-                                             : LaunchSwapGemm(A, B, C, M, N, K, lda, ldb, ldc, tile, stream);
+        if (tile.kernel == GemmKernel::WIDE) return LaunchWideGemm(A, B, C, M, N, K, lda, ldb, ldc, stream);
+        if (tile.kernel == GemmKernel::ROWS224) return LaunchPair224Gemm(A, B, C, M, N, K, lda, ldb, ldc, stream);
+        if (tile.kernel == GemmKernel::EXCHANGED) return LaunchSwapGemm(A, B, C, M, N, K, lda, ldb, ldc, tile, stream);
     }
     // one CTA per 128-row tile: few columns, HCOMM_GEMM_PAIR=0, or a device that cannot hold a cluster
     const int BN = (N % 256 == 0 || N >= 2048) ? 256 : 128;
@@ -406,12 +448,11 @@ extern "C" void HcommToolGemmTile(int M, int N, int K, int cap1, int cap2, int c
     if (tileWidth) *tileWidth = t.bn;
     if (pairsAlongK) *pairsAlongK = t.split;
 }
-// Which kernel that rule takes: 0 exchanged operands, 1 tiles of 256 x 512, 2 without pairs.
+// Which kernel that rule takes: 0 exchanged operands, 1 tiles of 256 x 512, 2 without pairs, 3 tiles of 256 tokens x 224 weights.
 extern "C" int HcommToolGemmKernel(int M, int N, int K, int cap1, int cap2, int cap4)
 {
     const int cap[3] = {cap1, cap2, cap4};
-    const hc::PairTile t = hc::PickPairTile(M, N, K, cap);
-    return t.single ? 2 : t.bn == hcgemm::kWideN ? 1 : 0;
+    return (int)hc::PickPairTile(M, N, K, cap).kernel;
 }
 // The blocks (256 weights, tileWidth tokens) of tile t of the GEMM with exchanged operands; returns the number of tiles.
 extern "C" int HcommToolGemmOrder(int M, int N, int K, int tileWidth, int t, int *weightBlock, int *tokenBlock)

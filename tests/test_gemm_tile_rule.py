@@ -65,6 +65,15 @@ def test_few_columns_of_many_rows_run_without_pairs():
     assert kernel(16384, 136, 256, *caps) != 2 and kernel(8192, 28672, 8192, *caps) == 1
 
 
+def test_round_batches_of_layers_224_wide():
+    caps = (74, 33, 15)
+    kernel = _lib.load().HcommToolGemmKernel
+    assert kernel(512, 14336, 8192, *caps) == 3 and kernel(2048, 14336, 8192, *caps) == 3 and kernel(512, 7168, 8192, *caps) == 3
+    # not a multiple of 256 tokens or of 224 weights, a shallower K, whole waves anyway
+    assert kernel(511, 14336, 8192, *caps) != 3 and kernel(512, 8192, 8192, *caps) != 3 and kernel(4096, 14336, 1024, *caps) != 3
+    assert kernel(8192, 28672, 8192, *caps) == 1
+
+
 @pytest.mark.parametrize("group", [0, 1, 3, 1000, 1 << 28, 1 << 30, 2147483647])
 @pytest.mark.parametrize("m,n,width", [(1000, 5000, 256), (33, 128256, 64), (700, 256, 32), (8192, 8, 224)])
 def test_every_tile_is_walked_once_whatever_group_is_asked_for(m, n, width, group):

@@ -147,3 +147,23 @@ def test_few_columns_of_many_rows(m, n, k):
     # one rounding to bf16 (half a step, 2^-9) and fp32 sums of k products (k * 2^-24 of the sum of magnitudes)
     bound = 2.0 ** -8 * ref.abs() + k * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t())
     assert bool(((full[:, :n].double() - ref).abs() <= bound).all())
+
+
+def test_round_batch_of_a_layer_224_wide():
+    # 256 x 224 tiles with the tokens as rows, operands and result of a longer pitch
+    from hcomm_b200 import _lib
+    from hcomm_b200.ops.gemm import gemm_bf16, take_kernel_error
+    m, n, k = 512, 14336, 4104
+    assert _lib.load().HcommToolGemmKernel(m, n, k, 74, 33, 15) == 3
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a = torch.randn(m, k + 8, device="cuda", generator=g).to(torch.bfloat16)[:, :k]
+    b = (torch.randn(n, k + 16, device="cuda", generator=g) * 0.05).to(torch.bfloat16)[:, :k]
+    full = torch.full((m, n + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    for _ in range(2):          # the second call behind the first
+        gemm_bf16(a, b, full[:, :n])
+    torch.cuda.synchronize()
+    assert take_kernel_error() == 0 and bool((full[:, n:] == 7.0).all())
+    ref = a.double() @ b.double().t()
+    # one rounding to bf16 (half a step, 2^-9) and fp32 sums of k products (k * 2^-24 of the sum of magnitudes)
+    bound = 2.0 ** -8 * ref.abs() + k * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t())
+    assert bool(((full[:, :n].double() - ref).abs() <= bound).all())
