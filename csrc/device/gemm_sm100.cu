@@ -5,7 +5,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <map>
 #include <mutex>
+#include <vector>
 
 #include "../core/log.h"
 #include "../core/per_device.h"
@@ -225,11 +227,11 @@ enum class GemmKernel { EXCHANGED = 0, WIDE = 1, SINGLE = 2, ROWS224 = 3 };     
 struct PairTile {
     int bn, split;              // WIDE: bn = 512
     GemmKernel kernel;
+    int group = 0;              // rasterisation group, 0 = by rule
 };
-PairTile PickPairTile(int M, int N, int K, const int (&cap)[3])
+// Calls f(tile, estimate in ns) for every tile that can take the shape.
+template <typename F> void EachTile(int M, int N, int K, const int (&cap)[3], bool wide, F f)
 {
-    PairTile best{32, 1, GemmKernel::EXCHANGED};
-    double bestNs = 0;
     const double kBlocks = (K + hcgemm::kBlockK - 1) / hcgemm::kBlockK, tilesW = (N + hcgemm::kPairM - 1) / hcgemm::kPairM;
     const double straddle = K % hcgemm::kBlockK ? 1.5 : 1;
     const bool few = N <= 128 && (N < 64 || K % hcgemm::kBlockK);       // from 64 columns on, lines of B that do not straddle suffice
@@ -247,28 +249,43 @@ PairTile PickPairTile(int M, int N, int K, const int (&cap)[3])
             const double multiply = std::ceil(kBlocks / split) * step, empty = 1000 + 500 * std::ceil(x / 64);
             const double l2Ns = tiles * kBlocks * (32768 + 128 * x) / 13500 * (M > 256 && waves > 2 ? straddle : 1);
             const double loop = std::max(waves > 1 ? waves * std::max(multiply, std::sqrt(0.94 * multiply * multiply + empty * empty)) : multiply, l2Ns);
-            const double ns = std::max(loop, hbmNs / (0.9 + 0.1 * std::min(1.0, active))) + (M <= 256 ? 0.2 * l2Ns : 0) + 3000 + 6 * x + (split > 1 ? 1500 + 8 * x : 0);
-            if (bestNs == 0 || ns < bestNs) { bestNs = ns; best = {bn, split, GemmKernel::EXCHANGED}; }
+            f(PairTile{bn, split, GemmKernel::EXCHANGED},
+              std::max(loop, hbmNs / (0.9 + 0.1 * std::min(1.0, active))) + (M <= 256 ? 0.2 * l2Ns : 0) + 3000 + 6 * x + (split > 1 ? 1500 + 8 * x : 0));
         }
     }
-    if (cap[0] > 0 && M > 256) {
+    if (cap[0] <= 0) return;
+    if (wide && M > 256) {
         const double tiles = (double)((M + hcgemm::kPairM - 1) / hcgemm::kPairM) * ((N + hcgemm::kWideN - 1) / hcgemm::kWideN);
-        const double waves = std::ceil(tiles / cap[0]), l2Ns = tiles * kBlocks * 98304 / 13500 * (waves > 2 ? straddle : 0);
-        const double ns = std::max({waves * (kBlocks * 690 + 4000), l2Ns, hbmNs}) + 3000;
-        if (ns < bestNs) { bestNs = ns; best = {hcgemm::kWideN, 1, GemmKernel::WIDE}; }
+        const double waves = std::ceil(tiles / cap[0]), l2Ns = tiles * kBlocks * 98304 / 13500 * (waves > 2 ? straddle : 1);
+        f(PairTile{hcgemm::kWideN, 1, GemmKernel::WIDE}, std::max({waves * (kBlocks * 690 + 4000), l2Ns, hbmNs}) + 3000);
     }
-    if (cap[0] > 0 && M % hcgemm::kPairM == 0 && N % 224 == 0 && N % 128 == 0 && K >= 4096) {
+    if (M % hcgemm::kPairM == 0 && N % 224 == 0 && N % 128 == 0 && K >= 4096) {
         const double tiles = (double)(M / hcgemm::kPairM) * (N / 224), waves = std::ceil(tiles / cap[0]);
         const double multiply = kBlocks * (48 + 1.28 * 224), l2Ns = tiles * kBlocks * (32768 + 128 * 224) / 13500;
-        // by three hundredths, less is chance
-        if ((std::max({waves * std::max(multiply, std::sqrt(0.94 * multiply * multiply + 3000.0 * 3000.0)), l2Ns, hbmNs}) + 3000 + 6 * 224) / 0.97 < bestNs)
-            best = {224, 1, GemmKernel::ROWS224};
+        // ahead by three hundredths, less is chance
+        f(PairTile{224, 1, GemmKernel::ROWS224},
+          (std::max({waves * std::max(multiply, std::sqrt(0.94 * multiply * multiply + 3000.0 * 3000.0)), l2Ns, hbmNs}) + 3000 + 6 * 224) / 0.97);
     }
     const double rows = (M + hcgemm::kBlockM - 1) / hcgemm::kBlockM, sms = 2.0 * cap[0];
     if (N <= 128 && M >= 2048 && K <= (rows <= sms ? 1024 : 512)) {
         const double tile = std::max(kBlocks * (K % hcgemm::kBlockK ? 240 : 200), 700.0);
-        if (std::max(std::ceil(rows / sms) * tile, hbmNs) + 2900 < bestNs) best = {128, 1, GemmKernel::SINGLE};
+        f(PairTile{128, 1, GemmKernel::SINGLE}, std::max(std::ceil(rows / sms) * tile, hbmNs) + 2900);
     }
+}
+// HCOMM_GEMM_WIDE=0 keeps the tiles at 256 columns or fewer.
+bool WideTiles()
+{
+    static const bool on = [] { const char *e = getenv("HCOMM_GEMM_WIDE"); return !(e && e[0] == '0'); }();
+    return on;
+}
+PairTile PickPairTile(int M, int N, int K, const int (&cap)[3], double *estimate = nullptr)
+{
+    PairTile best{32, 1, GemmKernel::EXCHANGED};
+    double bestNs = 0;
+    EachTile(M, N, K, cap, WideTiles(), [&](const PairTile &t, double ns) {
+        if (bestNs == 0 || ns < bestNs) { bestNs = ns; best = t; }
+    });
+    if (estimate) *estimate = bestNs;
     return best;
 }
 
@@ -289,14 +306,14 @@ cudaLaunchConfig_t PairConfig(cudaLaunchAttribute *at, int clusters, int cluster
     return cfg;
 }
 
-hcgemm::SwapShape ShapeOf(int M, int N, int K, int bn)
+hcgemm::SwapShape ShapeOf(int M, int N, int K, int bn, int group = 0)
 {
     hcgemm::SwapShape g = {};
     g.M = M; g.N = N; g.K = K;
     g.tilesW = (N + hcgemm::kPairM - 1) / hcgemm::kPairM;
     g.tilesT = (M + bn - 1) / bn;
     g.bn = bn; g.stages = hcgemm::SwapStages(bn);
-    g.group = std::min(PairGroupRows(K), g.tilesW);     // a group that the caller forces may be any number
+    g.group = std::min(group > 0 ? group : PairGroupRows(K), g.tilesW);     // a group that the caller forces may be any number
     return g;
 }
 
@@ -305,7 +322,7 @@ HcclResult LaunchSwapGemm(const void *A, const void *B, void *C, int M, int N, i
     CUtensorMap tmW, tmX;
     CHK_RET(MakeTensorMap2dBf16(&tmW, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, hcgemm::kBlockM, hcgemm::kBlockK));
     CHK_RET(MakeTensorMap2dBf16(&tmX, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)(tile.bn / 2), hcgemm::kBlockK));
-    hcgemm::SwapShape g = ShapeOf(M, N, K, tile.bn);
+    hcgemm::SwapShape g = ShapeOf(M, N, K, tile.bn, tile.group);
     g.C = (__nv_bfloat16 *)C; g.ldc = ldc;
     g.errFlag = GemmErrorFlag();
     const int tiles = g.tilesW * g.tilesT;
@@ -325,7 +342,7 @@ HcclResult LaunchSwapGemm(const void *A, const void *B, void *C, int M, int N, i
     return HCCL_SUCCESS;
 }
 
-HcclResult LaunchWideGemm(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, void *stream)
+HcclResult LaunchWideGemm(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, const PairTile &tile, void *stream)
 {
     CUtensorMap tmA, tmB, tmC;            // result tiles leave through TMA stores: boxes of 32 rows x 64 columns
     CHK_RET(MakeTensorMap2dBf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, hcgemm::kBlockM, hcgemm::kBlockK));
@@ -338,7 +355,7 @@ HcclResult LaunchWideGemm(const void *A, const void *B, void *C, int M, int N, i
     shape.errFlag = GemmErrorFlag();
     shape.phase = nullptr;
     // a wave of 74 such tiles loads the fewest panels at 12 rows x 6 columns
-    const int rows = PairGroupRows(K), group = g_forceGm.load() > 0 || rows >= 16 ? rows : 12;
+    const int rows = PairGroupRows(K), group = tile.group > 0 ? tile.group : g_forceGm.load() > 0 || rows >= 16 ? rows : 12;
     cudaLaunchAttribute at[2];
     const cudaLaunchConfig_t cfg = PairConfig(at, std::min(Limits().cap[0], shape.tilesM * shape.tilesN), 2, hcgemm::kWideThreads, hcgemm::ConfigWide<4>::kSmemBytes, stream);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, GemmBf16PairWideKernel, tmA, tmB, tmC, shape, group);
@@ -346,7 +363,7 @@ HcclResult LaunchWideGemm(const void *A, const void *B, void *C, int M, int N, i
     return HCCL_SUCCESS;
 }
 
-HcclResult LaunchPair224Gemm(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, void *stream)
+HcclResult LaunchPair224Gemm(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, const PairTile &tile, void *stream)
 {
     CUtensorMap tmA, tmB;
     CHK_RET(MakeTensorMap2dBf16(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, hcgemm::kBlockM, hcgemm::kBlockK));
@@ -361,15 +378,96 @@ HcclResult LaunchPair224Gemm(const void *A, const void *B, void *C, int M, int N
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = PairConfig(at, std::min(Limits().cap[0], shape.tilesM * shape.tilesN), 2, hcgemm::kThreads, hcgemm::Config2<224, 7>::kSmemBytes, stream);
     cfg.numAttrs = 1;           // the loop is the fused kernels', which do not wait for a kernel in front: an ordinary launch
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, GemmBf16Pair224Kernel, tmA, tmB, shape, epi, PairGroupRows(K));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, GemmBf16Pair224Kernel, tmA, tmB, shape, epi, tile.group > 0 ? tile.group : PairGroupRows(K));
     if (e != cudaSuccess) { HCCL_ERROR("GemmBf16 (256 x 224 tiles) launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
 
-PairTile ChoosePairTile(int M, int N, int K, const int (&cap)[3])
+// One launch of a tile's kernel on CTA pairs (all but SINGLE).
+HcclResult LaunchTile(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, const PairTile &tile, void *stream)
 {
-    PairTile t = PickPairTile(M, N, K, cap);
+    if (tile.kernel == GemmKernel::WIDE) return LaunchWideGemm(A, B, C, M, N, K, lda, ldb, ldc, tile, stream);
+    if (tile.kernel == GemmKernel::ROWS224) return LaunchPair224Gemm(A, B, C, M, N, K, lda, ldb, ldc, tile, stream);
+    return LaunchSwapGemm(A, B, C, M, N, K, lda, ldb, ldc, tile, stream);
+}
+
+// HCOMM_GEMM_AUTOTUNE=1: a large shape (2 M N K of 2e11 and more) seen for the first time is timed once with the tiles whose
+// estimates come within 15 % of the best, each with the rasterisation group halved, kept and doubled, on the caller's stream,
+// and the fastest is kept for the process.  Never while the stream is being captured, nor with a forced width, group or split.
+// Off by default: at the power cap the variants differ mostly through the clock that they leave the chip at, and timings of a
+// few launches each did not rank them the same from run to run.
+struct ShapeKey {
+    int M, N, K;
+    bool operator<(const ShapeKey &o) const { return M != o.M ? M < o.M : (N != o.N ? N < o.N : K < o.K); }
+};
+std::mutex g_tuneMu;
+std::map<ShapeKey, PairTile> g_tuned;
+
+PairTile MeasuredTile(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, const int (&cap)[3], const PairTile &rule, double estimate,
+                      void *stream)
+{
+    const ShapeKey key{M, N, K};
+    {
+        std::lock_guard<std::mutex> lk(g_tuneMu);
+        auto it = g_tuned.find(key);
+        if (it != g_tuned.end()) return it->second;
+    }
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing((cudaStream_t)stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) { cudaGetLastError(); return rule; }
+    std::vector<PairTile> cands;
+    EachTile(M, N, K, cap, WideTiles(), [&](PairTile t, double ns) {
+        if (ns > 1.15 * estimate || t.kernel == GemmKernel::SINGLE) return;
+        const int group = PairGroupRows(K);
+        for (int g : {group / 2, group, group * 2})
+            if (g >= 2 && g <= 32) { t.group = g; cands.push_back(t); }
+    });
+    if (cands.size() < 2) return rule;
+    // Five rounds over all candidates, two back-to-back launches each; the first round only warms up (module load, L2,
+    // clocks).  Odd rounds walk the list backwards so that a drift over a round does not favour one end of it, and a
+    // candidate's figure is the median of its four counted rounds, not its luckiest one.
+    cudaEvent_t ev[2];
+    if (cudaEventCreate(&ev[0]) != cudaSuccess) { cudaGetLastError(); return rule; }
+    if (cudaEventCreate(&ev[1]) != cudaSuccess) { cudaGetLastError(); cudaEventDestroy(ev[0]); return rule; }
+    const int count = (int)cands.size();
+    std::vector<std::vector<float>> samples(count);
+    bool ok = true;
+    for (int round = 0; round < 5 && ok; ++round) {
+        for (int i = 0; i < count && ok; ++i) {
+            const int c = (round & 1) ? count - 1 - i : i;
+            cudaEventRecord(ev[0], (cudaStream_t)stream);
+            for (int r = 0; r < 2 && ok; ++r) ok = LaunchTile(A, B, C, M, N, K, lda, ldb, ldc, cands[c], stream) == HCCL_SUCCESS;
+            cudaEventRecord(ev[1], (cudaStream_t)stream);
+            float ms = 0;
+            if (!ok || cudaEventSynchronize(ev[1]) != cudaSuccess || cudaEventElapsedTime(&ms, ev[0], ev[1]) != cudaSuccess) { cudaGetLastError(); ok = false; break; }
+            if (round > 0) samples[c].push_back(ms * 0.5f);
+        }
+    }
+    cudaEventDestroy(ev[0]);
+    cudaEventDestroy(ev[1]);
+    if (!ok) return rule;
+    int win = 0;
+    std::vector<float> median(count);
+    for (int i = 0; i < count; ++i) {
+        std::sort(samples[i].begin(), samples[i].end());
+        median[i] = 0.5f * (samples[i][1] + samples[i][2]);
+        if (median[i] < median[win]) win = i;
+    }
+    HCCL_INFO("GEMM %d x %d x %d: tile width %d, %d pairs along K, group %d chosen by measurement (%.3f ms; the estimate said %d / %d)", M, N, K, cands[win].bn,
+              cands[win].split, cands[win].group, median[win], rule.bn, rule.split);
+    std::lock_guard<std::mutex> lk(g_tuneMu);
+    return g_tuned.emplace(key, cands[win]).first->second;
+}
+
+PairTile ChoosePairTile(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, const int (&cap)[3], void *stream)
+{
+    static const bool measure = [] { const char *e = getenv("HCOMM_GEMM_AUTOTUNE"); return e && e[0] == '1'; }();
+    double estimate = 0;
+    PairTile t = PickPairTile(M, N, K, cap, &estimate);
     const int bn = ForcedPairTileWidth(), split = g_forceSplit.load(), kBlocks = (K + hcgemm::kBlockK - 1) / hcgemm::kBlockK;
+    if (measure && bn <= 0 && split <= 0 && 2.0 * M * N * K >= 2e11) {
+        PairGroupRows(K);               // the first call reads HCOMM_GEMM_GM
+        if (g_forceGm.load() <= 0) return MeasuredTile(A, B, C, M, N, K, lda, ldb, ldc, cap, t, estimate, stream);
+    }
     if (bn >= hcgemm::kWideN) t = {hcgemm::kWideN, 1, GemmKernel::WIDE};
     else if (bn > 0) t = {std::min(256, std::max(32, bn / 32 * 32)), t.split, GemmKernel::EXCHANGED};
     else if (split > 0 && t.kernel != GemmKernel::WIDE) t.kernel = GemmKernel::EXCHANGED;
@@ -389,10 +487,8 @@ HcclResult GemmBf16(const void *A, const void *B, void *C, int M, int N, int K, 
     static const bool pairEnabled = [] { const char *e = getenv("HCOMM_GEMM_PAIR"); return !(e && e[0] == '0'); }();
     const GemmLimits limits = Limits();
     if (pairEnabled && limits.cap[0] > 0) {
-        const PairTile tile = ChoosePairTile(M, N, K, limits.cap);
-        if (tile.kernel == GemmKernel::WIDE) return LaunchWideGemm(A, B, C, M, N, K, lda, ldb, ldc, stream);
-        if (tile.kernel == GemmKernel::ROWS224) return LaunchPair224Gemm(A, B, C, M, N, K, lda, ldb, ldc, stream);
-        if (tile.kernel == GemmKernel::EXCHANGED) return LaunchSwapGemm(A, B, C, M, N, K, lda, ldb, ldc, tile, stream);
+        const PairTile tile = ChoosePairTile(A, B, C, M, N, K, lda, ldb, ldc, limits.cap, stream);
+        if (tile.kernel != GemmKernel::SINGLE) return LaunchTile(A, B, C, M, N, K, lda, ldb, ldc, tile, stream);
     }
     // one CTA per 128-row tile: few columns, HCOMM_GEMM_PAIR=0, or a device that cannot hold a cluster
     const int BN = (N % 256 == 0 || N >= 2048) ? 256 : 128;
@@ -461,11 +557,13 @@ extern "C" int HcommToolGemmOrder(int M, int N, int K, int tileWidth, int t, int
     if (t >= 0 && t < g.tilesW * g.tilesT) hcgemm::SwapOrder(g, t, weightBlock, tokenBlock);
     return g.tilesW * g.tilesT;
 }
-// Kept for callers of earlier versions, which could time a shape at its first use: no measurement is made (0 / 0).
-extern "C" void HcommGemmGetTuned(int, int, int, int *tileWidth, int *groupRows)
+// Tile width and rasterisation group that the measurement at first use chose for a shape (0 / 0: none was made).
+extern "C" void HcommGemmGetTuned(int M, int N, int K, int *tileWidth, int *groupRows)
 {
-    if (tileWidth) *tileWidth = 0;
-    if (groupRows) *groupRows = 0;
+    std::lock_guard<std::mutex> lk(hc::g_tuneMu);
+    auto it = hc::g_tuned.find(hc::ShapeKey{M, N, K});
+    if (tileWidth) *tileWidth = it == hc::g_tuned.end() ? 0 : it->second.bn;
+    if (groupRows) *groupRows = it == hc::g_tuned.end() ? 0 : it->second.group;
 }
 extern "C" int HcommGemmTakeError(void)
 {

@@ -4,11 +4,14 @@
 
 C[M, N] = A[M, K] * B[N, K]^T.  The two implementations take turns (``rounds`` rounds of ``iters`` back-to-back calls
 each, CUDA events around every round), so a clock that drifts under the power cap touches both alike; the figure per
-implementation is the median of its rounds.  Operands of the default shapes exceed the L2.
+implementation is the median of its rounds.  With HCOMM_GEMM_AUTOTUNE=1 the first, untimed call lets the library measure
+and pick its tile width and rasterisation group for the shape and the choice is printed (0 / 0 otherwise: the model
+decided).  Operands of the default shapes exceed the L2.
 """
 from __future__ import annotations
 
 import argparse
+import ctypes
 import json
 import statistics
 import time
@@ -19,6 +22,7 @@ DEFAULT = "8192x28672x8192,8192x8192x28672,8192x8192x8192,8192x14336x8192,8192x8
 
 
 def main():
+    from .. import _lib
     from ..ops.gemm import gemm_bf16, take_kernel_error
     ap = argparse.ArgumentParser()
     ap.add_argument("--shapes", default=DEFAULT)
@@ -26,6 +30,7 @@ def main():
     ap.add_argument("--iters", type=int, default=5)
     ap.add_argument("--prespin", type=float, default=1.0)
     a = ap.parse_args()
+    lib = _lib.load()
     torch.cuda.set_device(0)
     w = torch.randn(4096, 4096, device="cuda", dtype=torch.bfloat16)
     t0 = time.time()
@@ -51,8 +56,10 @@ def main():
         c_ref = torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
         ours = lambda: gemm_bf16(x, wt, c_ours)
         ref = lambda: torch.matmul(x, wt.t(), out=c_ref)
-        ours(); ref()                                  # module load, cuBLAS' heuristics
+        ours(); ref()                                  # the library's measurement at first use, cuBLAS' heuristics
         torch.cuda.synchronize()
+        bn, gm = ctypes.c_int(0), ctypes.c_int(0)
+        lib.HcommGemmGetTuned(m, n, k, ctypes.byref(bn), ctypes.byref(gm))
         err = (c_ours.float() - c_ref.float()).abs().max().item()
         t_ours, t_ref = [], []
         for _ in range(a.rounds):
@@ -61,7 +68,8 @@ def main():
         mo, mr = statistics.median(t_ours), statistics.median(t_ref)
         fl = 2.0 * m * n * k
         print(json.dumps({"shape": [m, n, k], "ours_ms": round(mo, 4), "cublas_ms": round(mr, 4), "ours_tflops": round(fl / mo / 1e9, 1),
-                          "cublas_tflops": round(fl / mr / 1e9, 1), "speedup_vs_cublas": round(mr / mo, 3), "max_abs_diff": err}), flush=True)
+                          "cublas_tflops": round(fl / mr / 1e9, 1), "speedup_vs_cublas": round(mr / mo, 3), "tile_width": bn.value, "group_rows": gm.value,
+                          "max_abs_diff": err}), flush=True)
         del x, wt, c_ours, c_ref
     assert take_kernel_error() == 0
 

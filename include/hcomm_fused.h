@@ -32,7 +32,9 @@ int HcommGemmBf16(const void *A, const void *B, void *C, int M, int N, int K, in
 void HcommGemmSetTuning(int groupRows, int tileWidth);
 /* CTA pairs (1, 2 or 4) that share a tile of the plain GEMM along K; 0 = automatic. */
 void HcommGemmSetSplit(int pairsAlongK);
-/* Kept for callers of earlier versions, which could time a shape at its first use: no measurement is made, always 0 / 0. */
+/* With HCOMM_GEMM_AUTOTUNE=1, large shapes (2 * M * N * K >= 2e11) seen for the first time are timed once with the candidate
+ * tiles and groups on the caller's stream (not while it is being captured) and the fastest is kept for the process.
+ * Returns what was chosen for a shape, 0 / 0 if nothing was measured. */
 void HcommGemmGetTuned(int M, int N, int K, int *tileWidth, int *groupRows);
 /* Reads and clears the "a bounded wait expired inside a GEMM kernel" flag of the current device (0 = none). */
 int HcommGemmTakeError(void);
