@@ -23,8 +23,8 @@
 // overlap the experts' output, whose rows would otherwise be overwritten before they are read, and once the caller has
 // asked for the address of the slots.
 //
-// Device scratch (beyond inputs and outputs): numExperts u32 row cursors (second half of a 2 * numExperts table), cleared
-// by the route launch; the local row of every (token, k).
+// Device scratch (beyond inputs and outputs): numExperts u32 row cursors, cleared by the route launch and left as they are by
+// the dispatch (a single rank has none); the local row of every (token, k).
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -59,7 +59,7 @@ struct MoeParams {
     const __nv_bfloat16 *x;
     const int32_t *topkIdx;
     int numTokens;
-    uint32_t *scratch;                    // [2 * numExperts]: histogram, row cursors (zero between calls)
+    uint32_t *scratch;                    // [numExperts]: row cursors
     // combine
     const __nv_bfloat16 *y;
     const float *gates;
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(1024) MoeRouteKernel(const __grid_constant__ M
     const int tid = threadIdx.x;
     // four histograms, warps dealt over them: neighbouring lanes often hold the same expert and would queue for its counter
     __shared__ uint32_t sHist[4][kMaxExperts], sWarp[32];
-    uint32_t *cursor = p.scratch + E;
+    uint32_t *cursor = p.scratch;
     for (int e = tid; e < E; e += blockDim.x) {
 #pragma unroll
         for (int h = 0; h < 4; ++h) sHist[h][e] = 0;
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constan
     __shared__ uint32_t sBase[kMaxExperts], sWarp[16];
     __shared__ uint8_t *sRow[kClaims];
     __shared__ float *sScale[kClaims];
-    uint32_t *cursor = p.scratch + E;
+    uint32_t *cursor = p.scratch;
     const int t0 = (int)((int64_t)p.numTokens * blockIdx.x / gridDim.x), t1 = (int)((int64_t)p.numTokens * (blockIdx.x + 1) / gridDim.x);
     const int segs = H / 512, perRound = kClaims / K;
 
@@ -487,7 +487,7 @@ struct DeviceBlocks {
 // One block: the row cursors, the overflow count and the last dispatch's tokens, the local rows.  On failure nothing is kept.
 HcclResult MakeScratch(const DeviceBlocks &from, MoeCtx *m, int numExperts, int maxTokens, int topk)
 {
-    const size_t bytes = sizeof(uint32_t) * (2 * (size_t)numExperts + 64 + (size_t)maxTokens * topk);
+    const size_t bytes = sizeof(uint32_t) * ((size_t)numExperts + 64 + (size_t)maxTokens * topk);
     void *block = nullptr;
     cudaError_t e = from.take(&block, bytes);
     if (e != cudaSuccess || !block) {
@@ -503,7 +503,7 @@ HcclResult MakeScratch(const DeviceBlocks &from, MoeCtx *m, int numExperts, int 
         return HCCL_E_RUNTIME;
     }
     m->scratch = (uint32_t *)block;
-    m->overflow = m->scratch + 2 * numExperts;
+    m->overflow = m->scratch + numExperts;
     m->localRow = m->overflow + 64;
     return HCCL_SUCCESS;
 }
@@ -592,8 +592,9 @@ using namespace hc;
 //   * code that owns no handle it could hang a buffer on and would otherwise allocate and free around each call.
 //
 // Limits and rules:
-//   * a single rank counts in shared memory and does not touch the table;
-//   * at most kStaticScratchExperts experts (2 counters each, kStaticScratchBytes of device memory per process and
+//   * a single rank counts in shared memory and neither clears nor reads the table; the limits below hold for it all the
+//     same, so that a program meets them at any number of ranks;
+//   * at most kStaticScratchExperts experts (a counter each, kStaticScratchBytes of device memory per process and
 //     GPU, reserved when the library is loaded); larger exchanges are refused with HCCL_E_PARA;
 //   * the array's device address is looked up (cudaGetSymbolAddress) by HcommMoeCreate, which runs at set-up on the
 //     exchange's GPU; the dispatch call itself does no look-up, and it refuses (HCCL_E_PARA, before anything is queued)
@@ -606,8 +607,8 @@ using namespace hc;
 //   * ranks of one process that share a GPU (the single-GPU test arrangement) are refused: their launches are
 //     merged through a table that is created on demand, which this entry point promises not to do.
 constexpr int kStaticScratchExperts = 256;
-constexpr size_t kStaticScratchBytes = sizeof(uint32_t) * 2 * kStaticScratchExperts;
-static __device__ __align__(256) uint32_t g_staticDispatchScratch[2 * kStaticScratchExperts];
+constexpr size_t kStaticScratchBytes = sizeof(uint32_t) * kStaticScratchExperts;
+static __device__ __align__(256) uint32_t g_staticDispatchScratch[kStaticScratchExperts];
 
 // Device address of the table on the CURRENT device (in host code the array's name is only a stand-in for it).
 static uint32_t *ResolveStaticScratch()
@@ -811,8 +812,8 @@ int HcommMoeDispatchStaticScratch(void *handle, const void *x, const int32_t *to
     int st = c->state.load();
     if (st == (int)CommState::SUSPENDING || st == (int)CommState::SUSPENDED) return HCCL_E_SUSPENDING;
     CHK_RET(LaunchBarrierIfNeeded(c, stream));
-    // the kernel expects both counter rows at zero and the array may hold a previous call's leftovers
-    if (cudaMemsetAsync(m->staticScratch, 0, sizeof(uint32_t) * 2 * (size_t)m->lay.numExperts, (cudaStream_t)stream) != cudaSuccess) {
+    // the array may hold a previous call's leftovers
+    if (c->nRanks > 1 && cudaMemsetAsync(m->staticScratch, 0, sizeof(uint32_t) * (size_t)m->lay.numExperts, (cudaStream_t)stream) != cudaSuccess) {
         HCCL_ERROR("built-in dispatch scratch: clearing failed: %s", cudaGetErrorString(cudaGetLastError()));
         return HCCL_E_RUNTIME;
     }

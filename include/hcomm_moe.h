@@ -49,9 +49,10 @@ int HcommMoeTakeOverflow(void *handle);
 // HcommMoeDispatch with the kernel's per-expert counters kept in an array built into the library's device image
 // rather than in allocated memory: the call allocates nothing, on the device or through any library.  Same
 // arguments and results as HcommMoeDispatch.  This entry point has no counterpart in the reference library.
-// Up to 256 experts (2 KB of built-in scratch per process and GPU); larger exchanges return HCCL_E_PARA.
+// Up to 256 experts (1 KB of built-in scratch per process and GPU); larger exchanges return HCCL_E_PARA, with a single
+// rank too, which needs no counters in memory.
 // All calls on one GPU share the array: it is cleared at the start of every call, and calls that overlap in time
-// race on it.  The array's address is resolved by HcommMoeCreate (set-up time); the call must be made with the
+// race on it (not those of a single rank).  The array's address is resolved by HcommMoeCreate (set-up time); the call must be made with the
 // exchange's GPU current and is refused with HCCL_E_PARA otherwise.
 int HcommMoeDispatchStaticScratch(void *handle, const void *x, const int32_t *topkIdx, int numTokens, void *stream);
 #ifdef __cplusplus

@@ -330,12 +330,35 @@ def main():
         static_dispatch = _lib.load().HcommMoeDispatchStaticScratch
         static_dispatch.restype = ctypes.c_int
         static_dispatch.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
+        # The entry point that keeps its counters in the library's built-in device array (one process per GPU here: every rank
+        # uses its own GPU's array) against the ordinary one, twice in a row with different routings: the second call finds
+        # the first one's leftovers in the array.
+        other = torch.stack([torch.randperm(experts, device="cuda", generator=g)[:topk] for _ in range(tokens // 2)]).to(torch.int32).contiguous()
+
+        def snapshot():
+            # in a canonical order: the position inside a source rank's part of an expert depends on atomics
+            torch.cuda.synchronize()
+            offs, n = moe._offsets.clone(), int(moe._offsets[-1].item())
+            order = torch.argsort(moe._origin[:n])
+            expert = torch.bucketize(torch.arange(n, device="cuda"), offs[1:].long(), right=True)
+            return [offs, moe._origin[:n][order].clone(), expert[order], moe._rows[:n].view(torch.uint8)[order].clone(), moe._scales[:n][order].clone()]
+        wanted = []
+        for i in (idx, other):
+            moe.dispatch(x[:len(i)], i)
+            wanted.append(snapshot())
+            dist.barrier()
+        for _ in range(2):
+            for i, want in zip((idx, other), wanted):
+                rc = static_dispatch(moe._h, x.data_ptr(), i.data_ptr(), len(i), torch.cuda.current_stream().cuda_stream)
+                assert rc == 0, rc
+                for name, got, ref in zip(("offsets", "origins", "experts", "rows", "scales"), snapshot(), want):
+                    assert torch.equal(got, ref), ("static scratch", name)
+                dist.barrier()          # no rank writes into a peer's rows while that peer still compares them
+        stage("moe static scratch ok")
         for rep in range(3):
             if rep < 2:
                 rec = moe.dispatch(x, idx)
             else:
-                # the same exchange through the entry point that keeps its counters in the library's built-in device array
-                # (one process per GPU here: every rank uses its own GPU's array)
                 rc = static_dispatch(moe._h, x.data_ptr(), idx.data_ptr(), tokens, torch.cuda.current_stream().cuda_stream)
                 assert rc == 0, rc
                 rec = Received(moe._rows, moe._scales, moe._origin, moe._offsets)

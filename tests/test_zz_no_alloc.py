@@ -1,7 +1,8 @@
-"""HcommMoeDispatchStaticScratch: the dispatch kernel with its counters in the library's built-in device array.
+"""HcommMoeDispatchStaticScratch with one rank, called through the exported C symbol: it gives what HcommMoeDispatch gives,
+allocates nothing and refuses what it says it refuses.
 
-Called through the exported C symbol and compared with HcommMoeDispatch on the same inputs, twice in a row with
-different inputs (the second call finds the first call's leftovers in the shared array).
+One rank counts in shared memory, so the built-in counter array plays no part here: two calls in a row that share
+it are compared in the workers of the tests that run several ranks, each on a GPU of its own.
 """
 import ctypes
 
