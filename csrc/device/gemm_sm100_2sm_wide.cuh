@@ -74,14 +74,16 @@ __device__ __forceinline__ void GemmMainLoopPairWide(const CUtensorMap *tmA, con
     __syncthreads();
     ClusterSync();
     TcFenceAfter();
-    GridDependencyWait();   // every role, not only the producer: a bounded wait must not run down while the kernel in front still works
     const uint32_t tmemBase = st->tmemBase;
 
+    // Every role waits for the kernel in front before its first bounded wait, not only the producer: the bound must not run
+    // down while that kernel still works.
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (both CTAs)
         if (ElectOne()) {
             uint32_t it = 0;
             bool alive = true;
+            GridDependencyWait();           // up to here a CTA may run beside the tail of the kernel in front; all it writes follows its loads
             for (int t = firstTile; t < numTiles && alive; t += tileStep) {
                 int mb, nb;
                 order(t, g, &mb, &nb);
@@ -107,6 +109,7 @@ __device__ __forceinline__ void GemmMainLoopPairWide(const CUtensorMap *tmA, con
             constexpr uint32_t idesc = InstrDescBf16(kPairM, 256);
             uint32_t it = 0, tileIter = 0;
             bool alive = true;
+            GridDependencyWait();
             for (int t = firstTile; t < numTiles && alive; t += tileStep, ++tileIter) {
                 if (!MbarWait(&st->tmemEmpty[0], (tileIter & 1) ^ 1, &st->abort)) { alive = false; break; }
                 TcFenceAfter();
@@ -136,6 +139,7 @@ __device__ __forceinline__ void GemmMainLoopPairWide(const CUtensorMap *tmA, con
         uint8_t *mine = slab + lane * 128;                      // this lane's row of the slab
         uint32_t tileIter = 0;
         bool alive = true;
+        GridDependencyWait();
         for (int t = firstTile; t < numTiles && alive; t += tileStep, ++tileIter) {
             int mb, nb;
             order(t, g, &mb, &nb);

@@ -122,15 +122,17 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
     __syncthreads();
     ClusterSync();          // every barrier of the cluster is initialised before anything signals it
     TcFenceAfter();
-    GridDependencyWait();   // every role, not only the producer: a bounded wait must not run down while the kernel in front still works
     const uint32_t tmemBase = st->tmemBase;
 
+    // Every role waits for the kernel in front before its first bounded wait, not only the producer: the bound must not run
+    // down while that kernel still works.
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (both CTAs of a pair)
         if (ElectOne()) {
             int s = 0;
             uint32_t ph = 0;
             bool alive = true;
+            GridDependencyWait();           // up to here a CTA may run beside the tail of the kernel in front; all it writes follows its loads
             for (int t = firstTile; t < numTiles && alive; t += tileStep) {
                 int wb, tb;
                 SwapOrder(g, t, &wb, &tb);
@@ -155,6 +157,7 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
             int s = 0;
             uint32_t ph = 0, tileIter = 0;
             bool alive = true;
+            GridDependencyWait();
             for (int t = firstTile; t < numTiles && alive; t += tileStep, ++tileIter) {
                 const uint32_t acc = tileIter & 1, accPh = (tileIter >> 1) & 1;
                 if (!MbarWait(&st->tmemEmpty[acc], accPh ^ 1, &st->abort)) { alive = false; break; }
@@ -183,6 +186,7 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
         const int chunk = lane & 3, pair0 = lane >> 2;
         uint32_t tileIter = 0;
         bool alive = true;
+        GridDependencyWait();
         for (int t = firstTile; t < numTiles && alive; t += tileStep, ++tileIter) {
             int wb, tb;
             SwapOrder(g, t, &wb, &tb);
@@ -231,6 +235,7 @@ __device__ __forceinline__ void GemmMainLoopSwap(const CUtensorMap *tmW, const C
         int wb, tb;
         SwapOrder(g, firstTile, &wb, &tb);
         const int tokens = g.M - tb * g.bn < g.bn ? g.M - tb * g.bn : g.bn;
+        GridDependencyWait();
         if (MbarWait(&st->tmemFull[0], 0, &st->abort)) {
             TcFenceAfter();
             float *mine = (float *)smem + q * 32 + lane;
