@@ -7,6 +7,7 @@
     python -m hcomm_b200.utils.profile_cases allreduce       one-shot, two-shot all-reduce and all-gather kernels, two ranks sharing the GPU
     python -m hcomm_b200.utils.profile_cases fused_pair      the CTA-pair variants of the two fused kernels on a one-rank communicator
     python -m hcomm_b200.utils.profile_cases moe             MoE dispatch + combine, one rank (256 experts, top-8, hidden 7168)
+    python -m hcomm_b200.utils.profile_cases single          kernels of the single-GPU cases: the plain GEMM at five shapes, MoE, a scaled copy (two rounds of eight)
 
 Ranks that share the GPU run inside ONE cooperative launch (kernels that wait for each other are never separate
 launches on a GPU), so each case is a single process a profiler can wrap.  A few launches per kernel, a few hundred
@@ -169,10 +170,39 @@ def case_moe(reps=2):
     comm.destroy()
 
 
+def case_single(reps=2):
+    """Two rounds of: GEMM with exchanged operands (one, four and one pairs along K), with 256 x 224 tiles of tokens x weights and
+    without pairs, MoE dispatch and combine, all-reduce of one rank with a scale.  2 GB on the device."""
+    import hcomm_b200 as hb
+    from ..ops.gemm import gemm_bf16, take_kernel_error
+    from ..ops.moe import MoeExchange
+    comm = hb.Communicator(1, hb.get_root_info(), 0, buffer_mb=8)
+    e, k, h, t = 256, 8, 7168, 4096
+    moe = MoeExchange(comm, e, k, h, t, capacity_factor=1.0)
+    x = torch.randn(t, h, device="cuda").to(torch.bfloat16)
+    top = torch.randn(t, e, device="cuda").topk(k, dim=1)
+    idx, gates = top.indices.to(torch.int32).contiguous(), torch.softmax(top.values, 1).contiguous()
+    y = torch.randn(t * k, h, device="cuda", dtype=torch.bfloat16)
+    gemms = [(torch.randn(m, kk, device="cuda").to(torch.bfloat16), (torch.randn(n, kk, device="cuda") * 0.02).to(torch.bfloat16))
+             for m, n, kk in ((16, 28672, 8192), (96, 3584, 8192), (777, 14336, 4096), (512, 14336, 8192), (8192, 64, 512))]
+    bucket = torch.randn(33361921, device="cuda").to(torch.bfloat16)
+    scaled = torch.empty_like(bucket)
+    for _ in range(reps):
+        for a, w in gemms:
+            gemm_bf16(a, w)
+        moe.dispatch(x, idx)
+        moe.combine(y, gates)
+        comm.all_reduce_scaled(bucket, scaled, 0.125)
+    torch.cuda.synchronize()
+    assert take_kernel_error() == 0 and moe.overflow() == 0
+    moe.destroy()
+    comm.destroy()
+
+
 def main():
     torch.cuda.set_device(0)
     which = sys.argv[1] if len(sys.argv) > 1 else "gemm"
-    {"gemm": case_gemm, "gemm_up": case_gemm_up, "gemm_raster": case_gemm_raster, "fused": case_fused, "fused_pair": case_fused_pair, "allreduce": case_allreduce, "moe": case_moe}[which]()
+    {"gemm": case_gemm, "gemm_up": case_gemm_up, "gemm_raster": case_gemm_raster, "fused": case_fused, "fused_pair": case_fused_pair, "allreduce": case_allreduce, "moe": case_moe, "single": case_single}[which]()
     print(f"profile case {which}: done", flush=True)
 
 
