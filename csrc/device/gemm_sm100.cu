@@ -192,7 +192,8 @@ namespace {
 
 // Tile of the CTA-pair kernels for a shape: tokens per tile and pairs that share a tile along K for the one with exchanged
 // operands (gemm_sm100_swap.cuh), or 256 x 512 (gemm_sm100_2sm_wide.cuh).  The estimate below, in nanoseconds, was fitted to
-// timings of every tile at about 1600 shapes (M 1 .. 65536, N 8 .. 128256, K 64 .. 28672):
+// timings of every tile at about 1600 shapes (M 1 .. 65536, N 8 .. 128256, K 64 .. 28672).  It is not the best everywhere: one
+// shape in five is more than 5 % off its best tile, a few tokens with a K that is no multiple of 64 up to a third.
 //   * a 64-deep step of a 256 x bn tile takes 48 + 1.28 bn ns on the tensor core at the clock that a GPU under such load
 //     holds, but never less than its operands (16 KB of weights, 128 bytes per token and CTA) at 120 bytes per ns and SM;
 //   * tiles come in whole waves of the clusters that fit at once (74 of two CTAs, 33 of four, 15 of eight);
@@ -201,8 +202,8 @@ namespace {
 //     512: 2.7 / 3.1 / 4.2 us a tile; multiplying alone 0.4 / 1.5 / 3.0), which makes wide tiles the better ones:
 //     65536 x 4096 x 64 takes 119 us with 512/1, 310 with 64/1;
 //   * all operand traffic passes L2 at 13.5 TB/s, half as much again where K is no multiple of 64, so that rows straddle
-//     128-byte lines (seen from the third wave on: 16384 x 4096 x 1000 512/1 107 us, 256/1 122), every operand comes from HBM once at 6.5 TB/s, a tenth less when only a
-//     few SMs ask for it;
+//     128-byte lines (seen from the third wave on: 16384 x 4096 x 1000 512/1 107 us, 256/1 122); every operand comes from HBM
+//     once at 6.5 TB/s, a tenth less when only a few SMs ask for it;
 //     up to 256 tokens, where weights come from HBM and go to every token tile, a fifth of the L2 time adds to that of HBM
 //     (40 x 4096 x 4096 64/2 10.5 us, not 32/2 12.1);
 //   * a launch costs 3 us, emptying the last accumulator 6 ns per token, exchanging partial sums 1.5 us and 8 ns per token.
@@ -213,11 +214,13 @@ namespace {
 // 16 x 8192 x 28672 32/2 71 (165), 96 x 3584 x 8192 96/4 15 (51), 777 x 4096 x 14336 224/1 82 (97), 33 x 128256 x 4096
 // 64/1 165 (185), 5003 x 8192 x 3584 224/1 210 (235).  Half a second into a run at the power cap 8192 x 28672 x 8192 takes
 // 2929 with 256 x 512 and 3149 with 256 x 256 tiles (from a cool start 2988 and 2783), 8192 x 3584 x 8192 414 and 395.
+//
 // Results of at most 128 columns fill less than half of a tile's 256 weights, and all clusters read the same few lines of B at
 // the same time, which costs each step some ns for every cluster beyond 30.  The kernel without pairs (128 x 128 tiles, one
 // per SM) is the better one there from 2048 rows and up to a K of 1024, beyond 148 tiles up to 512: 16384 x 8 x 256 5.1 us (6.9
 // with the best exchanged tile), 8192 x 64 x 512 5.2 (6.1), 5956 x 24 x 936 7.8 (8.2); but 2048 x 64 x 1000 8.8 (6.4) where
 // few clusters do, 65536 x 8 x 1000 49 (38).  Below 2048 rows the exchanged tiles are ahead by a tenth and more.
+//
 // Layers are often a multiple of 224 wide (3584, 7168, 14336, 28672) and batches a multiple of 256 tokens.  Tiles of 256 tokens x
 // 224 weights, the roles not exchanged, then come out whole where 256 weights x any number of tokens leaves part of a wave
 // empty: 512 x 14336 x 8192 91 us (101 with 512/1), 256 x 14336 x 8192 52.8 (56), half a second into a run at the power cap
