@@ -652,10 +652,17 @@ int HcommMoeCreate(HcclComm comm, int numExperts, int topk, int hidden, int maxT
     L.totalBytes = off;
     HcclResult r = (HcclResult)HcommMemAlloc(&m->buf, L.totalBytes);
     if (r != HCCL_SUCCESS) { delete m; return r; }
-    r = MakeScratch({[](void **p, size_t n) { return cudaMalloc(p, n); }, cudaMemset, cudaFree}, m, numExperts, maxTokens, topk);
+    // Taking device memory waits for the GPU, so a single rank does it last, when what the caller has queued has run beside the
+    // registration.  With several ranks it comes first: taking a window back needs all of them.
+    const DeviceBlocks device = {[](void **p, size_t bytes) { return cudaMalloc(p, bytes); }, cudaMemset, cudaFree};
+    if (n > 1) r = MakeScratch(device, m, numExperts, maxTokens, topk);
     if (r != HCCL_SUCCESS) { HcommMemFree(m->buf); delete m; return r; }
     cudaMemset(m->buf, 0, L.offOrigin);
     r = HcclCommSymWinRegister(comm, m->buf, L.totalBytes, &m->win, 0);
+    if (r == HCCL_SUCCESS && n == 1) {
+        r = MakeScratch(device, m, numExperts, maxTokens, topk);
+        if (r != HCCL_SUCCESS) HcclCommSymWinDeregister(m->win);
+    }
     if (r != HCCL_SUCCESS) { cudaFree(m->scratch); HcommMemFree(m->buf); delete m; return r; }
     for (int q = 0; q < n; ++q) {
         void *pp = nullptr;
