@@ -61,3 +61,28 @@ def test_public_headers_compile_as_c():
         res = subprocess.run(["gcc", "-std=c11", "-fsyntax-only", "-Wall", f"-I{inc}", f"-I{cuda}", "-x", "c", "-"], input=f'#include "{rel}"\n',
                              capture_output=True, text=True)
         assert res.returncode == 0, f"{rel}:\n{res.stderr[-2000:]}"
+
+
+def test_kernels_resident_early_wait_for_the_kernel_in_front_before_any_bounded_wait():
+    """In a main loop that may be resident before the kernel in front has ended, every role waits for that end before its first
+    bounded wait: the bound would run down while that kernel still works, for instance waits for a late peer."""
+    seen = 0
+    for p in SOURCES:
+        text = p.read_text(errors="ignore")
+        if p.suffix != ".cuh" or "GridDependentsLaunch();" not in text:
+            continue
+        roles = re.split(r"//\s-{10,}", text[text.index("GridDependentsLaunch();"):])
+        for role in roles[1:]:
+            if "MbarWait(" not in role:
+                continue
+            seen += 1
+            assert 0 <= role.find("GridDependencyWait();") < role.index("MbarWait("), f"{p}: {role[:60]}"
+    assert seen >= 7          # producer, issuer, epilogue, and the split's accumulator
+
+
+def test_kernels_that_meet_other_ranks_let_nothing_start_early():
+    """griddepcontrol.launch_dependents in kernels that can run with several ranks is for a single rank only."""
+    text = (ROOT / "csrc" / "device" / "moe_kernels.cu").read_text()
+    lines = [ln for ln in text.splitlines() if "launch_dependents" in ln]
+    assert lines and all("if (p.overlaps)" in ln for ln in lines)
+    assert "hp.overlaps = m->comm->nRanks == 1;" in text
