@@ -197,12 +197,11 @@ bool TryLocal(Comm *c, const OpDesc &d, HcclResult *res)
         *res = HCCL_E_PARA;
         return true;
     }
-    // two rounds of the CTAs that fit at once (two of 512 threads per SM: 64 KB of loads in flight); small operands spread in
-    // shares of 32 KB, four 16-byte words per thread
-    static PerDevice<int> resident;
-    const int fit = resident.Get(c->device, [](int *n) { return (*n = FastMaxCoResidentCtas(FK_LOCAL, 512, 0)) > 0; });
-    const uint64_t most = 2 * (uint64_t)std::max(1, fit);
-    int ctas = (int)std::max<uint64_t>(1, std::min<uint64_t>(most, (count * esz + 32767) / 32768));
+    // one CTA of 512 threads per SM, loads for the next round in flight (see KLocal); small operands spread in shares of 8 KB, a
+    // 16-byte word per thread
+    static PerDevice<int> smCount;
+    const int sms = smCount.Get(c->device, [](int *n) { return (*n = FastSmCount()) > 0; });
+    int ctas = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)std::max(1, sms), (count * esz + 8191) / 8192));
     const int cap = EnvConfig::Get().maxCtas.value, forced = EnvConfig::Get().forceCtas.value;
     const uint32_t own = __atomic_load_n(&c->ctaLimit, __ATOMIC_RELAXED);
     if (cap > 0) ctas = std::min(ctas, cap);

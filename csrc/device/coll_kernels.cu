@@ -33,6 +33,7 @@
 
 #include "../alg/ir.h"
 #include "../core/log.h"
+#include "../core/dtype.h"
 #include "coll_kernels.h"
 #include "hcomm_device.cuh"
 
@@ -1269,78 +1270,154 @@ __global__ void __launch_bounds__(512) KIrInterp(const __grid_constant__ IrArgs 
 // ----------------------------------------------------------------------------------- single rank
 
 // A communicator of one rank: out = scale * in (or in as it is).  No peer shares the partition of the data, so there is no
-// staging, no window and no barrier, and the CTAs sweep the operand together, lanes side by side whatever the alignment:
-// words of W bytes, the widest that both buffers start on, four loads of each thread in flight.  Bound by HBM: 33.4 M bf16
-// values scaled into another buffer, 134 MB in all, take 29 us in back-to-back calls (79 with the staged two-shot kernel,
-// which kept half as many loads in flight and cut the operand into windows with barriers between them); a copy by the driver
-// takes 25.  One contiguous share per CTA instead of the common sweep cost 2 us.
-template <int BYTES> struct WordOf { using type = typename BitsOf<BYTES>::type; };
-template <> struct WordOf<16> { using type = uint4; };
-template <typename T, int W>
-__device__ __forceinline__ void LocalRange(const char *in, char *out, uint64_t words, bool useScale, float scale)
+// staging, no window and no barrier, and the CTAs sweep the operand together in 16-byte words of the result, whatever element
+// either buffer starts on: where the two start differently within 16 bytes (an operand is often a slice of a flat buffer), a
+// word is cut out of the two aligned words of `in` that hold it, the second of which comes from the neighbouring lane.
+// Only whole words inside the operand are read; up to 31 bytes at either end go element by element.
+// Bound by HBM.  One CTA per SM, whose loads of the next 48 KB are on their way while the ones before are being written; pieces
+// of 3 KB are dealt over the CTAs, so that small operands spread and the last round is an even one.  33.4 M bf16 values scaled
+// into another buffer, 134 MB: 22.5 us in back-to-back calls, three elements off 22.5 (26.7 and 55.3 with two rounds of two CTAs
+// per SM, no loads ahead, in words of the widest alignment that both buffers shared); 10.8 M fp32 values moved 10.2 us (17.7), 2048 1.9 (2.7).
+constexpr int kLocalWords = 6;          // words of a lane in flight: 4 take 25.1 us for 6's 23.8, 8 and more no less (134 MB)
+struct LocalSpan {
+    uint64_t head;          // bytes in front of the first whole word of `out`
+    uint64_t words;         // of `out`; shifted ones lie in one more of `in`
+    uint32_t delta;         // bytes by which that word's source starts beyond an aligned word of `in`
+};
+LocalSpan LocalSplit(uintptr_t in, uintptr_t out, uint64_t bytes)
 {
-    using V = typename WordOf<W>::type;
-    constexpr int N = W / (int)sizeof(T), U = 4;
-    union Word { V v; T e[N]; };
-    const uint64_t hi = words;
-    for (uint64_t i = (uint64_t)blockIdx.x * U * blockDim.x + threadIdx.x; i < hi; i += (uint64_t)gridDim.x * U * blockDim.x) {
-        Word w[U];
+    LocalSpan s;
+    s.head = (0 - out) & 15;
+    s.delta = (uint32_t)((in + s.head) & 15);
+    if (s.head < s.delta) s.head += 16;                                     // the word of `in` in front begins before the operand
+    // word i takes the words i and, when shifted, i + 1 of `in`, counted from in + head - delta
+    const uint64_t have = bytes + s.delta > s.head ? (bytes + s.delta - s.head) / 16 : 0;
+    s.words = s.delta == 0 || have == 0 ? have : have - 1;
+    if (s.words == 0) { s.head = 0; s.delta = 0; }                          // all of it is the tail
+    return s;
+}
+// What the kernel takes: no more than it needs, since every launch copies it.
+struct LocalArgs {
+    CommDev *dev;
+    const char *in;
+    char *out;
+    uint64_t bytes;
+    LocalSpan span;
+    float scale;
+    int useScale;
+};
+__device__ __forceinline__ uint4 LocalShift(const uint4 &lo, const uint4 &hi, uint32_t delta)
+{
+    uint32_t c[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (i + u * blockDim.x < hi) w[u].v = ((const V *)in)[i + u * blockDim.x];
+    for (int k = 0; k < 6; ++k) c[k] = (delta & 8) ? c[k + 2] : c[k];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (i + u * blockDim.x >= hi) continue;
-            if constexpr (!std::is_same<T, uint8_t>::value) {
-#pragma unroll
-                for (int j = 0; j < N; ++j) {
-                    const typename AccOf<T>::type a = Widen<T>(w[u].e[j]);
-                    w[u].e[j] = Narrow<T>(useScale ? ScaleAcc<typename AccOf<T>::type>(a, scale) : a);
-                }
-            }
-            ((V *)out)[i + u * blockDim.x] = w[u].v;
-        }
+    for (int k = 0; k < 5; ++k) c[k] = (delta & 4) ? c[k + 1] : c[k];
+    const uint32_t bits = (delta & 3) * 8;
+    return make_uint4(__funnelshift_r(c[0], c[1], bits), __funnelshift_r(c[1], c[2], bits), __funnelshift_r(c[2], c[3], bits), __funnelshift_r(c[3], c[4], bits));
+}
+template <typename T> __device__ __forceinline__ T LocalValue(T v, bool useScale, float scale)
+{
+    if constexpr (std::is_same<T, uint8_t>::value) return v;
+    else {
+        const typename AccOf<T>::type a = Widen<T>(v);
+        return Narrow<T>(useScale ? ScaleAcc<typename AccOf<T>::type>(a, scale) : a);
     }
 }
-template <typename T, int W>
-__device__ __forceinline__ void LocalMove(const char *in, char *out, uint64_t bytes, bool useScale, float scale)
+// src: the aligned word that word 0 of `out` begins in.  begun(): called once the first loads are on their way.
+template <typename T, bool SHIFTED, typename Begun>
+__device__ __forceinline__ void LocalRange(const uint4 *src, uint4 *out, const LocalSpan &s, bool useScale, float scale, Begun begun)
 {
-    HC_BOUNDS_OR_RETURN(in, bytes);
-    HC_BOUNDS_OR_RETURN(out, bytes);
-    LocalRange<T, W>(in, out, bytes / W, useScale, scale);
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x < (bytes % W) / sizeof(T)) {      // ragged end: fewer elements than a word
-        const uint64_t off = bytes / W * W + threadIdx.x * sizeof(T);
-        T v = *(const T *)(in + off);
-        if constexpr (!std::is_same<T, uint8_t>::value) {
-            const typename AccOf<T>::type a = Widen<T>(v);
-            v = Narrow<T>(useScale ? ScaleAcc<typename AccOf<T>::type>(a, scale) : a);
+    constexpr bool RAW = std::is_same<T, uint8_t>::value;
+    constexpr int N = 16 / (int)sizeof(T), U = kLocalWords;
+    union Word { uint4 v; typename std::conditional<RAW, uint32_t, T>::type e[RAW ? 4 : N]; };
+    const uint32_t keep = useScale ? 1u : 0u;               // bytes are moved as they are: 0
+    const int lane = threadIdx.x & 31;
+    const int64_t step = (int64_t)gridDim.x * U * blockDim.x;
+    const int64_t base = ((int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * (32 * U);     // of the warp's first piece
+    int64_t left = (int64_t)s.words - base;                 // words of `out` from the piece's first on
+    const int beyond = SHIFTED ? 1 : 0;                     // and one more of `in`
+    src += base + lane;
+    out += base + lane;
+    uint4 ahead[U], over = make_uint4(0, 0, 0, 0);          // this lane's words; lane 0: the word behind the piece
+    auto load = [&](const uint4 *from, int64_t n, int u) { if (u * 32 + lane < n + beyond && n > 0) ahead[u] = from[u * 32]; };
+    auto loadOver = [&](const uint4 *from, int64_t n) { if (SHIFTED && lane == 0 && U * 32 < n + beyond) over = from[U * 32]; };
+#pragma unroll
+    for (int u = 0; u < U; ++u) load(src, left, u);
+    loadOver(src, left);
+    begun();
+    while (left > 0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            Word w;
+            w.v = ahead[u];
+            if (SHIFTED) {
+                // lane 31 goes on in what lane 0 has of the next row of words
+                const uint4 give = lane != 0 ? ahead[u] : u + 1 < U ? ahead[u + 1 < U ? u + 1 : 0] : over;
+                uint4 hi;
+                hi.x = __shfl_sync(0xffffffffu, give.x, lane + 1);
+                hi.y = __shfl_sync(0xffffffffu, give.y, lane + 1);
+                hi.z = __shfl_sync(0xffffffffu, give.z, lane + 1);
+                hi.w = __shfl_sync(0xffffffffu, give.w, lane + 1);
+                w.v = LocalShift(ahead[u], hi, s.delta);
+            }
+            load(src + step, left - step, u);
+            if constexpr (RAW) {
+                // nothing to compute, but a store straight from the registers that the next load fills would hold that load up
+                w.v.x ^= keep; w.v.y ^= keep; w.v.z ^= keep; w.v.w ^= keep;
+            } else {
+#pragma unroll
+                for (int j = 0; j < N; ++j) w.e[j] = LocalValue<T>(w.e[j], useScale, scale);
+            }
+            if (u * 32 + lane < left) out[u * 32] = w.v;
         }
-        *(T *)(out + off) = v;
+        loadOver(src + step, left - step);
+        src += step;
+        out += step;
+        left -= step;
     }
 }
 template <typename T>
-__global__ void __launch_bounds__(512, 2) KLocal(const __grid_constant__ CollArgs byval, const CollArgs *emu)
+__device__ __forceinline__ void LocalEnds(const LocalArgs &a)
 {
-    HC_ARGS;
+    const uint64_t done = a.span.head + a.span.words * 16, ends = (a.span.head + a.bytes - done) / sizeof(T);
+    if (threadIdx.x < ends) {
+        const uint64_t off = threadIdx.x * sizeof(T), at = off < a.span.head ? off : off - a.span.head + done;
+        *(T *)(a.out + at) = LocalValue<T>(*(const T *)(a.in + at), a.useScale != 0, a.scale);
+    }
+}
+template <typename T, bool SHIFTED, typename Begun>
+__device__ __forceinline__ void LocalMove(const LocalArgs &a, Begun begun)
+{
+    LocalRange<T, SHIFTED>((const uint4 *)(a.in + a.span.head - a.span.delta), (uint4 *)(a.out + a.span.head), a.span, a.useScale != 0, a.scale, begun);
+    if (blockIdx.x == gridDim.x - 1) LocalEnds<T>(a);
+}
+template <typename T, bool SHIFTED>
+__global__ void __launch_bounds__(512, SHIFTED ? 1 : 2) KLocal(const __grid_constant__ LocalArgs a)
+{
     // launched with the stream-serialization attribute: resident before the kernel in front has ended, idle until it has
     asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
-    const LaunchState ls = KernelBegin(d);
-    const char *in = (const char *)a.in;
-    char *out = (char *)a.out;
-    const uint64_t bytes = a.count * sizeof(T);
-    if (!(std::is_same<T, uint8_t>::value && in == out)) {
-        const uintptr_t both = (uintptr_t)in | (uintptr_t)out;
-        if ((both & 15) == 0) LocalMove<T, 16>(in, out, bytes, a.useScale != 0, a.scale);
-        else if ((both & 7) == 0 && sizeof(T) <= 8) LocalMove<T, 8>(in, out, bytes, a.useScale != 0, a.scale);
-        else if constexpr (sizeof(T) <= 4) {
-            if ((both & 3) == 0) LocalMove<T, 4>(in, out, bytes, a.useScale != 0, a.scale);
-            else if constexpr (sizeof(T) <= 2) {
-                if ((both & 1) == 0) LocalMove<T, 2>(in, out, bytes, a.useScale != 0, a.scale);
-                else if constexpr (sizeof(T) == 1) LocalMove<T, 1>(in, out, bytes, a.useScale != 0, a.scale);
-            }
-        }
+    LaunchState ls = {};
+    uint32_t profile = 0;
+    const auto begun = [&] { ls = KernelBeginAlone(a.dev, &profile); };
+#ifdef HCOMM_DEBUG_BOUNDS
+    begun();
+    if (BoundsOk(a.in, a.bytes) && BoundsOk(a.out, a.bytes)) LocalMove<T, SHIFTED>(a, [] {});
+#else
+    LocalMove<T, SHIFTED>(a, begun);
+#endif
+    KernelEndAlone(a.dev, ls, profile);
+}
+template <bool SHIFTED> void *LocalKernelFor(int dtype)
+{
+    switch (dtype) {
+        case HCCL_DATA_TYPE_FP32: return (void *)KLocal<float, SHIFTED>;
+        case HCCL_DATA_TYPE_FP16: return (void *)KLocal<__half, SHIFTED>;
+        case HCCL_DATA_TYPE_BFP16: return (void *)KLocal<__nv_bfloat16, SHIFTED>;
+        case HCCL_DATA_TYPE_FP64: return (void *)KLocal<double, SHIFTED>;
+        case HCCL_DATA_TYPE_UINT8: return (void *)KLocal<uint8_t, SHIFTED>;
+        default: return nullptr;
     }
-    KernelEnd(d, ls, 0);
 }
 
 template <typename K> struct KernelOf { K fn; };
@@ -1407,15 +1484,7 @@ void *KernelFor(int kind, int dtype)
         case FK_SEND: return (void *)KSend;
         case FK_RECV: return (void *)KRecv;
         case FK_BARRIER: return (void *)KBarrier;
-        case FK_LOCAL:
-            switch (dtype) {
-                case HCCL_DATA_TYPE_FP32: return (void *)KLocal<float>;
-                case HCCL_DATA_TYPE_FP16: return (void *)KLocal<__half>;
-                case HCCL_DATA_TYPE_BFP16: return (void *)KLocal<__nv_bfloat16>;
-                case HCCL_DATA_TYPE_FP64: return (void *)KLocal<double>;
-                case HCCL_DATA_TYPE_UINT8: return (void *)KLocal<uint8_t>;
-                default: return nullptr;
-            }
+        case FK_LOCAL: return LocalKernelFor<false>(dtype);
         default: return ReduceKernelFor<>(kind, dtype);
     }
 }
@@ -1434,6 +1503,7 @@ void PreloadFastKernels()
             void *fn = KernelFor(k, dt);
             cudaFuncAttributes attr;
             if (fn) cudaFuncGetAttributes(&attr, fn);
+            if (k == FK_LOCAL && (fn = LocalKernelFor<true>(dt))) cudaFuncGetAttributes(&attr, fn);
         }
     for (int dt : dtypes) {
         void *fn = IrKernelFor(dt);
@@ -1467,6 +1537,16 @@ uint32_t FastKindBarriers(int32_t kind, int preBarrier)
     return k + (preBarrier ? 1 : 0);
 }
 
+int FastSmCount()
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return sms;
+}
+
 int FastMaxCoResidentCtas(int32_t kind, int threads, int ranksOnDevice)
 {
     void *fn = KernelFor(kind, HCCL_DATA_TYPE_FP32);
@@ -1498,6 +1578,11 @@ HcclResult LaunchFastKernel(const FastLaunch &l)
     bool coop = l.emuTable != nullptr;
     if (coop) e = cudaLaunchCooperativeKernel(fn, grid, block, params, 0, (cudaStream_t)l.stream);
     else if (l.kind == FK_LOCAL) {
+        const uint64_t bytes = args.count * DtypeSize((HcclDataType)args.dtype);
+        LocalArgs local = {args.dev, (const char *)args.in, (char *)args.out, bytes, LocalSplit((uintptr_t)args.in, (uintptr_t)args.out, bytes), args.scale, args.useScale};
+        if (args.dtype == HCCL_DATA_TYPE_UINT8 && args.in == args.out) { local.bytes = 0; local.span = {0, 0, 0}; }
+        if (local.span.delta != 0) fn = LocalKernelFor<true>(args.dtype);
+        params[0] = &local;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -1514,6 +1599,13 @@ HcclResult LaunchFastKernel(const FastLaunch &l)
     return HCCL_SUCCESS;
 }
 
+
+// The split of a single rank's copy: bytes in front, words, bytes by which their source is shifted.
+extern "C" void HcommToolLocalSplit(uint64_t in, uint64_t out, uint64_t bytes, uint64_t *head, uint64_t *words, uint32_t *delta)
+{
+    const LocalSpan s = LocalSplit((uintptr_t)in, (uintptr_t)out, bytes);
+    *head = s.head; *words = s.words; *delta = s.delta;
+}
 
 void *IrKernelFor(int dtype)
 {

@@ -243,6 +243,29 @@ __device__ __forceinline__ void KernelEnd(const CommDev *d, const LaunchState &s
         }
     }
 }
+// The same pair for a kernel of a single rank, which meets nobody: nothing waits for its stores but the end of the launch.  Its CTAs
+// read the state while their first loads are on their way, and the last one leaves after one atomic.
+__device__ __forceinline__ LaunchState KernelBeginAlone(const CommDev *d, uint32_t *profile)
+{
+    const LaunchState s = KernelBegin(d);
+    *profile = threadIdx.x == 0 ? d->profile : 0u;
+    return s;
+}
+__device__ __forceinline__ void KernelEndAlone(const CommDev *d, const LaunchState &s, uint32_t profile, uint32_t halvesUsed = 1)
+{
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    uint32_t *ctr = DevCounters(d);
+    if (profile) __threadfence();       // the time that is put down is that of the stores
+    if (gridDim.x > 1 && atomicInc(&ctr[2], gridDim.x - 1) != gridDim.x - 1) return;
+    *(volatile uint32_t *)&ctr[1] = s.seq - 1u + halvesUsed;
+    if (profile) {
+        const unsigned long long seq = atomicAdd(&DevOpCounters(d)[1], 1ull);
+        ((unsigned long long *)((char *)d + HC_DEV_TIMES_OFFSET))[2 * (seq % HC_DEV_TIME_SLOTS) + 1] = GlobalTimerNs();
+    } else {
+        atomicAdd(&DevOpCounters(d)[1], 1ull);
+    }
+}
 __device__ __forceinline__ char *CclHalf(const CommDev *d, int rank, uint32_t half)
 {
     return HcPeerHeap(d, rank) + d->bufOffset + (uint64_t)half * d->halfBytes;

@@ -1,0 +1,57 @@
+"""The copy kernel of a single rank: words of 16 bytes whatever element the buffers start on, the ends element by element."""
+import ctypes
+
+import pytest
+
+
+@pytest.mark.parametrize("bytes_", list(range(0, 140)) + [3071, 3072, 3073, 49152 + 5, 1 << 20])
+def test_split_reads_and_writes_inside_the_operand(bytes_):
+    from hcomm_b200 import _lib
+    lib = _lib.load()
+    head, words, delta = ctypes.c_uint64(), ctypes.c_uint64(), ctypes.c_uint32()
+    for i in range(16):
+        for o in range(16):
+            src, dst = 4096 + i, 8192 + o
+            lib.HcommToolLocalSplit(ctypes.c_uint64(src), ctypes.c_uint64(dst), ctypes.c_uint64(bytes_), ctypes.byref(head), ctypes.byref(words), ctypes.byref(delta))
+            h, w, d = head.value, words.value, delta.value
+            tail = bytes_ - h - 16 * w
+            assert 0 <= tail
+            if w == 0:
+                assert h == 0 and d == 0 and tail < 64
+                continue
+            assert h < 32 and tail < 32 and d < 16
+            first = src + h - d                     # the words of the source: one more than of the result where they are shifted
+            assert (dst + h) % 16 == 0 and first % 16 == 0
+            assert first >= src and first + 16 * (w + (d > 0)) <= src + bytes_
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,size", [("uint8", 1), ("bfloat16", 2), ("float32", 4), ("float64", 8)])
+def test_every_shift_between_the_buffers(name, size):
+    import torch
+
+    import hcomm_b200 as hb
+    dtype = getattr(torch, name)
+    torch.cuda.set_device(0)
+    comm = hb.Communicator(1, hb.get_root_info(), 0, buffer_mb=4)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(size)
+        steps = 16 // size
+        piece = 3072 // size                        # what a warp takes at a time
+        # no whole word; a piece and its neighbours; more pieces than one round of the grid's warps takes
+        for count in (1, 3 * steps, piece - 1, piece, piece + steps + 1, 8 * (1 << 20) // size + 5):
+            base = torch.randint(-100, 100, (count + 32,), device="cuda", generator=g).to(dtype)
+            for i in range(0, steps, max(1, steps // 8)):
+                for o in (0, 1, steps - 1):
+                    x = base[i:i + count]
+                    out = torch.full((count + 32,), 7, device="cuda", dtype=dtype)
+                    want = out.clone()
+                    want[o:o + count] = x
+                    comm.all_gather(x, out[o:o + count])
+                    assert torch.equal(out, want), (count, i, o)
+                    if dtype.is_floating_point:
+                        comm.all_reduce_scaled(x, out[o:o + count], 0.5)       # exact
+                        want[o:o + count] = x * 0.5
+                        assert torch.equal(out, want), (count, i, o)
+    finally:
+        comm.destroy()
