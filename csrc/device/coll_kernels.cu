@@ -1276,9 +1276,11 @@ __global__ void __launch_bounds__(512) KIrInterp(const __grid_constant__ IrArgs 
 // Only whole words inside the operand are read; up to 31 bytes at either end go element by element.
 // Bound by HBM.  One CTA per SM, whose loads of the next 48 KB are on their way while the ones before are being written; pieces
 // of 3 KB are dealt over the CTAs, so that small operands spread and the last round is an even one.  33.4 M bf16 values scaled
-// into another buffer, 134 MB: 22.5 us in back-to-back calls, three elements off 22.5 (26.7 and 55.3 with two rounds of two CTAs
-// per SM, no loads ahead, in words of the widest alignment that both buffers shared); 10.8 M fp32 values moved 10.2 us (17.7), 2048 1.9 (2.7).
+// into another buffer, 134 MB: 21.3 us in back-to-back calls, three elements off 22.7 (26.7 and 55.3 with two rounds of two CTAs
+// per SM, no loads ahead, in words of the widest alignment that both buffers shared); 10.8 M fp32 values moved 10.3 us (17.7), 2048 1.6 (2.7); 16.7 M fp32
+// three elements off 26.9 (36.2).
 constexpr int kLocalWords = 6;          // words of a lane in flight: 4 take 25.1 us for 6's 23.8, 8 and more no less (134 MB)
+constexpr int kLocalWordsShifted = 8;   // of shifted ones but 16-bit types, which do with 6: 26.9 us for 16.7 M fp32 values (30.3)
 struct LocalSpan {
     uint64_t head;          // bytes in front of the first whole word of `out`
     uint64_t words;         // of `out`; shifted ones lie in one more of `in`
@@ -1316,6 +1318,14 @@ __device__ __forceinline__ uint4 LocalShift(const uint4 &lo, const uint4 &hi, ui
     const uint32_t bits = (delta & 3) * 8;
     return make_uint4(__funnelshift_r(c[0], c[1], bits), __funnelshift_r(c[1], c[2], bits), __funnelshift_r(c[2], c[3], bits), __funnelshift_r(c[3], c[4], bits));
 }
+// Volatile, so that the loads ahead stay in front of the stores beside them.
+__device__ __forceinline__ uint4 LdWord(const uint4 *p)
+{
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void StWord(uint4 *p, const uint4 &v) { asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)); }
 template <typename T> __device__ __forceinline__ T LocalValue(T v, bool useScale, float scale)
 {
     if constexpr (std::is_same<T, uint8_t>::value) return v;
@@ -1329,7 +1339,7 @@ template <typename T, bool SHIFTED, typename Begun>
 __device__ __forceinline__ void LocalRange(const uint4 *src, uint4 *out, const LocalSpan &s, bool useScale, float scale, Begun begun)
 {
     constexpr bool RAW = std::is_same<T, uint8_t>::value;
-    constexpr int N = 16 / (int)sizeof(T), U = kLocalWords;
+    constexpr int N = 16 / (int)sizeof(T), U = SHIFTED && sizeof(T) != 2 ? kLocalWordsShifted : kLocalWords;
     union Word { uint4 v; typename std::conditional<RAW, uint32_t, T>::type e[RAW ? 4 : N]; };
     const uint32_t keep = useScale ? 1u : 0u;               // bytes are moved as they are: 0
     const int lane = threadIdx.x & 31;
@@ -1340,8 +1350,8 @@ __device__ __forceinline__ void LocalRange(const uint4 *src, uint4 *out, const L
     src += base + lane;
     out += base + lane;
     uint4 ahead[U], over = make_uint4(0, 0, 0, 0);          // this lane's words; lane 0: the word behind the piece
-    auto load = [&](const uint4 *from, int64_t n, int u) { if (u * 32 + lane < n + beyond && n > 0) ahead[u] = from[u * 32]; };
-    auto loadOver = [&](const uint4 *from, int64_t n) { if (SHIFTED && lane == 0 && U * 32 < n + beyond) over = from[U * 32]; };
+    auto load = [&](const uint4 *from, int64_t n, int u) { if (u * 32 + lane < n + beyond && n > 0) ahead[u] = LdWord(from + u * 32); };
+    auto loadOver = [&](const uint4 *from, int64_t n) { if (SHIFTED && lane == 0 && U * 32 < n + beyond) over = LdWord(from + U * 32); };
 #pragma unroll
     for (int u = 0; u < U; ++u) load(src, left, u);
     loadOver(src, left);
@@ -1369,7 +1379,7 @@ __device__ __forceinline__ void LocalRange(const uint4 *src, uint4 *out, const L
 #pragma unroll
                 for (int j = 0; j < N; ++j) w.e[j] = LocalValue<T>(w.e[j], useScale, scale);
             }
-            if (u * 32 + lane < left) out[u * 32] = w.v;
+            if (u * 32 + lane < left) StWord(out + u * 32, w.v);
         }
         loadOver(src + step, left - step);
         src += step;
@@ -1398,15 +1408,14 @@ __global__ void __launch_bounds__(512, SHIFTED ? 1 : 2) KLocal(const __grid_cons
     // launched with the stream-serialization attribute: resident before the kernel in front has ended, idle until it has
     asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
     LaunchState ls = {};
-    uint32_t profile = 0;
-    const auto begun = [&] { ls = KernelBeginAlone(a.dev, &profile); };
+    const auto begun = [&] { ls = KernelBeginAlone(a.dev); };
 #ifdef HCOMM_DEBUG_BOUNDS
     begun();
     if (BoundsOk(a.in, a.bytes) && BoundsOk(a.out, a.bytes)) LocalMove<T, SHIFTED>(a, [] {});
 #else
     LocalMove<T, SHIFTED>(a, begun);
 #endif
-    KernelEndAlone(a.dev, ls, profile);
+    KernelEndAlone(a.dev, ls);
 }
 template <bool SHIFTED> void *LocalKernelFor(int dtype)
 {

@@ -243,18 +243,26 @@ __device__ __forceinline__ void KernelEnd(const CommDev *d, const LaunchState &s
         }
     }
 }
-// The same pair for a kernel of a single rank, which meets nobody: nothing waits for its stores but the end of the launch.  Its CTAs
-// read the state while their first loads are on their way, and the last one leaves after one atomic.
-__device__ __forceinline__ LaunchState KernelBeginAlone(const CommDev *d, uint32_t *profile)
+// The same pair for a kernel of a single rank, which meets nobody: nothing waits for its stores but the end of the launch, and the
+// last CTA leaves after one atomic.  Whether times are recorded is fetched into shared memory meanwhile, so that it costs neither a
+// wait nor a register.
+__device__ __forceinline__ uint32_t *AloneProfile()
 {
-    const LaunchState s = KernelBegin(d);
-    *profile = threadIdx.x == 0 ? d->profile : 0u;
-    return s;
+    __shared__ uint32_t word;
+    return &word;
 }
-__device__ __forceinline__ void KernelEndAlone(const CommDev *d, const LaunchState &s, uint32_t profile, uint32_t halvesUsed = 1)
+__device__ __forceinline__ LaunchState KernelBeginAlone(const CommDev *d)
+{
+    if (threadIdx.x == 0)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(AloneProfile())), "l"(&d->profile) : "memory");
+    return KernelBegin(d);
+}
+__device__ __forceinline__ void KernelEndAlone(const CommDev *d, const LaunchState &s, uint32_t halvesUsed = 1)
 {
     __syncthreads();
     if (threadIdx.x != 0) return;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    const bool profile = *(volatile uint32_t *)AloneProfile() != 0;
     uint32_t *ctr = DevCounters(d);
     if (profile) __threadfence();       // the time that is put down is that of the stores
     if (gridDim.x > 1 && atomicInc(&ctr[2], gridDim.x - 1) != gridDim.x - 1) return;
