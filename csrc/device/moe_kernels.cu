@@ -76,8 +76,9 @@ constexpr uint32_t kNoRow = 0xffffffffu;
 // A single rank launches with the stream-serialization attribute: the CTAs are resident before the kernel in front has ended
 // and idle until it has, and the kernel behind may do the same.  Kernels that meet other ranks let nothing start early: what is
 // resident behind them would hold its SMs for as long as a peer is late.
-#define MOE_ARGS                                                                               \
-    const MoeParams &p = (table != nullptr) ? table[blockIdx.y] : byval;                       \
+#define MOE_ARGS MOE_ARGS_OF(table != nullptr)
+#define MOE_ARGS_OF(merged)                                                                    \
+    const MoeParams &p = (merged) ? table[blockIdx.y] : byval;                                 \
     if (p.overlaps) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");            \
     asm volatile("griddepcontrol.wait;" ::: "memory")
 
@@ -165,6 +166,32 @@ __global__ void __launch_bounds__(1024) MoeRouteKernel(const __grid_constant__ M
     KernelEnd(d, ls, 1, 0);
 }
 
+// A lane's 16 values as fp8, the scale of their block of 128: the eight lanes that share a block sit next to each other.
+__device__ __forceinline__ uint4 Quantise(const uint4 &lo, const uint4 &hi, float *blockScale)
+{
+    // the largest magnitude of the lane's 16 values (a maximum of bf16 values is exact in bf16)
+    const uint4 cur[2] = {lo, hi};
+    const __nv_bfloat162 *x2 = (const __nv_bfloat162 *)cur;
+    __nv_bfloat162 m2 = __habs2(x2[0]);
+#pragma unroll
+    for (int j = 1; j < 8; ++j) m2 = __hmax2(m2, __habs2(x2[j]));
+    float amax = fmaxf(0.f, fmaxf(__low2float(m2), __high2float(m2)));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+    const float scale = fmaxf(amax, 1e-4f) / 448.0f;   // values are divided (not multiplied by a reciprocal): bit-exact with x / scale
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 f0 = __bfloat1622float2(x2[2 * j]), f1 = __bfloat1622float2(x2[2 * j + 1]);
+        const __nv_fp8x2_storage_t first = __nv_cvt_float2_to_fp8x2(make_float2(f0.x / scale, f0.y / scale), __NV_SATFINITE, __NV_E4M3);
+        const __nv_fp8x2_storage_t second = __nv_cvt_float2_to_fp8x2(make_float2(f1.x / scale, f1.y / scale), __NV_SATFINITE, __NV_E4M3);
+        w[j] = (uint32_t)first | ((uint32_t)second << 16);
+    }
+    *blockScale = scale;
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // Dispatch, second launch (any number of CTAs, an ordinary launch that can share the GPU with expert GEMMs): every CTA
 // derives from the owners' count tables where this rank's rows of each expert start, claims the rows of its tokens, then
 // quantises and sends them, and meets its namesakes on the other ranks once all of its rows are on their way.
@@ -172,13 +199,7 @@ __global__ void __launch_bounds__(1024) MoeRouteKernel(const __grid_constant__ M
 // at HBM rate, and no less with a sixth of the divisions; 64 tokens 9 us (39).  A CTA owns whole tokens and its 16 warps share them in
 // pieces of 512 values, so that few tokens still occupy many warps and the claims cost one round of atomics per CTA, not one
 // per token.
-//
-// LOCAL (single rank): no route launch in front.  Every CTA counts the choices of all tokens, those of tokens before its own
-// apart: offsets and its first row of every expert follow without a word from another CTA, and rows are claimed from counters
-// in shared memory.  64 tokens 8.4 us, 4096 tokens 70 (route and dispatch: 5.3 + 8.9
-// and 9.9 + 69).
 constexpr int kClaims = 512;           // (token, k) pairs that a CTA claims at a time: one per thread
-template <bool LOCAL>
 __global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constant__ MoeParams byval, const MoeParams *table)
 {
     MOE_ARGS;
@@ -205,48 +226,6 @@ __global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constan
     // where do my rows of expert e start at its owner?  before them: all rows of the owner's earlier experts,
     // and the rows of this expert that come from lower ranks.  Every thread fetches the n counts of two experts
     // from their owner (independent loads, one NVLink round trip), then the prefix runs inside the CTA.
-    if constexpr (LOCAL) {
-        // two pairs of histograms, warps dealt over them: choices of tokens before t0, choices of the others
-        __shared__ uint32_t sCount[2][2][kMaxExperts];
-        for (int e = tid; e < E; e += blockDim.x) sCount[0][0][e] = sCount[0][1][e] = sCount[1][0][e] = sCount[1][1][e] = 0;
-        __syncthreads();
-        const int total = p.numTokens * K, mine = t0 * K, stride = blockDim.x;
-        for (int i = tid; i < total; i += 16 * stride) {        // sixteen loads in flight
-            int e[16];
-#pragma unroll
-            for (int u = 0; u < 16; ++u) e[u] = i + u * stride < total ? p.topkIdx[i + u * stride] : -1;
-#pragma unroll
-            for (int u = 0; u < 16; ++u)
-                if (e[u] >= 0 && e[u] < E) atomicAdd(&sCount[warp & 1][i + u * stride < mine ? 0 : 1][e[u]], 1u);
-        }
-        __syncthreads();
-        uint32_t before[2] = {0, 0}, tot[2] = {0, 0};
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int e = 2 * tid + j;
-            if (e < E) {
-                before[j] = sCount[0][0][e] + sCount[1][0][e];
-                tot[j] = before[j] + sCount[0][1][e] + sCount[1][1][e];
-            }
-        }
-        uint32_t first = BlockExclusiveScan(tot[0] + tot[1], sWarp);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int e = 2 * tid + j;
-            if (e < E) {
-                sBase[e] = first + before[j];
-                if (blockIdx.x == 0) {
-                    // offsets for the grouped GEMM, clamped to the receive capacity like the route launch's
-                    const uint32_t cap = (uint32_t)p.lay.maxRecvRows;
-                    Counts(p, me)[e] = tot[j];
-                    ExpertOffsets(p, me)[e] = first < cap ? first : cap;
-                    if (e == E - 1) ExpertOffsets(p, me)[E] = first + tot[j] < cap ? first + tot[j] : cap;
-                }
-                first += tot[j];
-            }
-        }
-        __syncthreads();
-    } else
     {
         uint32_t tot[2] = {0, 0}, below[2] = {0, 0};
 #pragma unroll
@@ -286,7 +265,7 @@ __global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constan
             const int e = p.topkIdx[tk];
             uint32_t slot = kNoRow, local = 0;
             if (e >= 0 && e < E) {
-                slot = LOCAL ? atomicAdd(&sBase[e], 1u) : sBase[e] + atomicAdd(&cursor[e], 1u);
+                slot = sBase[e] + atomicAdd(&cursor[e], 1u);
                 if (slot >= (uint32_t)p.lay.maxRecvRows) { atomicAdd(p.overflow, 1u); slot = kNoRow; }
             }
             Valid(p, me)[tk] = slot != kNoRow ? 1 : 0;
@@ -307,27 +286,8 @@ __global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constan
         for (int it = warp; it < items; it += warps) {
             const uint4 ca = a, cb = b;
             if (it + warps < items) { a = LdStream16(src + (size_t)(it + warps) * 512); b = LdStream16(src + (size_t)(it + warps) * 512 + 8); }
-            // the largest magnitude of the lane's 16 values (a maximum of bf16 values is exact in bf16)
-            const uint4 cur[2] = {ca, cb};
-            const __nv_bfloat162 *x2 = (const __nv_bfloat162 *)cur;
-            __nv_bfloat162 m2 = __habs2(x2[0]);
-#pragma unroll
-            for (int j = 1; j < 8; ++j) m2 = __hmax2(m2, __habs2(x2[j]));
-            float amax = fmaxf(0.f, fmaxf(__low2float(m2), __high2float(m2)));
-            // the 8 lanes that share a 128-value block sit next to each other
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-            const float scale = fmaxf(amax, 1e-4f) / 448.0f;   // values are divided (not multiplied by a reciprocal): bit-exact with x / scale
-            uint32_t w[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 f0 = __bfloat1622float2(x2[2 * j]), f1 = __bfloat1622float2(x2[2 * j + 1]);
-                const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(f0.x / scale, f0.y / scale), __NV_SATFINITE, __NV_E4M3);
-                const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(f1.x / scale, f1.y / scale), __NV_SATFINITE, __NV_E4M3);
-                w[j] = (uint32_t)lo | ((uint32_t)hi << 16);
-            }
-            const uint4 q = make_uint4(w[0], w[1], w[2], w[3]);
+            float scale;
+            const uint4 q = Quantise(ca, cb, &scale);
             const int tok = it / segs, seg = it - tok * segs, c0 = tok * K;
             for (int k = 0; k < K; ++k) {
                 uint8_t *row = sRow[c0 + k];
@@ -340,8 +300,144 @@ __global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constan
     }
     // all rows of this CTA are on their way; once every local CTA has passed its barrier (= the kernel has ended) all
     // CTAs of all ranks have sent
-    if (!LOCAL) CrossRankBarrier(d, ls.epoch0 + 1);
+    CrossRankBarrier(d, ls.epoch0 + 1);
     KernelEnd(d, ls, 1);
+}
+
+// Dispatch of a single rank: one launch, nobody to exchange counts with.  The two CTAs of a cluster count the choices of all tokens
+// together, half of them each, those of tokens before the cluster's apart, and read one another's counts: offsets and the first
+// row of every expert for every CTA follow without a word from another cluster, and rows are claimed from counters in shared
+// memory.  Then as above: the warps share the CTA's tokens in pieces of 512 values.
+// Bound by memory, and before that by the shared-memory atomics that count, during which memory is idle: hence, beyond kCountAlone
+// choices, one CTA of 1024 threads per SM and pairs of them, a quarter of the atomics of two CTAs of 512 that each count alone.  With
+// fewer choices the second CTA is worth more, and meeting costs more than counting (1024 x 8: 20.0 us alone, 23.5 in pairs; 2000 x 8:
+// 38.5 and 36.8).  4096 x 7168 to 8 of 256 experts 68.5 us (71.8 with every CTA counting alone), 9000 x 512 to 16 of 1024 29.6 (49.2), 64
+// tokens 7.1 (8.4).  Tried and no faster: rows put together in shared memory and sent with one bulk copy each (73 - 87 us), loads four
+// pieces ahead through shared memory (74.7), clusters of four CTAs of 512 (not all resident: 87).
+constexpr int kLocalThreads = 1024;
+constexpr int kCountAlone = 12288;
+
+__device__ __forceinline__ uint32_t LdClusterWord(const uint32_t *mine, uint32_t rank)
+{
+    uint32_t addr, v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+
+__global__ void __launch_bounds__(kLocalThreads, 1) MoeDispatchLocalKernel(const __grid_constant__ MoeParams byval, const MoeParams *)
+{
+    const MoeParams &p = byval;         // never merged with another rank's launch
+    if (p.overlaps) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const CommDev *d = p.dev;
+    const LaunchState ls = KernelBeginAlone(d);
+    const int E = p.lay.numExperts, K = p.lay.topk, H = p.lay.hidden;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    // choices of tokens before the cluster's and of the others, each twice: neighbouring lanes often hold the same expert and would
+    // queue for its counter, so the warps are dealt over two; and those of this CTA's tokens
+    __shared__ uint32_t sCount[2][2][kMaxExperts], sOwn[kMaxExperts], sBase[kMaxExperts], sWarp[32], sSlot[kLocalThreads];      // one claim of a row per thread at a time
+    uint32_t rank, ranks;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(ranks));
+    const auto firstToken = [&](uint32_t cta) { return (int)((int64_t)p.numTokens * cta / gridDim.x); };
+    const int t0 = firstToken(blockIdx.x), t1 = firstToken(blockIdx.x + 1), segs = H / 512, all = (t1 - t0) * segs;
+
+    // the first piece of this warp, and the choice that this thread claims a row for, are on their way while the rows are being found
+    uint4 a = make_uint4(0, 0, 0, 0), b = a;
+    const __nv_bfloat16 *src = p.x + (size_t)t0 * H + lane * 16;         // pieces of consecutive tokens are consecutive in x
+    auto fetch = [&](int item) { if (item < all) { a = LdStream16(src + (size_t)item * 512); b = LdStream16(src + (size_t)item * 512 + 8); } };
+    fetch(warp);
+    const int perRound = (int)blockDim.x / K, claimed = (t1 - t0 < perRound ? t1 - t0 : perRound) * K;
+    const int choice = tid < claimed ? p.topkIdx[(size_t)t0 * K + tid] : -1;
+
+    for (int e = tid; e < E; e += blockDim.x) sCount[0][0][e] = sCount[0][1][e] = sCount[1][0][e] = sCount[1][1][e] = sOwn[e] = 0;
+    __syncthreads();
+    {
+        const int total = p.numTokens * K, stride = blockDim.x, before = firstToken(blockIdx.x - rank) * K;
+        const int lo = (int)((int64_t)total * rank / ranks), hi = (int)((int64_t)total * (rank + 1) / ranks);
+        for (int i = lo + tid; i < hi; i += 16 * stride) {        // sixteen loads in flight
+            int e[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) e[u] = i + u * stride < hi ? p.topkIdx[i + u * stride] : -1;
+#pragma unroll
+            for (int u = 0; u < 16; ++u)
+                if (e[u] >= 0 && e[u] < E) atomicAdd(&sCount[warp & 1][i + u * stride < before ? 0 : 1][e[u]], 1u);
+        }
+        if (ranks > 1)
+            for (int i = t0 * K + tid; i < t1 * K; i += stride) {
+                const int e = p.topkIdx[i];
+                if (e >= 0 && e < E) atomicAdd(&sOwn[e], 1u);
+            }
+    }
+    if (ranks > 1) cg::this_cluster().sync();
+    else __syncthreads();
+    uint32_t first = 0, tot = 0;        // of expert tid: choices of tokens before this CTA's, of all
+    if (tid < E) {
+        first = sCount[0][0][tid] + sCount[1][0][tid];
+        tot = sCount[0][1][tid] + sCount[1][1][tid];
+        if (ranks > 1) {
+            const uint32_t peer = rank ^ 1u;
+            const uint32_t b0 = LdClusterWord(&sCount[0][0][tid], peer), b1 = LdClusterWord(&sCount[1][0][tid], peer);
+            const uint32_t a0 = LdClusterWord(&sCount[0][1][tid], peer), a1 = LdClusterWord(&sCount[1][1][tid], peer), own = LdClusterWord(&sOwn[tid], peer);
+            first += b0 + b1;
+            tot += a0 + a1 + first;
+            if (rank) first += own;
+        } else {
+            tot += first;
+        }
+    }
+    const uint32_t start = BlockExclusiveScan(tot, sWarp);
+    if (tid < E) {
+        sBase[tid] = start + first;
+        if (blockIdx.x == 0) {
+            // offsets for the grouped GEMM, clamped to the receive capacity like the route launch's
+            const uint32_t cap = (uint32_t)p.lay.maxRecvRows;
+            Counts(p, 0)[tid] = tot;
+            ExpertOffsets(p, 0)[tid] = start < cap ? start : cap;
+            if (tid == E - 1) ExpertOffsets(p, 0)[E] = start + tot < cap ? start + tot : cap;
+        }
+    }
+    if (ranks > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");       // its partner's counts have been read
+    __syncthreads();
+
+    if (blockIdx.x == 0 && tid == 0) p.overflow[1] = (uint32_t)p.numTokens;
+    int it = warp;
+    for (int r0 = t0; r0 < t1; r0 += perRound) {
+        const int tokens = t1 - r0 < perRound ? t1 - r0 : perRound;
+        if (tid < tokens * K) {
+            const size_t tk = (size_t)r0 * K + tid;
+            const int e = r0 == t0 ? choice : p.topkIdx[tk];
+            uint32_t slot = kNoRow;
+            if (e >= 0 && e < E) {
+                slot = atomicAdd(&sBase[e], 1u);
+                if (slot >= (uint32_t)p.lay.maxRecvRows) { atomicAdd(p.overflow, 1u); slot = kNoRow; }
+            }
+            Valid(p, 0)[tk] = slot != kNoRow ? 1 : 0;
+            if (slot != kNoRow) Origin(p, 0)[slot] = (uint32_t)tk;
+            p.localRow[tk] = slot + 1;          // kNoRow + 1 = 0: nowhere
+            sSlot[tid] = slot;
+        }
+        __syncthreads();
+        for (const int end = (r0 - t0 + tokens) * segs; it < end; it += warps) {
+            const uint4 ca = a, cb = b;
+            fetch(it + warps);
+            float scale;
+            const uint4 q = Quantise(ca, cb, &scale);
+            const int tok = it / segs - (r0 - t0), seg = it % segs;
+            uint8_t *row = Rows(p, 0) + seg * 512 + lane * 16;
+            float *rowScale = Scales(p, 0) + seg * 4 + (lane >> 3);
+            for (int k = 0; k < K; ++k) {
+                const uint32_t slot = sSlot[tok * K + k];
+                if (slot == kNoRow) continue;
+                *(uint4 *)(row + (size_t)slot * H) = q;
+                if ((lane & 7) == 0) rowScale[(size_t)slot * (H / kBlock)] = scale;
+            }
+        }
+        __syncthreads();        // the claims of the next round overwrite these
+    }
+    if (ranks > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // nobody leaves while another reads its counts
+    KernelEndAlone(d, ls);
 }
 
 // Combine, first launch: every expert output row of another rank's token (all rows with allThroughSlots) goes home, into slot (token, k) of that rank; each
@@ -379,18 +475,19 @@ __global__ void __launch_bounds__(512) MoeCombineSendKernel(const __grid_constan
 }
 
 // Combine, second launch (local): gate-weighted sum of the K rows of every local token, fp32 accumulation in the order of k.
-// Bound by memory: 2 k H bytes in, 2 H out per token; 3001 x 7168, 8 experts each, a tenth masked, 58 us (205 with every row
-// copied to its slot first), 54 at HBM rate; 64 tokens 6 us (13 + 43).  A warp takes segsPerItem segments of 256 columns of a token; lane k
+// Bound by memory: 2 k H bytes in, 2 H out per token; 3001 x 7168, 8 experts each, a tenth masked, 57 us (205 with every row
+// copied to its slot first), 54 at HBM rate; 64 tokens 4.5 us (13 + 43).  A warp takes segsPerItem segments of 256 columns of a token; lane k
 // finds the k-th row's address one item ahead, and every lane keeps the loads of eight rows of a segment in flight.
 constexpr int kSumThreads = 256, kSumCtasPerSm = 2;     // 128 registers a thread: eight addresses and gates of rows beside their loads; three CTAs spill and take 67 us for 58
-// BATCHES: groups of eight rows that K calls for.
-template <int BATCHES>
+// BATCHES: groups of eight rows that K calls for.  MERGED: ranks of one GPU in one launch; a choice at run time would put the
+// arguments behind a pointer.
+template <int BATCHES, bool MERGED>
 __global__ void __launch_bounds__(kSumThreads, kSumCtasPerSm) MoeCombineSumKernel(const __grid_constant__ MoeParams byval, const MoeParams *table)
 {
-    MOE_ARGS;
+    MOE_ARGS_OF(MERGED);
     const CommDev *d = p.dev;
     LaunchState ls = {};
-    if (p.countsLaunch) ls = KernelBegin(d);
+    if (p.countsLaunch) ls = KernelBeginAlone(d);
     const int me = d->rank, K = p.lay.topk, H = p.lay.hidden;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warpsPerCta = blockDim.x >> 5;
     const int segs = H / 256, perToken = (segs + p.segsPerItem - 1) / p.segsPerItem;
@@ -459,7 +556,13 @@ __global__ void __launch_bounds__(kSumThreads, kSumCtasPerSm) MoeCombineSumKerne
             *(uint4 *)((char *)(p.out + (size_t)t * H) + col) = outv;
         }
     }
-    if (p.countsLaunch) KernelEnd(d, ls, 1);
+    if (p.countsLaunch) KernelEndAlone(d, ls);
+}
+
+void *SumKernel(int topk, bool merged)
+{
+    if (topk <= 8) return merged ? (void *)MoeCombineSumKernel<1, true> : (void *)MoeCombineSumKernel<1, false>;
+    return merged ? (void *)MoeCombineSumKernel<2, true> : (void *)MoeCombineSumKernel<2, false>;
 }
 
 struct MoeCtx {
@@ -535,7 +638,7 @@ int MoeCtas(const Comm *c, int sms, int64_t useful)
 // One launch of `kernel` with `ctas` CTAs of `threads` threads.  Ordinary launches: nothing in these kernels waits for
 // another CTA of the same launch.  Ranks that share a GPU (tests) are merged into one cooperative launch with `emuCtas`
 // CTAs per rank, because their kernels wait for each other.
-HcclResult LaunchMoe(MoeCtx *m, void *kernel, const MoeParams &hp, int id, void *stream, int ctas, int emuCtas, int threads)
+HcclResult LaunchMoe(MoeCtx *m, void *kernel, const MoeParams &hp, int id, void *stream, int ctas, int emuCtas, int threads, int cluster = 1)
 {
     Comm *c = m->comm;
     const MoeParams *none = nullptr;
@@ -550,12 +653,18 @@ HcclResult LaunchMoe(MoeCtx *m, void *kernel, const MoeParams &hp, int id, void 
                                 });
     }
     void *args[] = {(void *)&hp, (void *)&none};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas, 1, 1); cfg.blockDim = dim3(threads, 1, 1); cfg.stream = (cudaStream_t)stream;
-    cfg.attrs = at; cfg.numAttrs = hp.overlaps ? 1 : 0;        // kernels that meet other ranks hold no SM before their turn
+    cfg.attrs = at;
+    if (hp.overlaps) {          // kernels that meet other ranks hold no SM before their turn
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        at[cfg.numAttrs].val.clusterDim.x = cluster; at[cfg.numAttrs].val.clusterDim.y = 1; at[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
     cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, args);
     if (e != cudaSuccess) { HCCL_ERROR("MoE launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
@@ -565,9 +674,15 @@ HcclResult LaunchMoe(MoeCtx *m, void *kernel, const MoeParams &hp, int id, void 
 HcclResult LaunchDispatch(MoeCtx *m, const MoeParams &hp, int routeId, int dispatchId, void *stream)
 {
     const int sms = MoeSms(), ctas = MoeCtas(m->comm, sms, hp.numTokens), emuCtas = std::max(1, sms / (int)m->comm->nRanks);
-    if (m->comm->nRanks == 1) return LaunchMoe(m, (void *)MoeDispatchKernel<true>, hp, dispatchId, stream, ctas, emuCtas, 512);
+    if (m->comm->nRanks == 1) {
+        // a thread per expert in any case
+        const bool many = (int64_t)hp.numTokens * m->lay.topk > kCountAlone;
+        const int threads = many || m->lay.numExperts > kLocalThreads / 2 ? kLocalThreads : kLocalThreads / 2;
+        const int mine = threads == kLocalThreads ? std::min(ctas, sms) : ctas, cluster = many && mine >= 2 ? 2 : 1;
+        return LaunchMoe(m, (void *)MoeDispatchLocalKernel, hp, dispatchId, stream, mine / cluster * cluster, emuCtas, threads, cluster);
+    }
     CHK_RET(LaunchMoe(m, (void *)MoeRouteKernel, hp, routeId, stream, 1, 1, 1024));
-    return LaunchMoe(m, (void *)MoeDispatchKernel<false>, hp, dispatchId, stream, ctas, emuCtas, 512);
+    return LaunchMoe(m, (void *)MoeDispatchKernel, hp, dispatchId, stream, ctas, emuCtas, 512);
 }
 
 }  // namespace
@@ -673,11 +788,10 @@ int HcommMoeCreate(HcclComm comm, int numExperts, int topk, int hidden, int maxT
     m->staticScratch = ResolveStaticScratch();       // set-up time, the exchange's GPU is current
     cudaFuncAttributes fa;
     cudaFuncGetAttributes(&fa, MoeRouteKernel);
-    cudaFuncGetAttributes(&fa, MoeDispatchKernel<false>);
-    cudaFuncGetAttributes(&fa, MoeDispatchKernel<true>);
+    cudaFuncGetAttributes(&fa, MoeDispatchKernel);
+    cudaFuncGetAttributes(&fa, MoeDispatchLocalKernel);
     cudaFuncGetAttributes(&fa, MoeCombineSendKernel);
-    cudaFuncGetAttributes(&fa, MoeCombineSumKernel<1>);
-    cudaFuncGetAttributes(&fa, MoeCombineSumKernel<2>);
+    for (bool merged : {false, true}) cudaFuncGetAttributes(&fa, SumKernel(topk, merged));
     cudaDeviceSynchronize();
     *handle = m;
     if (layoutOut) *layoutOut = L;
@@ -783,7 +897,7 @@ int HcommMoeCombineRows(void *handle, const void *y, uint64_t yRows, const float
     hp.segsPerItem = (int64_t)numTokens * ((segs + 3) / 4) >= (int64_t)warps * kSumCtasPerSm * sms ? 4 : 1;
     const int64_t items = (int64_t)numTokens * ((segs + hp.segsPerItem - 1) / hp.segsPerItem);
     const int forced = ForcedMoeCtas(), most = forced > 0 ? forced : kSumCtasPerSm * sms;
-    return LaunchMoe(m, m->lay.topk <= 8 ? (void *)MoeCombineSumKernel<1> : (void *)MoeCombineSumKernel<2>, hp, 9104, stream, (int)std::max<int64_t>(1, std::min<int64_t>(most, (items + warps - 1) / warps)), emuCtas, kSumThreads);
+    return LaunchMoe(m, SumKernel(m->lay.topk, c->emuSameDevice && c->nRanks > 1), hp, 9104, stream, (int)std::max<int64_t>(1, std::min<int64_t>(most, (items + warps - 1) / warps)), emuCtas, kSumThreads);
 }
 
 // ------------------------------------------------------------------ dispatch without any allocation

@@ -278,3 +278,41 @@ def test_result_inside_the_experts_output_and_rows_in_the_landing_area(n, hidden
     finally:
         run_ranks(n, lambda r: moes[r].destroy())
         run_ranks(n, lambda r: comms[r].destroy())
+
+
+@pytest.mark.parametrize("experts,topk,hidden,tokens,masked", [
+    (256, 8, 7168, 1, False),           # a token, one CTA
+    (8, 1, 512, 4096, True),            # as many choices as every CTA counts alone, and one more
+    (8, 1, 512, 4097, True),
+    (256, 8, 7168, 4145, True),         # the pairs' tokens do not come out even
+    (1024, 16, 512, 9600, False),       # a CTA claims rows twice, all counters
+    (64, 3, 8192, 3001, True),
+])
+def test_single_rank_dispatch_counts_and_claims(experts, topk, hidden, tokens, masked):
+    import hcomm_b200 as hb
+    from hcomm_b200.ops.moe import MoeExchange, quantize_e4m3_1x128
+    torch.cuda.set_device(0)
+    comm = hb.Communicator(1, hb.get_root_info(), 0, buffer_mb=8)
+    moe = MoeExchange(comm, experts, topk, hidden, tokens, capacity_factor=1.0)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(tokens)
+        x = torch.randn(tokens, hidden, device="cuda", generator=g).to(torch.bfloat16)
+        idx = torch.rand(tokens, experts, device="cuda", generator=g).topk(topk, dim=1).indices.to(torch.int32).contiguous()
+        if masked:
+            idx[torch.rand(tokens, topk, device="cuda", generator=g) < 0.2] = -1
+        rec = moe.dispatch(x, idx)
+        flat = idx.flatten().long()
+        kept = flat >= 0
+        n = int(kept.sum())
+        assert rec.num_rows == n and moe.overflow() == 0
+        counts = torch.bincount(flat[kept], minlength=experts)
+        assert torch.equal(rec.expert_offsets[1:].long(), counts.cumsum(0)) and int(rec.expert_offsets[0]) == 0
+        at = rec.origin[:n]
+        assert torch.equal(at.sort().values, kept.nonzero().flatten())
+        assert bool((flat[at].diff() >= 0).all())
+        q, scale = quantize_e4m3_1x128(x)
+        assert torch.equal(rec.rows[:n].view(torch.uint8), q.view(torch.uint8)[at // topk]) and torch.equal(rec.scales[:n], scale[at // topk])
+        assert torch.equal(moe.sent.flatten()[:tokens * topk] != 0, kept)
+    finally:
+        moe.destroy()
+        comm.destroy()
