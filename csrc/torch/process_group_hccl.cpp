@@ -546,10 +546,13 @@ c10::intrusive_ptr<c10d::Backend> CreateBackend(const c10::intrusive_ptr<c10d::S
     return pg;
 }
 
+bool AddNativeCalls(PyObject *module);      // native_calls.cpp
+
 }  // namespace hcomm_torch
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
 {
+    if (!hcomm_torch::AddNativeCalls(m.ptr())) throw py::error_already_set();
     using hcomm_torch::ProcessGroupHccl;
     py::class_<ProcessGroupHccl, c10d::Backend, c10::intrusive_ptr<ProcessGroupHccl>>(m, "ProcessGroupHCCL")
         .def("allreduce_scaled", &ProcessGroupHccl::AllreduceScaled, py::arg("input"), py::arg("output"), py::arg("scale"),

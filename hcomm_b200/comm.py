@@ -13,6 +13,7 @@ from typing import Optional, Sequence
 import numpy as np
 
 from . import _lib
+from ._ext import Short
 from ._lib import HcclError, check
 
 _NP_DTYPES = {
@@ -23,6 +24,10 @@ _NP_DTYPES = {
 _OPS = {"sum": _lib.SUM, "prod": _lib.PROD, "max": _lib.MAX, "min": _lib.MIN}
 
 
+# the short way of an operator and its number there
+_SHORT = {name: (Short("collective", entry), kind) for kind, (name, entry) in enumerate([
+    ("all_reduce", "HcclAllReduce"), ("all_reduce_scaled", "HcclAllReduceScaled"), ("reduce_scatter", "HcclReduceScatter"), ("all_gather", "HcclAllGather"),
+    ("all_to_all", "HcclAlltoAll")])}
 _TORCH_DTYPES = {}         # filled at the first tensor: importing this module does not import torch
 
 
@@ -158,8 +163,17 @@ class Communicator:
             return ctypes.c_void_p(int(stream))
         return ctypes.c_void_p(inferred) if inferred else None
 
+    def _short(self, name, send, recv, stream, op=0, scale=0.0):
+        """Whether the operator was launched the short way: torch tensors on the current stream."""
+        if stream is not None or isinstance(send, np.ndarray):
+            return False
+        call, kind = _SHORT[name]
+        return call(kind, send, recv, self._h.value, op, scale, self.size) is not None
+
     def all_reduce(self, send, recv=None, op: str = "sum", stream=None):
         recv = send if recv is None else recv
+        if self._short("all_reduce", send, recv, stream, _OPS[op]):
+            return recv
         sp, n, dt, st = describe(send)
         rp, _, _, _ = describe(recv)
         check(self._lib.HcclAllReduce(ctypes.c_void_p(sp), ctypes.c_void_p(rp), ctypes.c_uint64(n), dt, _OPS[op], self._h, self._stream(stream, st)),
@@ -168,6 +182,8 @@ class Communicator:
 
     def all_reduce_scaled(self, send, recv=None, scale: float = 1.0, stream=None):
         recv = send if recv is None else recv
+        if self._short("all_reduce_scaled", send, recv, stream, 0, scale):
+            return recv
         sp, n, dt, st = describe(send)
         rp, _, rdt, _ = describe(recv)
         check(self._lib.HcclAllReduceScaled(ctypes.c_void_p(sp), ctypes.c_void_p(rp), ctypes.c_uint64(n), dt, rdt, ctypes.c_float(scale), self._h,
@@ -180,6 +196,8 @@ class Communicator:
         return buf
 
     def reduce_scatter(self, send, recv, op: str = "sum", stream=None):
+        if self._short("reduce_scatter", send, recv, stream, _OPS[op]):
+            return recv
         sp, _, dt, st = describe(send)
         rp, n, _, _ = describe(recv)
         check(self._lib.HcclReduceScatter(ctypes.c_void_p(sp), ctypes.c_void_p(rp), ctypes.c_uint64(n), dt, _OPS[op], self._h, self._stream(stream, st)),
@@ -194,6 +212,8 @@ class Communicator:
         return recv
 
     def all_gather(self, send, recv, stream=None):
+        if self._short("all_gather", send, recv, stream):
+            return recv
         sp, n, dt, st = describe(send)
         rp, _, _, _ = describe(recv)
         check(self._lib.HcclAllGather(ctypes.c_void_p(sp), ctypes.c_void_p(rp), ctypes.c_uint64(n), dt, self._h, self._stream(stream, st)), "HcclAllGather")
@@ -207,6 +227,8 @@ class Communicator:
         return recv
 
     def all_to_all(self, send, recv, stream=None):
+        if self._short("all_to_all", send, recv, stream):
+            return recv
         sp, n, dt, st = describe(send)
         rp, _, _, _ = describe(recv)
         per = n // self.size

@@ -10,10 +10,17 @@ import ctypes
 import torch
 
 from .. import _lib
+from .._ext import Short
 from .._stream import raw_stream
 
 
+_short_gemm = Short("gemm_bf16", "HcommGemmBf16")
+
+
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    r = _short_gemm(a, b, out)
+    if r is not None:
+        return r
     if not (a.is_cuda and b.is_cuda):
         raise RuntimeError("gemm_bf16 runs on a CUDA device; the tcgen05 kernel has no CPU path")
     if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:

@@ -17,8 +17,13 @@ from dataclasses import dataclass
 import torch
 
 from .. import _lib
+from .._ext import Short
 from .._stream import raw_stream
 from ..comm import Communicator
+
+
+_short_dispatch = Short("moe_dispatch", "HcommMoeDispatch")
+_short_combine = Short("moe_combine", "HcommMoeCombineRows")
 
 
 class MoeLayout(ctypes.Structure):
@@ -78,6 +83,8 @@ class MoeExchange:
         self.sent = _view(ptrs[0].value - self.layout.offRows + self.layout.offValid, (max_tokens, topk), torch.uint8, dev)
 
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor) -> Received:
+        if _short_dispatch(self._h.value, x, topk_idx, self.hidden, self.topk) is not None:
+            return Received(self._rows, self._scales, self._origin, self._offsets)
         assert x.dtype == torch.bfloat16 and x.is_contiguous() and x.shape[1] == self.hidden
         assert topk_idx.dtype == torch.int32 and topk_idx.is_contiguous() and topk_idx.shape == (x.shape[0], self.topk)
         stream = raw_stream(x)
@@ -86,6 +93,9 @@ class MoeExchange:
         return Received(self._rows, self._scales, self._origin, self._offsets)
 
     def combine(self, y: torch.Tensor, gates: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+        r = _short_combine(self._h.value, y, gates, out, self.hidden)
+        if r is not None:
+            return r
         assert y.dtype == torch.bfloat16 and y.is_contiguous() and y.shape[1] == self.hidden
         assert gates.dtype == torch.float32 and gates.is_contiguous()
         t = gates.shape[0]

@@ -13,36 +13,13 @@ exposes the communicator management that backend sits on).
 """
 from __future__ import annotations
 
-import importlib.util
-import sys
-from pathlib import Path
-
 import torch
 import torch.distributed as dist
 
-from .. import _lib
+from .._ext import extension
 from ..comm import Communicator
 
-_EXT = None
 BACKEND_NAME = "hccl"
-
-
-def extension():
-    """The compiled extension module; built on first use when the shared object is missing."""
-    global _EXT
-    if _EXT is not None:
-        return _EXT
-    _lib.load()                                   # libhcomm.so first: the extension links against it
-    path = Path(__file__).resolve().parent.parent / "lib" / "_hcomm_torch.so"
-    if not path.exists():
-        from .. import build
-        build.build_torch_extension()
-    spec = importlib.util.spec_from_file_location("_hcomm_torch", str(path))
-    mod = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(mod)
-    sys.modules["_hcomm_torch"] = mod
-    _EXT = mod
-    return mod
 
 
 def _create(store, rank, size, timeout):
