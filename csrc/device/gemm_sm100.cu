@@ -53,10 +53,10 @@ GemmBf16SwapKernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     hcgemm::GemmMainLoopSwap<SPLIT>(&tmW, &tmX, shape);
 }
 
-// What the plain GEMM's kernels find on a device: clusters of 1, 2 and 4 CTA pairs that it holds at once, 0 where a kernel
+// What the plain GEMM's kernels find on a device: clusters of 1 to 4 CTA pairs that it holds at once, 0 where a kernel
 // cannot run, and whether the kernels without pairs have their shared memory.
 struct GemmLimits {
-    int cap[3];
+    int cap[4];
     bool single;
 };
 template <typename Kernel> bool AllowShared(Kernel *kernel, int bytes)
@@ -89,7 +89,8 @@ GemmLimits Limits()
     if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return {}; }
     return limits.Get(dev, [](GemmLimits *l) {
         const bool wide = AllowShared(GemmBf16PairWideKernel, hcgemm::ConfigWide<4>::kSmemBytes) && AllowShared(GemmBf16Pair224Kernel, hcgemm::Config2<224, 7>::kSmemBytes);
-        const bool one = ClustersAtOnce<1>(&l->cap[0]), two = ClustersAtOnce<2>(&l->cap[1]), four = ClustersAtOnce<4>(&l->cap[2]);
+        const bool one = ClustersAtOnce<1>(&l->cap[0]), two = ClustersAtOnce<2>(&l->cap[1]), four = ClustersAtOnce<4>(&l->cap[3]);
+        ClustersAtOnce<3>(&l->cap[2]);      // a device that holds none goes without
         if (!wide) l->cap[0] = 0;
         l->single = AllowShared(GemmBf16Kernel<256>, hcgemm::Config<256>::kSmemBytes) && AllowShared(GemmBf16Kernel<128>, hcgemm::Config<128>::kSmemBytes);
         return wide && one && two && four && l->single;
@@ -206,7 +207,8 @@ namespace {
 //     once at 6.5 TB/s, a tenth less when only a few SMs ask for it;
 //     up to 256 tokens, where weights come from HBM and go to every token tile, a fifth of the L2 time adds to that of HBM
 //     (40 x 4096 x 4096 64/2 10.5 us, not 32/2 12.1);
-//   * a launch costs 3 us, emptying the last accumulator 6 ns per token, exchanging partial sums 1.5 us and 8 ns per token.
+//   * a launch costs 3 us, emptying the last accumulator 6 ns per token, exchanging partial sums 0.6 us and 10 ns per token (three
+//     pairs up to 128 tokens only: beyond them they won nothing).
 //     Tiles are shared along K only where their clusters all fit at once: a further wave starts from nothing;
 //   * a 256 x 512 tile moves a quarter less operand data than two of 256 x 256, and under the power cap that sets the clock:
 //     690 ns a step against 752, but 4 us in which nothing overlaps the emptying of its one accumulator.
@@ -233,27 +235,27 @@ struct PairTile {
     int group = 0;              // rasterisation group, 0 = by rule
 };
 // Calls f(tile, estimate in ns) for every tile that can take the shape.
-template <typename F> void EachTile(int M, int N, int K, const int (&cap)[3], bool wide, F f)
+template <typename F> void EachTile(int M, int N, int K, const int (&cap)[4], bool wide, F f)
 {
     const double kBlocks = (K + hcgemm::kBlockK - 1) / hcgemm::kBlockK, tilesW = (N + hcgemm::kPairM - 1) / hcgemm::kPairM;
     const double straddle = K % hcgemm::kBlockK ? 1.5 : 1;
     const bool few = N <= 128 && (N < 64 || K % hcgemm::kBlockK);       // from 64 columns on, lines of B that do not straddle suffice
     const double hbmNs = 2.0 * ((double)M * K + (double)N * K + (double)M * N) / 6500.0;
-    for (int si = 0; si < 3; ++si) {
-        const int split = 1 << si;
-        if (cap[si] <= 0 || (split > 1 && kBlocks < 4 * split)) continue;
+    for (int split = 1; split <= 4; ++split) {
+        const int fit = cap[split - 1];
+        if (fit <= 0 || (split == 3 && M > 128) || (split > 1 && kBlocks < 4 * split)) continue;
         for (int bn = 256; bn >= 32; bn -= 32) {
             if (bn - 32 >= M) continue;                             // a narrower tile holds every token
             const double tiles = tilesW * ((M + bn - 1) / bn), x = std::min(bn, M);
-            const double waves = std::ceil(tiles / cap[si]), active = std::min(tiles, (double)cap[si]) * split / cap[0];
+            const double waves = std::ceil(tiles / fit), active = std::min(tiles, (double)fit) * split / cap[0];
             if (split > 1 && waves > 1) continue;
-            const double crowd = few ? (K <= 1024 ? 4 : 2) * std::max(0.0, std::min(tiles, (double)cap[si]) - 30) : 0;
+            const double crowd = few ? (K <= 1024 ? 4 : 2) * std::max(0.0, std::min(tiles, (double)fit) - 30) : 0;
             const double step = std::max(48 + 1.28 * bn, (16384 + 64 * x) / 120) + crowd;
             const double multiply = std::ceil(kBlocks / split) * step, empty = 1000 + 500 * std::ceil(x / 64);
             const double l2Ns = tiles * kBlocks * (32768 + 128 * x) / 13500 * (M > 256 && waves > 2 ? straddle : 1);
             const double loop = std::max(waves > 1 ? waves * std::max(multiply, std::sqrt(0.94 * multiply * multiply + empty * empty)) : multiply, l2Ns);
             f(PairTile{bn, split, GemmKernel::EXCHANGED},
-              std::max(loop, hbmNs / (0.9 + 0.1 * std::min(1.0, active))) + (M <= 256 ? 0.2 * l2Ns : 0) + 3000 + 6 * x + (split > 1 ? 1500 + 8 * x : 0));
+              std::max(loop, hbmNs / (0.9 + 0.1 * std::min(1.0, active))) + (M <= 256 ? 0.2 * l2Ns : 0) + 3000 + 6 * x + (split > 1 ? 600 + 10 * x : 0));
         }
     }
     if (cap[0] <= 0) return;
@@ -281,7 +283,7 @@ bool WideTiles()
     static const bool on = [] { const char *e = getenv("HCOMM_GEMM_WIDE"); return !(e && e[0] == '0'); }();
     return on;
 }
-PairTile PickPairTile(int M, int N, int K, const int (&cap)[3], double *estimate = nullptr)
+PairTile PickPairTile(int M, int N, int K, const int (&cap)[4], double *estimate = nullptr)
 {
     PairTile best{32, 1, GemmKernel::EXCHANGED};
     double bestNs = 0;
@@ -335,6 +337,7 @@ HcclResult LaunchSwapGemm(const void *A, const void *B, void *C, int M, int N, i
     cudaError_t e;
     switch (tile.split) {
         case 4: e = cudaLaunchKernelEx(&cfg, GemmBf16SwapKernel<4>, tmW, tmX, g); break;
+        case 3: e = cudaLaunchKernelEx(&cfg, GemmBf16SwapKernel<3>, tmW, tmX, g); break;
         case 2: e = cudaLaunchKernelEx(&cfg, GemmBf16SwapKernel<2>, tmW, tmX, g); break;
         default: e = cudaLaunchKernelEx(&cfg, GemmBf16SwapKernel<1>, tmW, tmX, g); break;
     }
@@ -406,7 +409,7 @@ struct ShapeKey {
 std::mutex g_tuneMu;
 std::map<ShapeKey, PairTile> g_tuned;
 
-PairTile MeasuredTile(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, const int (&cap)[3], const PairTile &rule, double estimate,
+PairTile MeasuredTile(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, const int (&cap)[4], const PairTile &rule, double estimate,
                       void *stream)
 {
     const ShapeKey key{M, N, K};
@@ -461,7 +464,7 @@ PairTile MeasuredTile(const void *A, const void *B, void *C, int M, int N, int K
     return g_tuned.emplace(key, cands[win]).first->second;
 }
 
-PairTile ChoosePairTile(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, const int (&cap)[3], void *stream)
+PairTile ChoosePairTile(const void *A, const void *B, void *C, int M, int N, int K, int lda, int ldb, int ldc, const int (&cap)[4], void *stream)
 {
     static const bool measure = [] { const char *e = getenv("HCOMM_GEMM_AUTOTUNE"); return e && e[0] == '1'; }();
     double estimate = 0;
@@ -474,7 +477,7 @@ PairTile ChoosePairTile(const void *A, const void *B, void *C, int M, int N, int
     if (bn >= hcgemm::kWideN) t = {hcgemm::kWideN, 1, GemmKernel::WIDE};
     else if (bn > 0) t = {std::min(256, std::max(32, bn / 32 * 32)), t.split, GemmKernel::EXCHANGED};
     else if (split > 0 && t.kernel != GemmKernel::WIDE) t.kernel = GemmKernel::EXCHANGED;
-    if (t.bn <= 256 && (split == 1 || split == 2 || split == 4) && split <= kBlocks && cap[split / 2] > 0) t.split = split;
+    if (t.bn <= 256 && split >= 1 && split <= 4 && split <= kBlocks && cap[split - 1] > 0) t.split = split;
     return t;
 }
 
@@ -534,7 +537,7 @@ extern "C" void HcommGemmSetTuning(int groupRows, int tileWidth)
     hc::g_forceGm.store(groupRows > 0 ? groupRows : 0);
     hc::g_forceBn.store(tileWidth > 0 ? tileWidth : 0);
 }
-// CTA pairs (1, 2 or 4) that share a tile along K; 0 = automatic.
+// CTA pairs (1 to 4) that share a tile along K; 0 = automatic.
 extern "C" void HcommGemmSetSplit(int pairsAlongK)
 {
     hc::g_forceSplit.store(pairsAlongK);
@@ -542,15 +545,29 @@ extern "C" void HcommGemmSetSplit(int pairsAlongK)
 // The rule behind the automatic choice, for a device that holds cap1, cap2 and cap4 clusters of 1, 2 and 4 CTA pairs at once.
 extern "C" void HcommToolGemmTile(int M, int N, int K, int cap1, int cap2, int cap4, int *tileWidth, int *pairsAlongK)
 {
-    const int cap[3] = {cap1, cap2, cap4};
+    const int cap[4] = {cap1, cap2, 0, cap4};
     const hc::PairTile t = hc::PickPairTile(M, N, K, cap);
     if (tileWidth) *tileWidth = t.bn;
     if (pairsAlongK) *pairsAlongK = t.split;
 }
+// The same for a device that holds caps[0] .. caps[3] clusters of 1 .. 4 pairs (HcommToolGemmTile: none of three).
+extern "C" void HcommToolGemmTileOf(int M, int N, int K, const int *caps, int *tileWidth, int *pairsAlongK)
+{
+    const int cap[4] = {caps[0], caps[1], caps[2], caps[3]};
+    const hc::PairTile t = hc::PickPairTile(M, N, K, cap);
+    if (tileWidth) *tileWidth = t.bn;
+    if (pairsAlongK) *pairsAlongK = t.split;
+}
+// What the current device holds.
+extern "C" void HcommToolGemmCaps(int *caps)
+{
+    const hc::GemmLimits l = hc::Limits();
+    for (int i = 0; i < 4; ++i) caps[i] = l.cap[i];
+}
 // Which kernel that rule takes: 0 exchanged operands, 1 tiles of 256 x 512, 2 without pairs, 3 tiles of 256 tokens x 224 weights.
 extern "C" int HcommToolGemmKernel(int M, int N, int K, int cap1, int cap2, int cap4)
 {
-    const int cap[3] = {cap1, cap2, cap4};
+    const int cap[4] = {cap1, cap2, 0, cap4};
     return (int)hc::PickPairTile(M, N, K, cap).kernel;
 }
 // The blocks (256 weights, tileWidth tokens) of tile t of the GEMM with exchanged operands; returns the number of tiles.

@@ -9,7 +9,7 @@
 //     Weights come in multiples of 256 nearly always, tokens in any number: 16 decoded tokens cost a 32-column tile
 //     instead of 128 or 256 rows of which 16 are real, and 777 tokens cost 800 columns instead of 1024 rows;
 //   * edges need no other kernel: TMA fills rows beyond M and N with zeros and the epilogue leaves them out.
-// SPLIT pairs of one cluster share a tile along K (1, 2 or 4 pairs): each multiplies its part of K, parks its fp32
+// SPLIT pairs of one cluster share a tile along K (1 to 4 pairs): each multiplies its part of K, parks its fp32
 // accumulator in its own shared memory (the ring is idle by then), and after one cluster barrier every pair adds the
 // SPLIT partial sums of its share of the tokens over distributed shared memory, in the order of K.  Nothing goes through
 // global memory, nothing has to be cleared, no CTA waits for one that may not be resident, and the result does not

@@ -13,7 +13,7 @@
 //                     the CTA's threads claim the rows of its tokens' experts in parallel (atomics on the row cursors),
 //                     then its warps quantise 512 values of a token at a time and store them to the token's k rows;
 //                     each CTA ends with one cross-rank barrier with its namesakes
-// A single rank has no counts to exchange: one launch, in which every CTA counts all choices itself.
+// A single rank has no counts to exchange: one launch, in which CTAs count all choices alone or in pairs.
 // Combine, rank r (owner of experts) - two ordinary launches, one when there is a single rank:
 //   send  one warp per row received from ANOTHER rank: the bf16 expert output goes to slot (token, k) of the token's rank;
 //         cross-rank barrier

@@ -167,3 +167,32 @@ def test_round_batch_of_a_layer_224_wide():
     # one rounding to bf16 (half a step, 2^-9) and fp32 sums of k products (k * 2^-24 of the sum of magnitudes)
     bound = 2.0 ** -8 * ref.abs() + k * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t())
     assert bool(((full[:, :n].double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 1000), (33, 1032, 4096), (128, 3584, 1000), (160, 4096, 1024), (129, 776, 2056), (257, 264, 520)])
+@pytest.mark.parametrize("split", [1, 2, 3, 4])
+def test_every_number_of_parts_of_k(m, n, k, split):
+    from hcomm_b200 import _lib
+    from hcomm_b200.ops.gemm import gemm_bf16, take_kernel_error
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    a = torch.randn(m, k + 8, device="cuda", generator=g).to(torch.bfloat16)[:, :k]
+    b = (torch.randn(n, k, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    full = torch.full((m, n + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    lib = _lib.load()
+    ref = a.double() @ b.double().t()
+    # one rounding to bf16 (half a step, 2^-9) and fp32 sums of k products (k * 2^-24 of the sum of magnitudes)
+    bound = 2.0 ** -8 * ref.abs() + k * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t())
+    try:
+        for width in (32, 96, 160, 192):
+            lib.HcommGemmSetTuning(0, width)
+            lib.HcommGemmSetSplit(split)
+            for _ in range(2):          # the second call behind the first
+                full.fill_(7.0)
+                gemm_bf16(a, b, full[:, :n])
+                gemm_bf16(a, b, full[:, :n])
+            torch.cuda.synchronize()
+            assert take_kernel_error() == 0 and bool((full[:, n:] == 7.0).all())
+            assert bool(((full[:, :n].double() - ref).abs() <= bound).all()), width
+    finally:
+        lib.HcommGemmSetTuning(0, 0)
+        lib.HcommGemmSetSplit(0)
