@@ -193,11 +193,11 @@ namespace {
 
 // Tile of the CTA-pair kernels for a shape: tokens per tile and pairs that share a tile along K for the one with exchanged
 // operands (gemm_sm100_swap.cuh), or 256 x 512 (gemm_sm100_2sm_wide.cuh).  The estimate below, in nanoseconds, was fitted to
-// timings of every tile at about 1600 shapes (M 1 .. 65536, N 8 .. 128256, K 64 .. 28672).  It is not the best everywhere: one
-// shape in five is more than 5 % off its best tile, a few tokens with a K that is no multiple of 64 up to a third.
+// timings of every tile at about 1600 shapes (M 1 .. 65536, N 8 .. 128256, K 64 .. 28672).  It is not the best everywhere: of
+// 150 shapes up to 700 tokens 11 are 4 - 13 % off their best tile.
 //   * a 64-deep step of a 256 x bn tile takes 48 + 1.28 bn ns on the tensor core at the clock that a GPU under such load
 //     holds, but never less than its operands (16 KB of weights, 128 bytes per token and CTA) at 120 bytes per ns and SM;
-//   * tiles come in whole waves of the clusters that fit at once (74 of two CTAs, 33 of four, 15 of eight);
+//   * tiles come in whole waves of the clusters that fit at once (74 of two CTAs, 33 of four, 22 of six, 15 of eight);
 //   * a tile's accumulator is emptied while the next tile is multiplied, in 1 us and 0.5 for every 64 tokens begun.  Where K is
 //     shallow neither hides the other: measured, the two add up like the sides of a right angle (256 tokens, K of 64 / 256 /
 //     512: 2.7 / 3.1 / 4.2 us a tile; multiplying alone 0.4 / 1.5 / 3.0), which makes wide tiles the better ones:
