@@ -16,9 +16,11 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include "hccl/hccl_types.h"
+#include "released.h"
 
 namespace {
 
+using hcomm_torch::Released;
 using AllReduceFn = int (*)(void *, void *, uint64_t, int, int, void *, void *);
 using AllReduceScaledFn = int (*)(void *, void *, uint64_t, int, int, float, void *, void *);
 using AllGatherFn = int (*)(void *, void *, uint64_t, int, void *, void *);
@@ -68,14 +70,6 @@ int TypeCode(at::ScalarType t)
         case at::kHalf: return HCCL_DATA_TYPE_FP16; case at::kBFloat16: return HCCL_DATA_TYPE_BFP16; case at::kDouble: return HCCL_DATA_TYPE_FP64;
         default: return -1;
     }
-}
-
-template <typename Call> int Released(Call call)
-{
-    PyThreadState *save = PyEval_SaveThread();
-    const int rc = call();
-    PyEval_RestoreThread(save);
-    return rc;
 }
 
 // A matrix of bf16 whose rows are contiguous and whose sizes the entry points can take.

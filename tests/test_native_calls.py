@@ -1,5 +1,23 @@
 """The short way from Python to the C entry points: taken for plain CUDA tensors, left to the general way for anything else."""
+import subprocess
+import sys
+import sysconfig
+from pathlib import Path
+
 import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+
+
+def test_the_interpreter_lock_is_held_again_behind_an_exception(tmp_path):
+    # an allocation that fails inside an entry point comes out of it as a C++ exception, of which a Python error is made
+    so = tmp_path / "released_probe.so"
+    cmd = ["g++", "-std=c++17", "-O1", "-shared", "-fPIC", f"-I{sysconfig.get_paths()['include']}", str(ROOT / "tests" / "released_probe.cc"), "-o", str(so)]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    assert res.returncode == 0, res.stderr
+    program = "import released_probe as p; print(*p.returns(), p.throws(), *p.returns())"
+    res = subprocess.run([sys.executable, "-c", program], capture_output=True, text=True, timeout=60, cwd=tmp_path)
+    assert res.returncode == 0 and res.stdout.split() == ["0", "1", "1", "0", "1"], res.stdout + res.stderr
 
 
 def test_without_a_gpu_the_general_way_is_taken():
