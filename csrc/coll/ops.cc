@@ -197,11 +197,9 @@ bool TryLocal(Comm *c, const OpDesc &d, HcclResult *res)
         *res = HCCL_E_PARA;
         return true;
     }
-    // one CTA of 512 threads per SM, loads for the next round in flight (see KLocal); small operands spread in shares of 8 KB, a
-    // 16-byte word per thread
     static PerDevice<int> smCount;
     const int sms = smCount.Get(c->device, [](int *n) { return (*n = FastSmCount()) > 0; });
-    int ctas = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)std::max(1, sms), (count * esz + 8191) / 8192));
+    int ctas = LocalCtas(count * esz, (((uintptr_t)a.in ^ (uintptr_t)a.out) & 15) != 0, std::max(1, sms));
     const int cap = EnvConfig::Get().maxCtas.value, forced = EnvConfig::Get().forceCtas.value;
     const uint32_t own = __atomic_load_n(&c->ctaLimit, __ATOMIC_RELAXED);
     if (cap > 0) ctas = std::min(ctas, cap);

@@ -1298,6 +1298,20 @@ LocalSpan LocalSplit(uintptr_t in, uintptr_t out, uint64_t bytes)
     if (s.words == 0) { s.head = 0; s.delta = 0; }                          // all of it is the tail
     return s;
 }
+}  // namespace
+// CTAs of the copy, for a device of `sms` SMs:
+//   * up to 3 MB, which 64 CTAs hold in one round, no more than 64: the next call's CTAs then find SMs of their own and do not wait
+//     for this call's to leave theirs.  us a call in replayed graphs, bf16 values: 1 MB 2.9 (4.0 with 128 CTAs, 3.6 with the 32 of before),
+//     2 MB 3.1 (4.2 with 148), 3 MB 3.5 (4.3), but 4 MB 4.5 (4.2); calls from Python 2 MB of fp32 4.1 (4.8), 2.8 MB 4.1 (5.0);
+//   * from 160 MB on where nothing is shifted, two rounds of the two CTAs per SM that fit: calls from Python 268 MB of fp32 moved
+//     88.3 us (91.9 with one per SM), scaled 89.3 (92.7), 180 MB scaled 61.5 (63.5); in graphs 164 MB 57.7 (58.5), 134 MB 47.1 (47.2).
+//     Shifted fp32 values of 268 MB take 104.7 so and 100.1 with one per SM.
+int LocalCtas(uint64_t bytes, bool shifted, int sms)
+{
+    if (bytes <= (3u << 20)) return (int)std::max<uint64_t>(1, std::min<uint64_t>(std::min(64, sms), (bytes + 8191) / 8192));
+    return !shifted && bytes >= (160u << 20) ? 4 * sms : sms;
+}
+namespace {
 // What the kernel takes: no more than it needs, since every launch copies it.
 struct LocalArgs {
     CommDev *dev;
@@ -1609,6 +1623,7 @@ HcclResult LaunchFastKernel(const FastLaunch &l)
 }
 
 
+extern "C" int HcommToolLocalCtas(uint64_t bytes, int shifted, int sms) { return LocalCtas(bytes, shifted != 0, sms); }
 // The split of a single rank's copy: bytes in front, words, bytes by which their source is shifted.
 extern "C" void HcommToolLocalSplit(uint64_t in, uint64_t out, uint64_t bytes, uint64_t *head, uint64_t *words, uint32_t *delta)
 {

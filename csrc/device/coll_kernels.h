@@ -112,6 +112,8 @@ uint32_t FastKindBarriers(int32_t kind, int preBarrier);
 // FK_LOCAL: whether a data type changes under it without a scale (16-bit floats pass through fp32, which gives every NaN one
 // form); all others are moved as bytes (launch those with HCCL_DATA_TYPE_UINT8 and the count in bytes).
 bool LocalNeedsType(int32_t dtype, bool scaled);
+// FK_LOCAL: CTAs for an operand of that many bytes whose buffers start alike within 16 bytes, or differently (shifted).
+int LocalCtas(uint64_t bytes, bool shifted, int sms);
 // SMs of the current device, 0 when it cannot be asked.
 int FastSmCount();
 // Upper bound of CTAs per rank for which all CTAs of `ranksOnDevice` ranks are co-resident.

@@ -25,6 +25,20 @@ def test_split_reads_and_writes_inside_the_operand(bytes_):
             assert first >= src and first + 16 * (w + (d > 0)) <= src + bytes_
 
 
+def test_ctas():
+    from hcomm_b200 import _lib
+    ctas = _lib.load().HcommToolLocalCtas
+
+    def of(bytes_, shifted=0, sms=148):
+        return ctas(ctypes.c_uint64(bytes_), shifted, sms)
+    assert [of(b) for b in (0, 1, 8192, 8193, 1 << 18)] == [1, 1, 1, 2, 32]
+    # as many as leave SMs to the next call, while they hold the operand in one round
+    assert of(1 << 20) == of(2 << 20) == of(3 << 20) == of(1 << 20, 1) == 64 and of(1 << 20, 0, 20) == 20
+    assert of((3 << 20) + 1) == of((160 << 20) - 1) == of((3 << 20) + 1, 1) == 148
+    # more rounds for the largest ones whose buffers start alike
+    assert of(160 << 20) == of(1 << 40) == 592 and of(1 << 28, 1) == 148
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("name,size", [("uint8", 1), ("bfloat16", 2), ("float32", 4), ("float64", 8)])
 def test_every_shift_between_the_buffers(name, size):
