@@ -308,14 +308,12 @@ __global__ void __launch_bounds__(512, 2) MoeDispatchKernel(const __grid_constan
 // together, half of them each, those of tokens before the cluster's apart, and read one another's counts: offsets and the first
 // row of every expert for every CTA follow without a word from another cluster, and rows are claimed from counters in shared
 // memory.  Then as above: the warps share the CTA's tokens in pieces of 512 values.
-// Bound by memory, and before that by the shared-memory atomics that count, during which memory is idle: hence, beyond kCountAlone
-// choices, one CTA of 1024 threads per SM and pairs of them, a quarter of the atomics of two CTAs of 512 that each count alone.  With
-// fewer choices the second CTA is worth more, and meeting costs more than counting (1024 x 8: 20.0 us alone, 23.5 in pairs; 2000 x 8:
-// 38.5 and 36.8).  4096 x 7168 to 8 of 256 experts 68.5 us (71.8 with every CTA counting alone), 9000 x 512 to 16 of 1024 29.6 (49.2), 64
+// Bound by memory, and before that by the shared-memory atomics that count, during which memory is idle: hence, with many choices,
+// one CTA of 1024 threads per SM and pairs of them, a quarter of the atomics of two CTAs of 512 that each count alone (the rule stands
+// at LocalDispatchShape).  4096 x 7168 to 8 of 256 experts 68.5 us (71.8 with every CTA counting alone), 9000 x 512 to 16 of 1024 29.6 (49.2), 64
 // tokens 7.1 (8.4).  Tried and no faster: rows put together in shared memory and sent with one bulk copy each (73 - 87 us), loads four
 // pieces ahead through shared memory (74.7), clusters of four CTAs of 512 (not all resident: 87).
 constexpr int kLocalThreads = 1024;
-constexpr int kCountAlone = 12288;
 
 __device__ __forceinline__ uint32_t LdClusterWord(const uint32_t *mine, uint32_t rank)
 {
@@ -670,16 +668,28 @@ HcclResult LaunchMoe(MoeCtx *m, void *kernel, const MoeParams &hp, int id, void 
     return HCCL_SUCCESS;
 }
 
+// The launch of a single rank's dispatch; `ctas`: as many as it may have.  A thread per expert in any case.
+// Counting alone and in pairs, us: counting takes time by the choice and is the larger part where rows are small (256 experts, 8 each,
+// 512 wide: 2048 tokens 11.3 and 11.4, 4096 15.7 and 13.7; 4096 wide: 2048 21.7 and 24.1, 3072 33.0 and 33.0), until there is so much to move that half as many, larger CTAs
+// do it better whatever the counting (8 experts, 1 each, 8192 wide: 10000 tokens 69.6 and 67.2; 2 each: 6144 49.8 and 50.3, 8192 63.2 and 62.5).
+struct DispatchShape {
+    int ctas, threads, cluster;
+};
+DispatchShape LocalDispatchShape(int64_t tokens, int topk, int experts, int hidden, int ctas, int sms)
+{
+    const bool many = tokens * topk > (hidden <= 1024 ? 17000 : 24000) || tokens * hidden > 55000000;
+    const int threads = many || experts > kLocalThreads / 2 ? kLocalThreads : kLocalThreads / 2;
+    const int mine = threads == kLocalThreads ? std::min(ctas, sms) : ctas, cluster = many && mine >= 2 ? 2 : 1;
+    return {mine / cluster * cluster, threads, cluster};
+}
+
 // The launches of a dispatch; hp.scratch holds the row cursors (a single rank needs none).
 HcclResult LaunchDispatch(MoeCtx *m, const MoeParams &hp, int routeId, int dispatchId, void *stream)
 {
     const int sms = MoeSms(), ctas = MoeCtas(m->comm, sms, hp.numTokens), emuCtas = std::max(1, sms / (int)m->comm->nRanks);
     if (m->comm->nRanks == 1) {
-        // a thread per expert in any case
-        const bool many = (int64_t)hp.numTokens * m->lay.topk > kCountAlone;
-        const int threads = many || m->lay.numExperts > kLocalThreads / 2 ? kLocalThreads : kLocalThreads / 2;
-        const int mine = threads == kLocalThreads ? std::min(ctas, sms) : ctas, cluster = many && mine >= 2 ? 2 : 1;
-        return LaunchMoe(m, (void *)MoeDispatchLocalKernel, hp, dispatchId, stream, mine / cluster * cluster, emuCtas, threads, cluster);
+        const DispatchShape l = LocalDispatchShape(hp.numTokens, m->lay.topk, m->lay.numExperts, m->lay.hidden, ctas, sms);
+        return LaunchMoe(m, (void *)MoeDispatchLocalKernel, hp, dispatchId, stream, l.ctas, emuCtas, l.threads, l.cluster);
     }
     CHK_RET(LaunchMoe(m, (void *)MoeRouteKernel, hp, routeId, stream, 1, 1, 1024));
     return LaunchMoe(m, (void *)MoeDispatchKernel, hp, dispatchId, stream, ctas, emuCtas, 512);
@@ -944,6 +954,13 @@ int HcommMoeDispatchStaticScratch(void *handle, const void *x, const int32_t *to
     hp.x = (const __nv_bfloat16 *)x; hp.topkIdx = topkIdx; hp.numTokens = numTokens;
     ++c->opSeq;
     return LaunchDispatch(m, hp, 9105, 9103, stream);
+}
+
+// The launch of a single rank's dispatch: shape = CTAs, threads of each, CTAs that count together.
+void HcommToolMoeDispatchShape(int tokens, int topk, int experts, int hidden, int ctas, int sms, int *shape)
+{
+    const DispatchShape l = LocalDispatchShape(tokens, topk, experts, hidden, ctas, sms);
+    shape[0] = l.ctas; shape[1] = l.threads; shape[2] = l.cluster;
 }
 
 // An exchange's device block from stand-in allocators in host memory: failing 0 = none, 1 = taking it, 2 = clearing it.

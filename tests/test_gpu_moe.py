@@ -282,8 +282,10 @@ def test_result_inside_the_experts_output_and_rows_in_the_landing_area(n, hidden
 
 @pytest.mark.parametrize("experts,topk,hidden,tokens,masked", [
     (256, 8, 7168, 1, False),           # a token, one CTA
-    (8, 1, 512, 4096, True),            # as many choices as every CTA counts alone, and one more
-    (8, 1, 512, 4097, True),
+    (8, 1, 512, 17000, True),           # as many choices as every CTA counts alone, and one more
+    (8, 1, 512, 17001, True),
+    (64, 3, 2048, 8001, True),          # in pairs, whose threads do not come out even in choices of a token
+    (8, 1, 8192, 6714, False),          # in pairs for what there is to move
     (256, 8, 7168, 4145, True),         # the pairs' tokens do not come out even
     (1024, 16, 512, 9600, False),       # a CTA claims rows twice, all counters
     (64, 3, 8192, 3001, True),
