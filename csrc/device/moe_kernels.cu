@@ -323,6 +323,8 @@ __device__ __forceinline__ uint32_t LdClusterWord(const uint32_t *mine, uint32_t
     return v;
 }
 
+// PER: experts of a thread.
+template <int PER>
 __global__ void __launch_bounds__(kLocalThreads, 1) MoeDispatchLocalKernel(const __grid_constant__ MoeParams byval, const MoeParams *)
 {
     const MoeParams &p = byval;         // never merged with another rank's launch
@@ -339,12 +341,12 @@ __global__ void __launch_bounds__(kLocalThreads, 1) MoeDispatchLocalKernel(const
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(ranks));
     const auto firstToken = [&](uint32_t cta) { return (int)((int64_t)p.numTokens * cta / gridDim.x); };
-    const int t0 = firstToken(blockIdx.x), t1 = firstToken(blockIdx.x + 1), segs = H / 512, all = (t1 - t0) * segs;
+    const int t0 = firstToken(blockIdx.x), t1 = firstToken(blockIdx.x + 1), segs = H / 512, pieces = (t1 - t0) * segs;
 
     // the first piece of this warp, and the choice that this thread claims a row for, are on their way while the rows are being found
     uint4 a = make_uint4(0, 0, 0, 0), b = a;
     const __nv_bfloat16 *src = p.x + (size_t)t0 * H + lane * 16;         // pieces of consecutive tokens are consecutive in x
-    auto fetch = [&](int item) { if (item < all) { a = LdStream16(src + (size_t)item * 512); b = LdStream16(src + (size_t)item * 512 + 8); } };
+    auto fetch = [&](int item) { if (item < pieces) { a = LdStream16(src + (size_t)item * 512); b = LdStream16(src + (size_t)item * 512 + 8); } };
     fetch(warp);
     const int perRound = (int)blockDim.x / K, claimed = (t1 - t0 < perRound ? t1 - t0 : perRound) * K;
     const int choice = tid < claimed ? p.topkIdx[(size_t)t0 * K + tid] : -1;
@@ -370,31 +372,42 @@ __global__ void __launch_bounds__(kLocalThreads, 1) MoeDispatchLocalKernel(const
     }
     if (ranks > 1) cg::this_cluster().sync();
     else __syncthreads();
-    uint32_t first = 0, tot = 0;        // of expert tid: choices of tokens before this CTA's, of all
-    if (tid < E) {
-        first = sCount[0][0][tid] + sCount[1][0][tid];
-        tot = sCount[0][1][tid] + sCount[1][1][tid];
-        if (ranks > 1) {
-            const uint32_t peer = rank ^ 1u;
-            const uint32_t b0 = LdClusterWord(&sCount[0][0][tid], peer), b1 = LdClusterWord(&sCount[1][0][tid], peer);
-            const uint32_t a0 = LdClusterWord(&sCount[0][1][tid], peer), a1 = LdClusterWord(&sCount[1][1][tid], peer), own = LdClusterWord(&sOwn[tid], peer);
-            first += b0 + b1;
-            tot += a0 + a1 + first;
-            if (rank) first += own;
-        } else {
-            tot += first;
+    uint32_t first[PER], tot[PER], all = 0;         // of this thread's experts: choices of tokens before this CTA's, of all
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int e = tid * PER + j;
+        first[j] = tot[j] = 0;
+        if (e < E) {
+            first[j] = sCount[0][0][e] + sCount[1][0][e];
+            tot[j] = sCount[0][1][e] + sCount[1][1][e];
+            if (ranks > 1) {
+                const uint32_t peer = rank ^ 1u;
+                const uint32_t b0 = LdClusterWord(&sCount[0][0][e], peer), b1 = LdClusterWord(&sCount[1][0][e], peer);
+                const uint32_t a0 = LdClusterWord(&sCount[0][1][e], peer), a1 = LdClusterWord(&sCount[1][1][e], peer), own = LdClusterWord(&sOwn[e], peer);
+                first[j] += b0 + b1;
+                tot[j] += a0 + a1 + first[j];
+                if (rank) first[j] += own;
+            } else {
+                tot[j] += first[j];
+            }
         }
+        all += tot[j];
     }
-    const uint32_t start = BlockExclusiveScan(tot, sWarp);
-    if (tid < E) {
-        sBase[tid] = start + first;
-        if (blockIdx.x == 0) {
-            // offsets for the grouped GEMM, clamped to the receive capacity like the route launch's
-            const uint32_t cap = (uint32_t)p.lay.maxRecvRows;
-            Counts(p, 0)[tid] = tot;
-            ExpertOffsets(p, 0)[tid] = start < cap ? start : cap;
-            if (tid == E - 1) ExpertOffsets(p, 0)[E] = start + tot < cap ? start + tot : cap;
+    uint32_t start = BlockExclusiveScan(all, sWarp);
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int e = tid * PER + j;
+        if (e < E) {
+            sBase[e] = start + first[j];
+            if (blockIdx.x == 0) {
+                // offsets for the grouped GEMM, clamped to the receive capacity like the route launch's
+                const uint32_t cap = (uint32_t)p.lay.maxRecvRows;
+                Counts(p, 0)[e] = tot[j];
+                ExpertOffsets(p, 0)[e] = start < cap ? start : cap;
+                if (e == E - 1) ExpertOffsets(p, 0)[E] = start + tot[j] < cap ? start + tot[j] : cap;
+            }
         }
+        start += tot[j];
     }
     if (ranks > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");       // its partner's counts have been read
     __syncthreads();
@@ -668,17 +681,20 @@ HcclResult LaunchMoe(MoeCtx *m, void *kernel, const MoeParams &hp, int id, void 
     return HCCL_SUCCESS;
 }
 
-// The launch of a single rank's dispatch; `ctas`: as many as it may have.  A thread per expert in any case.
+// The launch of a single rank's dispatch; `ctas`: as many as it may have.
 // Counting alone and in pairs, us: counting takes time by the choice and is the larger part where rows are small (256 experts, 8 each,
 // 512 wide: 2048 tokens 11.3 and 11.4, 4096 15.7 and 13.7; 4096 wide: 2048 21.7 and 24.1, 3072 33.0 and 33.0), until there is so much to move that half as many, larger CTAs
 // do it better whatever the counting (8 experts, 1 each, 8192 wide: 10000 tokens 69.6 and 67.2; 2 each: 6144 49.8 and 50.3, 8192 63.2 and 62.5).
+// Beyond 512 experts a thread of 512 has two, which beats half as many CTAs of 1024 (1024 experts, 8 each: 64 x 2048 6.3 us and 7.7, 512
+// x 8192 14.7 and 16.8, 1750 x 4096 19.9 and 22.7) but for many choices of small rows (1536 x 512 11.0 and 10.3).
 struct DispatchShape {
     int ctas, threads, cluster;
 };
 DispatchShape LocalDispatchShape(int64_t tokens, int topk, int experts, int hidden, int ctas, int sms)
 {
     const bool many = tokens * topk > (hidden <= 1024 ? 17000 : 24000) || tokens * hidden > 55000000;
-    const int threads = many || experts > kLocalThreads / 2 ? kLocalThreads : kLocalThreads / 2;
+    const bool smallRows = experts > kLocalThreads / 2 && hidden < 1024 && tokens * topk > 9000;
+    const int threads = many || smallRows ? kLocalThreads : kLocalThreads / 2;
     const int mine = threads == kLocalThreads ? std::min(ctas, sms) : ctas, cluster = many && mine >= 2 ? 2 : 1;
     return {mine / cluster * cluster, threads, cluster};
 }
@@ -689,7 +705,8 @@ HcclResult LaunchDispatch(MoeCtx *m, const MoeParams &hp, int routeId, int dispa
     const int sms = MoeSms(), ctas = MoeCtas(m->comm, sms, hp.numTokens), emuCtas = std::max(1, sms / (int)m->comm->nRanks);
     if (m->comm->nRanks == 1) {
         const DispatchShape l = LocalDispatchShape(hp.numTokens, m->lay.topk, m->lay.numExperts, m->lay.hidden, ctas, sms);
-        return LaunchMoe(m, (void *)MoeDispatchLocalKernel, hp, dispatchId, stream, l.ctas, emuCtas, l.threads, l.cluster);
+        void *kernel = m->lay.numExperts > l.threads ? (void *)MoeDispatchLocalKernel<2> : (void *)MoeDispatchLocalKernel<1>;
+        return LaunchMoe(m, kernel, hp, dispatchId, stream, l.ctas, emuCtas, l.threads, l.cluster);
     }
     CHK_RET(LaunchMoe(m, (void *)MoeRouteKernel, hp, routeId, stream, 1, 1, 1024));
     return LaunchMoe(m, (void *)MoeDispatchKernel, hp, dispatchId, stream, ctas, emuCtas, 512);
@@ -799,7 +816,8 @@ int HcommMoeCreate(HcclComm comm, int numExperts, int topk, int hidden, int maxT
     cudaFuncAttributes fa;
     cudaFuncGetAttributes(&fa, MoeRouteKernel);
     cudaFuncGetAttributes(&fa, MoeDispatchKernel);
-    cudaFuncGetAttributes(&fa, MoeDispatchLocalKernel);
+    cudaFuncGetAttributes(&fa, MoeDispatchLocalKernel<1>);
+    cudaFuncGetAttributes(&fa, MoeDispatchLocalKernel<2>);
     cudaFuncGetAttributes(&fa, MoeCombineSendKernel);
     for (bool merged : {false, true}) cudaFuncGetAttributes(&fa, SumKernel(topk, merged));
     cudaDeviceSynchronize();

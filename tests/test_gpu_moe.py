@@ -288,6 +288,9 @@ def test_result_inside_the_experts_output_and_rows_in_the_landing_area(n, hidden
     (8, 1, 8192, 6714, False),          # in pairs for what there is to move
     (256, 8, 7168, 4145, True),         # the pairs' tokens do not come out even
     (1024, 16, 512, 9600, False),       # a CTA claims rows twice, all counters
+    (1024, 16, 512, 560, True),         # two experts to a thread, none of them left over
+    (513, 3, 1024, 700, True),          # nearly all of them left over
+    (1000, 16, 512, 600, True),         # one to a thread, nobody's partner
     (64, 3, 8192, 3001, True),
 ])
 def test_single_rank_dispatch_counts_and_claims(experts, topk, hidden, tokens, masked):

@@ -36,6 +36,9 @@ def test_launch_of_a_single_ranks_dispatch():
     assert shape(2048, 8, 256, 4096) == shape(3000, 8, 256, 4096) == alone and shape(3001, 8, 256, 4096) == pairs
     # by what has to be moved
     assert shape(6713, 1, 8, 8192) == alone and shape(6714, 1, 8, 8192) == pairs
+    # two experts to a thread, but for many choices of small rows
+    assert shape(1750, 8, 1024, 4096) == shape(1124, 8, 1024, 512) == alone and shape(1126, 8, 1024, 512) == (148, 1024, 1)
+    assert shape(9000, 16, 1024, 512) == pairs
     # however few CTAs it may have
     assert shape(1, 8, 256, 7168, ctas=1) == (1, 512, 1)
     assert shape(4096, 8, 256, 7168, ctas=1) == (1, 1024, 1) and shape(4096, 8, 256, 7168, ctas=3) == (2, 1024, 2)
