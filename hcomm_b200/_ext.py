@@ -5,12 +5,15 @@ import ctypes
 import importlib.util
 import os
 import sys
+import threading
+import warnings
 from pathlib import Path
 
 from . import _lib
 
 _MODULE = None
 _CALLS = False          # not looked for yet
+_LOCK = threading.RLock()       # any thread's first call may be the one that loads
 _PATH = Path(__file__).resolve().parent / "lib" / "_hcomm_torch.so"
 
 
@@ -20,31 +23,38 @@ def extension():
     if _MODULE is not None:
         return _MODULE
     import torch.distributed                      # noqa: F401  the backend class derives from one of its types
-    _lib.load()                                   # libhcomm.so first: the extension links against it
-    if not _PATH.exists():
-        from . import build
-        build.build_torch_extension()
-    spec = importlib.util.spec_from_file_location("_hcomm_torch", str(_PATH))
-    mod = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(mod)
-    sys.modules["_hcomm_torch"] = mod
-    _MODULE = mod
-    return mod
+    with _LOCK:
+        if _MODULE is None:
+            _lib.load()                           # libhcomm.so first: the extension links against it
+            if not _PATH.exists():
+                from . import build
+                build.build_torch_extension()
+            spec = importlib.util.spec_from_file_location("_hcomm_torch", str(_PATH))
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+            sys.modules["_hcomm_torch"] = mod
+            _MODULE = mod
+    return _MODULE
 
 
 def native_calls():
     """The extension where calls can take the short way through it, else None: without a GPU, with another build of the library
-    selected, or where the extension was not built."""
+    selected, or where the extension was not built or does not load."""
     global _CALLS
-    if _CALLS is False:
-        import torch
-        found = None
-        if not os.environ.get("HCOMM_LIBRARY") and _PATH.exists() and torch.cuda.is_available():
-            try:
-                found = extension()
-            except ImportError:                   # built against another torch
-                found = None
-        _CALLS = found
+    if _CALLS is not False:
+        return _CALLS
+    import torch
+    with _LOCK:
+        if _CALLS is False:
+            found = failed = None
+            if not os.environ.get("HCOMM_LIBRARY") and _PATH.exists() and torch.cuda.is_available():
+                try:
+                    found = extension()
+                except ImportError as e:          # built against another torch
+                    failed = e
+            _CALLS = found
+            if failed is not None:
+                warnings.warn(f"{_PATH.name} does not load, calls take the longer way through Python: {failed}", stacklevel=2)
     return _CALLS
 
 

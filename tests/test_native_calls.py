@@ -20,6 +20,52 @@ def test_the_interpreter_lock_is_held_again_behind_an_exception(tmp_path):
     assert res.returncode == 0 and res.stdout.split() == ["0", "1", "1", "0", "1"], res.stdout + res.stderr
 
 
+def test_threads_that_come_at_once_get_one_extension():
+    # ranks may be threads of one process, and any operator may be the first call
+    program = """
+import sys, threading, time
+import torch.distributed
+from hcomm_b200 import _ext, _lib
+if not _ext._PATH.exists():
+    _ext.extension()
+    _ext._MODULE = None
+load = _lib.load
+_lib.load = lambda: (time.sleep(0.2), load())[1]        # all of them are between the first look and the load
+torch.cuda.is_available = lambda: True
+found = []
+threads = [threading.Thread(target=lambda f=f: found.append(f())) for f in [_ext.extension, _ext.native_calls] * 4]
+for t in threads:
+    t.start()
+for t in threads:
+    t.join()
+print(len(found), len({id(m) for m in found}), found[0] is sys.modules["_hcomm_torch"], _ext.native_calls() is found[0])
+"""
+    res = subprocess.run([sys.executable, "-c", program], capture_output=True, text=True, timeout=240, cwd=ROOT)
+    assert res.returncode == 0 and res.stdout.split() == ["8", "1", "True", "True"], res.stdout + res.stderr
+
+
+def test_an_extension_that_does_not_load_is_said_once(monkeypatch, tmp_path):
+    import warnings
+
+    import torch
+
+    from hcomm_b200 import _ext
+
+    def fails():
+        raise ImportError("undefined symbol")
+    (tmp_path / "ext.so").touch()
+    monkeypatch.setattr(_ext, "_CALLS", False)
+    monkeypatch.setattr(_ext, "_PATH", tmp_path / "ext.so")
+    monkeypatch.setattr(_ext, "extension", fails)
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    monkeypatch.delenv("HCOMM_LIBRARY", raising=False)
+    with pytest.warns(UserWarning, match="undefined symbol"):
+        assert _ext.native_calls() is None
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        assert _ext.native_calls() is None
+
+
 def test_without_a_gpu_the_general_way_is_taken():
     import torch
 
