@@ -81,6 +81,13 @@ template <int SPLIT> bool ClustersAtOnce(int *n)
     HCCL_INFO("GEMM clusters of %d CTAs resident at once: %d", 2 * SPLIT, *n);
     return true;
 }
+// cap[i] = what ask(pairs of a cluster, &n) says of i + 1; false where one of them failed: that is no answer to keep, unlike none at once.
+template <typename Ask> bool ClusterCaps(int *cap, Ask ask)
+{
+    bool all = true;
+    for (int pairs = 1; pairs <= 4; ++pairs) all = ask(pairs, &cap[pairs - 1]) && all;
+    return all;
+}
 // The limits of the current device: shared memory limits are a device's own, so its first call sets them.
 GemmLimits Limits()
 {
@@ -89,11 +96,12 @@ GemmLimits Limits()
     if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return {}; }
     return limits.Get(dev, [](GemmLimits *l) {
         const bool wide = AllowShared(GemmBf16PairWideKernel, hcgemm::ConfigWide<4>::kSmemBytes) && AllowShared(GemmBf16Pair224Kernel, hcgemm::Config2<224, 7>::kSmemBytes);
-        const bool one = ClustersAtOnce<1>(&l->cap[0]), two = ClustersAtOnce<2>(&l->cap[1]), four = ClustersAtOnce<4>(&l->cap[3]);
-        ClustersAtOnce<3>(&l->cap[2]);      // a device that holds none goes without
+        const bool clusters = ClusterCaps(l->cap, [](int pairs, int *n) {
+            return pairs == 1 ? ClustersAtOnce<1>(n) : pairs == 2 ? ClustersAtOnce<2>(n) : pairs == 3 ? ClustersAtOnce<3>(n) : ClustersAtOnce<4>(n);
+        });
         if (!wide) l->cap[0] = 0;
         l->single = AllowShared(GemmBf16Kernel<256>, hcgemm::Config<256>::kSmemBytes) && AllowShared(GemmBf16Kernel<128>, hcgemm::Config<128>::kSmemBytes);
-        return wide && one && two && four && l->single;
+        return wide && clusters && l->single;
     });
 }
 
@@ -557,6 +565,11 @@ extern "C" void HcommToolGemmTileOf(int M, int N, int K, const int *caps, int *t
     const hc::PairTile t = hc::PickPairTile(M, N, K, cap);
     if (tileWidth) *tileWidth = t.bn;
     if (pairsAlongK) *pairsAlongK = t.split;
+}
+// What is made of a device's answers, the clusters of 1 to 4 pairs that it holds at once, negative ones failures; whether they are kept.
+extern "C" int HcommToolGemmClusterCaps(const int *answers, int *caps)
+{
+    return hc::ClusterCaps(caps, [&](int pairs, int *n) { *n = std::max(0, answers[pairs - 1]); return answers[pairs - 1] >= 0; });
 }
 // What the current device holds.
 extern "C" void HcommToolGemmCaps(int *caps)

@@ -23,3 +23,15 @@ def test_a_failed_query_is_repeated():
 
 def test_devices_beyond_the_table_are_asked_every_time():
     assert ask((64, 5), (64, 6), (-1, 7)) == (3, [5, 6, 7])
+
+
+def test_what_a_gemm_finds_is_kept_only_if_every_query_was_answered():
+    def kept(*answers):
+        caps = (ctypes.c_int * 4)(*[-7] * 4)
+        return bool(_lib.load().HcommToolGemmClusterCaps((ctypes.c_int * 4)(*answers), caps)), list(caps)
+    assert kept(74, 33, 22, 15) == (True, [74, 33, 22, 15])
+    assert kept(74, 33, 0, 15) == (True, [74, 33, 0, 15])           # a device that holds no cluster of three pairs
+    for i in range(4):
+        answers = [74, 33, 22, 15]
+        answers[i] = -1
+        assert kept(*answers) == (False, [max(0, n) for n in answers])
