@@ -550,7 +550,7 @@ extern "C" void HcommGemmSetSplit(int pairsAlongK)
 {
     hc::g_forceSplit.store(pairsAlongK);
 }
-// The rule behind the automatic choice, for a device that holds cap1, cap2 and cap4 clusters of 1, 2 and 4 CTA pairs at once.
+// The rule behind the automatic choice, for a device that holds cap1, cap2 and cap4 clusters of 1, 2 and 4 CTA pairs at once and none of 3.
 extern "C" void HcommToolGemmTile(int M, int N, int K, int cap1, int cap2, int cap4, int *tileWidth, int *pairsAlongK)
 {
     const int cap[4] = {cap1, cap2, 0, cap4};
@@ -558,13 +558,14 @@ extern "C" void HcommToolGemmTile(int M, int N, int K, int cap1, int cap2, int c
     if (tileWidth) *tileWidth = t.bn;
     if (pairsAlongK) *pairsAlongK = t.split;
 }
-// The same for a device that holds caps[0] .. caps[3] clusters of 1 .. 4 pairs (HcommToolGemmTile: none of three).
-extern "C" void HcommToolGemmTileOf(int M, int N, int K, const int *caps, int *tileWidth, int *pairsAlongK)
+// The same for a device that holds caps[0] .. caps[3] clusters of 1 .. 4 pairs.  Returns which kernel, numbered as below.
+extern "C" int HcommToolGemmTileOf(int M, int N, int K, const int *caps, int *tileWidth, int *pairsAlongK)
 {
     const int cap[4] = {caps[0], caps[1], caps[2], caps[3]};
     const hc::PairTile t = hc::PickPairTile(M, N, K, cap);
     if (tileWidth) *tileWidth = t.bn;
     if (pairsAlongK) *pairsAlongK = t.split;
+    return (int)t.kernel;
 }
 // What is made of a device's answers, the clusters of 1 to 4 pairs that it holds at once, negative ones failures; whether they are kept.
 extern "C" int HcommToolGemmClusterCaps(const int *answers, int *caps)

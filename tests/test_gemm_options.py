@@ -19,9 +19,8 @@ def test_wide_tiles_can_be_switched_off():
 import ctypes
 from hcomm_b200 import _lib
 lib = _lib.load()
-bn, split = ctypes.c_int(), ctypes.c_int()
-lib.HcommToolGemmTile(8192, 28672, 8192, 74, 33, 15, ctypes.byref(bn), ctypes.byref(split))
-print(lib.HcommToolGemmKernel(8192, 28672, 8192, 74, 33, 15), bn.value)
+bn, caps = ctypes.c_int(), (ctypes.c_int * 4)(74, 33, 22, 15)
+print(lib.HcommToolGemmTileOf(8192, 28672, 8192, caps, ctypes.byref(bn), None), bn.value)
 """
     assert run(program, HCOMM_GEMM_WIDE="1").split() == ["1", "512"]
     kernel, width = run(program, HCOMM_GEMM_WIDE="0").split()

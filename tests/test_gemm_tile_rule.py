@@ -30,6 +30,52 @@ def test_every_shape_gets_a_tile_that_the_kernel_takes(caps):
                 assert split == 1 or (k + 63) // 64 >= 4 * split, "a part of K that is hardly a step"
 
 
+B200 = (74, 33, 22, 15)         # clusters of one to four pairs that one holds at once
+
+
+def choice(m, n, k, caps=B200):
+    """(kernel, tokens per tile, pairs that share a tile) on a device that holds so many clusters of one to four pairs."""
+    bn, split = ctypes.c_int(), ctypes.c_int()
+    kernel = _lib.load().HcommToolGemmTileOf(m, n, k, (ctypes.c_int * 4)(*caps), ctypes.byref(bn), ctypes.byref(split))
+    return kernel, bn.value, split.value
+
+
+@pytest.mark.parametrize("caps", [B200, (8, 4, 3, 2), (74, 0, 24, 0)])
+def test_every_shape_gets_a_tile_where_three_pairs_may_share_one(caps):
+    sizes = [8, 72, 136, 264, 768, 1000, 1024, 3584, 4096, 5000, 8192, 28672, 128256]
+    shared = 0
+    for m in [1, 15, 32, 33, 64, 65, 96, 127, 128, 129, 160, 200, 256, 257, 300, 777, 1024, 5003, 100000]:
+        for n in sizes:
+            for k in sizes:
+                kernel, bn, split = choice(m, n, k, caps)
+                assert 1 <= split <= 4 and (split == 1 or caps[split - 1] > 0), (m, n, k, split)
+                if kernel != 0:
+                    assert split == 1 and bn == {1: 512, 2: 128, 3: 224}[kernel]
+                    continue
+                assert 32 <= bn <= 256 and bn % 32 == 0 and bn - 32 < m, (m, n, k, bn)
+                if split > 1:
+                    assert (k + 63) // 64 >= 4 * split, "a part of K that is hardly a step"
+                    assert -(-n // 256) * -(-m // bn) <= caps[split - 1], "shared tiles in more than one wave"
+                    assert split != 3 or m <= 128, "three pairs beyond what they were measured to win"
+                    shared += split == 3
+    assert shared > 0
+
+
+def test_known_choices_of_a_b200():
+    # as on devices without clusters of three pairs, below, but for the shapes that three pairs win
+    for m, n, k, kernel, bn, split in [(16, 8192, 28672, 0, 32, 2), (16, 28672, 8192, 0, 32, 1), (96, 3584, 8192, 0, 96, 4), (33, 128256, 4096, 0, 64, 1),
+                                       (8192, 28672, 8192, 1, 512, 1), (777, 14336, 4096, 0, 160, 1), (8192, 3584, 8192, 0, 224, 1), (65536, 4096, 64, 1, 512, 1),
+                                       (16384, 8, 256, 2, 128, 1), (5956, 24, 936, 2, 128, 1), (512, 14336, 8192, 3, 224, 1)]:
+        assert choice(m, n, k) == (kernel, bn, split), (m, n, k)
+    # us with three pairs, and with what is taken without: 10.0 and 10.1, 10.4 and 11.4, 24.2 and 25.9
+    for m, n, k, bn, without in [(40, 4096, 4096, 64, (64, 2)), (64, 4096, 4096, 64, (32, 2)), (96, 4096, 14336, 96, (96, 2))]:
+        assert choice(m, n, k) == (0, bn, 3), (m, n, k)
+        assert choice(m, n, k, (74, 33, 0, 15)) == (0, *without), (m, n, k)
+    # limits of three pairs: tokens, steps of K, one wave
+    assert choice(128, 4096, 14336)[2] == 3 and choice(129, 4096, 14336)[2] != 3
+    assert choice(16, 4096, 14336, (74, 33, 15, 15))[2] != 3 and choice(16, 5000, 11 * 64)[2] != 3
+
+
 def test_known_choices():
     caps = (74, 33, 15)
     assert pick(16, 8192, 28672, caps) == (32, 2)       # 32 tiles: two pairs each, so that enough SMs ask for the weights

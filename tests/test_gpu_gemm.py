@@ -130,12 +130,28 @@ def test_oversized_raster_group(width):
     assert take_kernel_error() == 0 and torch.equal(got, want)
 
 
+def device_caps():
+    """Clusters of one to four CTA pairs that the current device holds at once: what its choices go by."""
+    import ctypes
+
+    from hcomm_b200 import _lib
+    caps = (ctypes.c_int * 4)()
+    _lib.load().HcommToolGemmCaps(caps)
+    return caps
+
+
+def test_the_device_holds_clusters_of_every_number_of_pairs():
+    caps = list(device_caps())
+    # a pair fills two SMs
+    assert all(n > 0 for n in caps) and all(caps[i] * (i + 1) <= caps[0] for i in range(4)) and caps[0] >= caps[1] >= caps[2] >= caps[3]
+
+
 @pytest.mark.parametrize("m,n,k", [(4097, 8, 64), (12800, 128, 8), (5003, 72, 136), (8192, 24, 1000), (19000, 8, 72), (40001, 64, 512)])
 def test_few_columns_of_many_rows(m, n, k):
     # the kernel without pairs is the one that runs here; rows of a longer pitch in, a result inside a wider matrix
     from hcomm_b200 import _lib
     from hcomm_b200.ops.gemm import gemm_bf16, take_kernel_error
-    assert _lib.load().HcommToolGemmKernel(m, n, k, 74, 33, 15) == 2
+    assert _lib.load().HcommToolGemmTileOf(m, n, k, device_caps(), None, None) == 2
     g = torch.Generator(device="cuda").manual_seed(m)
     a = torch.randn(m, k + 8, device="cuda", generator=g).to(torch.bfloat16)[:, :k]
     b = (torch.randn(n, k, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
@@ -154,7 +170,7 @@ def test_round_batch_of_a_layer_224_wide():
     from hcomm_b200 import _lib
     from hcomm_b200.ops.gemm import gemm_bf16, take_kernel_error
     m, n, k = 512, 14336, 4104
-    assert _lib.load().HcommToolGemmKernel(m, n, k, 74, 33, 15) == 3
+    assert _lib.load().HcommToolGemmTileOf(m, n, k, device_caps(), None, None) == 3
     g = torch.Generator(device="cuda").manual_seed(m)
     a = torch.randn(m, k + 8, device="cuda", generator=g).to(torch.bfloat16)[:, :k]
     b = (torch.randn(n, k + 16, device="cuda", generator=g) * 0.05).to(torch.bfloat16)[:, :k]
@@ -179,6 +195,7 @@ def test_every_number_of_parts_of_k(m, n, k, split):
     b = (torch.randn(n, k, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
     full = torch.full((m, n + 8), 7.0, device="cuda", dtype=torch.bfloat16)
     lib = _lib.load()
+    assert device_caps()[split - 1] > 0             # or the forced number would be left out
     ref = a.double() @ b.double().t()
     # one rounding to bf16 (half a step, 2^-9) and fp32 sums of k products (k * 2^-24 of the sum of magnitudes)
     bound = 2.0 ** -8 * ref.abs() + k * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t())

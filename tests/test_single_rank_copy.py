@@ -51,9 +51,17 @@ def test_every_shift_between_the_buffers(name, size):
     try:
         g = torch.Generator(device="cuda").manual_seed(size)
         steps = 16 // size
-        piece = 3072 // size                        # what a warp takes at a time
-        # no whole word; a piece and its neighbours; more pieces than one round of the grid's warps takes
-        for count in (1, 3 * steps, piece - 1, piece, piece + steps + 1, 8 * (1 << 20) // size + 5):
+        # what a warp takes at a time: six words of each lane, and eight of the shifted ones but 16-bit types; 16 warps of a CTA per SM
+        pieces = {3072 // size, 4096 // size}
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        # no whole word; a piece and its neighbours; the last size that few CTAs take, and the first that all do; two and three rounds
+        # of all of them and an odd rest, in either kernel's pieces
+        counts = {1, 3 * steps, (3 << 20) // size, (3 << 20) // size + 1}
+        for piece in pieces:
+            counts |= {piece - 1, piece, piece + steps + 1}
+        for words in (6, 8):
+            counts |= {rounds * sms * 16 * words * 512 // size + 3 * 4096 // size + 5 for rounds in (1, 2)}
+        for count in sorted(counts):
             base = torch.randint(-100, 100, (count + 32,), device="cuda", generator=g).to(dtype)
             for i in range(0, steps, max(1, steps // 8)):
                 for o in (0, 1, steps - 1):
@@ -67,5 +75,30 @@ def test_every_shift_between_the_buffers(name, size):
                         comm.all_reduce_scaled(x, out[o:o + count], 0.5)       # exact
                         want[o:o + count] = x * 0.5
                         assert torch.equal(out, want), (count, i, o)
+    finally:
+        comm.destroy()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,size", [("uint8", 1), ("bfloat16", 2), ("float32", 4)])
+def test_the_largest_operands_take_more_ctas(name, size):
+    import torch
+
+    import hcomm_b200 as hb
+    dtype = getattr(torch, name)
+    torch.cuda.set_device(0)
+    comm = hb.Communicator(1, hb.get_root_info(), 0, buffer_mb=4)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(size)
+        for count in ((160 << 20) // size - 1, (160 << 20) // size, (201 << 20) // size + 7):
+            base = torch.randint(-100, 100, (count + 32,), device="cuda", generator=g).to(dtype)
+            for i, o in ((0, 0), (5, 5), (0, 3)):           # alike, alike off a word, differently
+                x = base[i:i + count]
+                out = torch.full((count + 32,), 7, device="cuda", dtype=dtype)
+                comm.all_gather(x, out[o:o + count])
+                assert torch.equal(out[o:o + count], x) and bool((out[:o] == 7).all()) and bool((out[o + count:] == 7).all()), (count, i, o)
+                if dtype.is_floating_point:
+                    comm.all_reduce_scaled(x, out[o:o + count], 0.5)           # exact
+                    assert torch.equal(out[o:o + count], x * 0.5) and bool((out[o + count:] == 7).all()), (count, i, o)
     finally:
         comm.destroy()
