@@ -1274,13 +1274,14 @@ __global__ void __launch_bounds__(512) KIrInterp(const __grid_constant__ IrArgs 
 // either buffer starts on: where the two start differently within 16 bytes (an operand is often a slice of a flat buffer), a
 // word is cut out of the two aligned words of `in` that hold it, the second of which comes from the neighbouring lane.
 // Only whole words inside the operand are read; up to 31 bytes at either end go element by element.
-// Bound by HBM.  One CTA per SM, whose loads of the next 48 KB are on their way while the ones before are being written; pieces
-// of 3 KB are dealt over the CTAs, so that small operands spread and the last round is an even one.  33.4 M bf16 values scaled
-// into another buffer, 134 MB: 21.3 us in back-to-back calls, three elements off 22.7 (26.7 and 55.3 with two rounds of two CTAs
-// per SM, no loads ahead, in words of the widest alignment that both buffers shared); 10.8 M fp32 values moved 10.3 us (17.7), 2048 1.6 (2.7); 16.7 M fp32
-// three elements off 26.9 (36.2).
-constexpr int kLocalWords = 6;          // words of a lane in flight: 4 take 25.1 us for 6's 23.8, 8 and more no less (134 MB)
-constexpr int kLocalWordsShifted = 8;   // of shifted ones but 16-bit types, which do with 6: 26.9 us for 16.7 M fp32 values (30.3)
+// Bound by HBM.  CTAs of 512 threads (how many: LocalCtas), whose loads of the next round are on their way while the one before is being
+// written.  A warp takes a piece of 32 lanes x 6 words, 3 KB, at a time, or 8 words, 4 KB, where those are shifted and the type is not a
+// 16-bit one; pieces are dealt over the CTAs, so that small operands spread over them and the last round is an even one.
+// us a call in replayed graphs, before in words of the widest alignment that both buffers shared, two rounds of two CTAs per SM, no loads
+// ahead: 33.4 M bf16 values scaled into another buffer, 134 MB in all, 21.3 (26.7), three elements off 22.7 (55.3); 10.8 M fp32 values
+// moved 10.3 (17.7), 2048 1.6 (2.7); 16.7 M fp32 three elements off 26.9 (36.2).  Calls from Python: the bf16 values 24.0 (28.5).
+constexpr int kLocalWords = 6;          // words of a lane in flight: 4 take 25.1 us for 6's 23.8, 8 and more no less (134 MB, calls from Python)
+constexpr int kLocalWordsShifted = 8;   // of shifted ones but 16-bit types, which do with 6: 26.9 us for 16.7 M fp32 values (30.3); why was not found
 struct LocalSpan {
     uint64_t head;          // bytes in front of the first whole word of `out`
     uint64_t words;         // of `out`; shifted ones lie in one more of `in`

@@ -214,10 +214,13 @@ namespace {
 //     128-byte lines (seen from the third wave on: 16384 x 4096 x 1000 512/1 107 us, 256/1 122); every operand comes from HBM
 //     once at 6.5 TB/s, a tenth less when only a few SMs ask for it;
 //     up to 256 tokens, where weights come from HBM and go to every token tile, a fifth of the L2 time adds to that of HBM
-//     (40 x 4096 x 4096 64/2 10.5 us, not 32/2 12.1);
+//     (64 x 4096 x 4096 64/3 10.4 us, not 32/2 11.4);
 //   * a launch costs 3 us, emptying the last accumulator 6 ns per token, exchanging partial sums 0.6 us and 10 ns per token (three
 //     pairs up to 128 tokens only: beyond them they won nothing).
-//     Tiles are shared along K only where their clusters all fit at once: a further wave starts from nothing;
+//     Tiles are shared along K only where their clusters all fit at once: a further wave starts from nothing.
+//     Beyond 128 tokens the exchange costs more than this where a call follows its like: 8192 x 3584, 174 tokens 192/2 18.1 us, 96/1 17.8;
+//     227 256/2 20.4, 128/1 19.7.  Priced at 18 ns for each such token a first call takes longer (33.5 us for 30.5) and two layers together
+//     no less (176 and 223 tokens through 8192 / 3584 37.4 and 41.0 for 37.2 and 40.8), so the price stays;
 //   * a 256 x 512 tile moves a quarter less operand data than two of 256 x 256, and under the power cap that sets the clock:
 //     690 ns a step against 752, but 4 us in which nothing overlaps the emptying of its one accumulator.
 // Examples, us, against the fixed choice before (128 x 256 tiles of one CTA below 256 rows or at ragged ones):
